@@ -447,14 +447,14 @@ int ldsc_l2_workspace_bytes(const ldsc_l2_args* a, uint64_t n_indiv, uint64_t* b
     const uint64_t K = a->annot ? a->n_annot : 1;
     const uint32_t d = a->sketch_d;
     const bool exact_i8 = !d && a->precision == LDSC_PRECISION_INT8;
-    const int ta = (exact_i8 || d) ? 64 : 128, tb = 128;
+    const int ta = TILE_RECORDS, tb = TILE_RECORDS;
     const uint64_t ntiles = band_tiles(L.left, ta, tb).size();
     uint64_t b = m * (12 + 32 + 16 * K) + 8 * m + 8 * (ntiles + 1) + 64;  // stats, l2/aeff, left, tiles
     if (d && a->sketch_maf_aware) b += 16 * m;
     // f64 r2u tiles (K > 1) or per-tile row / column sums (K = 1), CSR tile lists
     const uint64_t nt_room = ntiles + ntiles / 8;  // the run's headroom on tile-count buffers
     b += (K > 1 ? (uint64_t)8 * ta * tb * nt_room : (uint64_t)8 * (ta + tb) * nt_room) + 8 * nt_room +
-         4 * (m / 64 + m / 128 + 4);
+         4 * (2 * (m / 128) + 4);
     if (a->annot && !a->annot_on_device) b += 8 * m * K;
     if (a->bed_idx) b += 8 * m;
     if (a->keep_iids) b += 8 * a->n_keep;
@@ -722,7 +722,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     // place when the records are the panel rows in order and every individual
     // is used
     const bool fused_i8 = exact_i8 && !a->bed_idx && !a->keep_iids && (ctx->flags & LDSC_CTX_FUSED_OPERANDS);
-    const int ta = (exact_i8 || d) ? 64 : 128, tb = 128;  // tcgen05 tiles: 64 x 128 records
+    const int ta = TILE_RECORDS, tb = TILE_RECORDS;
     pf.gram_kind = d ? 2u : (exact_i8 ? 1u : 0u);
 
     cudaStream_t s = ctx->stream;
@@ -1041,10 +1041,10 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                         ec.pcol += t0 * tb;
                         if (fused_i8)
                             CK(launch_gram_i8_packed(pv.rows, pv.pitch, n_used, m, ctx->tiles.as<Tile>() + t0,
-                                                     (int64_t)(t1 - t0), ec, nullptr, ctx->sms, s));
+                                                     (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, s));
                         else
                             CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>() + t0,
-                                              (int64_t)(t1 - t0), ec, nullptr, ctx->sms, s));
+                                              (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, s));
                         ctx->kernels++;
                     }
                     t0 = t1;
@@ -1134,7 +1134,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             ec.prow += t0 * ta;
             ec.pcol += t0 * tb;
             CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>() + t0, (int64_t)(t1 - t0), ec,
-                              nullptr, ctx->sms, s));
+                              nullptr, 0, ctx->sms, s));
             ctx->kernels++;
             t0 = t1;
         }
@@ -1144,13 +1144,13 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     if (!tiles.empty() && !stream_gram && !overlap) {
         if (d) {
             CK(launch_gram_tf32(ctx->xsk.as<float>(), ld_sk, m, ctx->tiles.as<Tile>(), (int64_t)tiles.size(), ep,
-                                maf_aware ? 1 : 0, nullptr, ctx->sms, s));
+                                maf_aware ? 1 : 0, ctx->sms, s));
         } else if (fused_i8) {
             CK(launch_gram_i8_packed(pv.rows, pv.pitch, n_used, m, ctx->tiles.as<Tile>(), (int64_t)tiles.size(), ep,
-                                     nullptr, ctx->sms, s));
+                                     nullptr, 0, ctx->sms, s));
         } else if (exact_i8) {
             CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>(), (int64_t)tiles.size(), ep,
-                              nullptr, ctx->sms, s));
+                              nullptr, 0, ctx->sms, s));
         } else {
             CK(launch_gram_f64(ctx->xf64.as<double>(), ld_f64, ld_f64, ctx->tiles.as<Tile>(), (int64_t)tiles.size(),
                                ep, ctx->sms, s));
@@ -1414,7 +1414,8 @@ int ldsc_debug_gram_i8_tile(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t k0,
     CK(launch_finalize_stats(m, n, st, nullptr, 1, 0, 0.0, ctx->aeff.as<double>(), ctx->l2.as<double>(), s));
     CK(cudaMemsetAsync(ctx->left.p, 0, 8 * (size_t)m, s));
     CK(cudaMemsetAsync(ctx->err.p, 0, 16, s));
-    Tile t{(uint32_t)(k0 / 64), (uint32_t)(j0 / 128)};
+    Tile t{(uint32_t)(k0 / TILE_RECORDS), (uint32_t)(j0 / TILE_RECORDS)};
+    const int dbg_row = (int)(k0 % TILE_RECORDS);
     CK(cudaMemcpyAsync(ctx->tiles.p, &t, sizeof(Tile), cudaMemcpyHostToDevice, s));
     EpilogueArgs ep{};
     ep.left = ctx->left.as<int64_t>();
@@ -1430,10 +1431,10 @@ int ldsc_debug_gram_i8_tile(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t k0,
     ep.err = ctx->err.as<unsigned int>();
     if (fused)
         CK(launch_gram_i8_packed(panel->rows, panel->pitch, n, m, ctx->tiles.as<Tile>(), 1, ep,
-                                 ctx->dbg.as<int32_t>(), ctx->sms, s));
+                                 ctx->dbg.as<int32_t>(), dbg_row, ctx->sms, s));
     else
         CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld, m, ctx->tiles.as<Tile>(), 1, ep, ctx->dbg.as<int32_t>(),
-                          ctx->sms, s));
+                          dbg_row, ctx->sms, s));
     ctx->kernels += 3;
     unsigned int herr[4];
     CK(cudaMemcpyAsync(out, ctx->dbg.p, 4 * 128 * 256, cudaMemcpyDeviceToHost, s));

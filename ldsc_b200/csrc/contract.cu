@@ -4,7 +4,7 @@
 // in both directions (src/l2/compute.rs:1869-1893, 2259-2314):
 //     l2[window] += R_ab * A_chunk,   l2[chunk] += R_ab^T * A_window (+ R_bb A_chunk).
 // Here the Gram kernels leave every band tile's masked r2u values in global
-// memory (f64, row k of the tile = TB values) and these passes do the two
+// memory (f64, row j of the tile = TA values) and these passes do the two
 // products per block of rows: pass "by right block" owns l2 rows j of one
 // right block, pass "by left block" owns l2 rows k of one left block, so no
 // row is written by two CTAs of a pass and the summation order is fixed.
@@ -47,9 +47,9 @@ struct MmaShape {
     static constexpr int SPT = NS / JS_M;                  // staged steps per tile
     static constexpr int WARPS = (OB / 32) * (MK / 32);
     static constexpr int THREADS = 32 * WARPS;
-    // r2u stage: BY_RIGHT [JS_M k][TB j], BY_LEFT [TA k][JS_M j]
-    static constexpr int RLD = BY_RIGHT ? TB + 4 : JS_M + 4;
-    static constexpr int RROWS = BY_RIGHT ? JS_M : TA;
+    // r2u stage: BY_RIGHT [TB j][JS_M k], BY_LEFT [JS_M j][TA k]
+    static constexpr int RLD = BY_RIGHT ? JS_M + 4 : TA + 4;
+    static constexpr int RROWS = BY_RIGHT ? TB : JS_M;
     static constexpr int R_ELEMS = RROWS * RLD;
     static constexpr int A_ELEMS = MK * SLD;
     static constexpr int STAGE = R_ELEMS + A_ELEMS;          // doubles per buffer
@@ -109,18 +109,18 @@ __global__ void __launch_bounds__(MmaShape<TA, TB, BY_RIGHT>::THREADS)
             double* Rs = smm + b * S::STAGE;
             double* As = Rs + S::R_ELEMS;
             if (BY_RIGHT) {
-                // rows k = js .. js + 31 of the tile, all TB values: 16-byte pieces
+                // all TB rows j, values k = js .. js + 31: 16-byte pieces
 #pragma unroll
-                for (int q = tid; q < JS_M * TB / 2; q += NTH) {
-                    const int r = q / (TB / 2), cc = 2 * (q % (TB / 2));
-                    cp_async16(Rs + r * RLD + cc, src + (size_t)(js + r) * TB + cc);
+                for (int q = tid; q < TB * JS_M / 2; q += NTH) {
+                    const int r = q / (JS_M / 2), cc = 2 * (q % (JS_M / 2));
+                    cp_async16(Rs + r * RLD + cc, src + (size_t)r * TA + js + cc);
                 }
             } else {
-                // all TA rows, values js .. js + 31
+                // rows j = js .. js + 31, all TA values
 #pragma unroll
-                for (int q = tid; q < TA * JS_M / 2; q += NTH) {
-                    const int r = q / (JS_M / 2), cc = 2 * (q % (JS_M / 2));
-                    cp_async16(Rs + r * RLD + cc, src + (size_t)r * TB + js + cc);
+                for (int q = tid; q < JS_M * TA / 2; q += NTH) {
+                    const int r = q / (TA / 2), cc = 2 * (q % (TA / 2));
+                    cp_async16(Rs + r * RLD + cc, src + (size_t)(js + r) * TA + cc);
                 }
             }
             // annotation column c0 + c of summed record s at aeff[s + (c0 + c) m]; consecutive threads
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(MmaShape<TA, TB, BY_RIGHT>::THREADS)
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const int orow = 32 * rg + 8 * i + fr;  // output row of the fragment
-                        a[i] = BY_RIGHT ? Rs[(kk + fc) * RLD + orow] : Rs[orow * RLD + kk + fc];
+                        a[i] = BY_RIGHT ? Rs[orow * RLD + kk + fc] : Rs[(kk + fc) * RLD + orow];
                     }
 #pragma unroll
                     for (int j = 0; j < 4; j++) b[j] = As[(32 * cg + 8 * j + fr) * SLD + kk + fc];
@@ -226,16 +226,13 @@ cudaError_t launch_contract(const double* rtiles, int ta, int tb, const Tile* ti
     };
 #define LDSC_CONTRACT(TA_, TB_, BR_) \
     go(k_contract_mma<TA_, TB_, BR_>, MmaShape<TA_, TB_, BR_>::smem, MmaShape<TA_, TB_, BR_>::THREADS)
-    if (ta == 64 && tb == 128) return by_right ? LDSC_CONTRACT(64, 128, true) : LDSC_CONTRACT(64, 128, false);
     if (ta == 128 && tb == 128) return by_right ? LDSC_CONTRACT(128, 128, true) : LDSC_CONTRACT(128, 128, false);
 #undef LDSC_CONTRACT
     return cudaErrorInvalidValue;
 }
 
 cudaError_t preload_contract() {
-    cudaError_t e = preload_kernel(k_contract_mma<64, 128, true>);
-    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<64, 128, false>);
-    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<128, 128, true>);
+    cudaError_t e = preload_kernel(k_contract_mma<128, 128, true>);
     if (e == cudaSuccess) e = preload_kernel(k_contract_mma<128, 128, false>);
     if (e == cudaSuccess) e = preload_kernel(k_l2_reduce);
     return e;

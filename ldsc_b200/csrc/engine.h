@@ -39,6 +39,9 @@ struct RecStats {
     double* pq;        // (maf (1 - maf))^pq_exp, may be null
 };
 
+// Records per side of a band tile (left block x right block), every form.
+constexpr int TILE_RECORDS = 128;
+
 // Band tile: A block (k side, left SNPs) x B block (j side, right SNPs).
 struct Tile {
     uint32_t a_blk;
@@ -62,7 +65,7 @@ struct EpilogueArgs {
     double n_inv_sq;          // 1 / N^2       (sketch form)
     double sketch_d;          // d as double   (sketch form)
     unsigned int* err;        // device error word (non-zero = a bounded wait gave up)
-    double* rtiles;           // K > 1: tile t's masked r2u values, ta rows (k) x tb (j) f64 at t * ta * tb
+    double* rtiles;           // K > 1: tile t's masked r2u values, tb rows (j) x ta (k) f64 at t * ta * tb
     // K = 1: tile t's row sums (ta values at prow + t * ta: sum_j r2u a_j for
     // each left record k) and column sums (tb values at pcol + t * tb), added
     // to l2 in a fixed order by launch_l2_reduce; null = atomics into l2
@@ -99,11 +102,12 @@ cudaError_t launch_gram_f64(const double* x, uint64_t ld, uint64_t kdim, const T
                             int64_t n_tiles, const EpilogueArgs& ep, int sms,
                             cudaStream_t stream);
 
-// INT8 tcgen05 band Gram + exact epilogue (TA = 64, TB = 128 records per tile).
+// INT8 tcgen05 band Gram + exact epilogue (128 x 128 records per tile).
 // ops: 2*m rows of `ld` bytes.  dbg (optional) receives the raw accumulators
-// of the first tile (128 x 256 int32).
+// of the first tile's left records dbg_row .. dbg_row + 63 (128 x 256 int32,
+// genotype and mask rows / columns interleaved).
 cudaError_t launch_gram_i8(const uint8_t* ops, uint64_t ld, int64_t m, const Tile* tiles,
-                           int64_t n_tiles, const EpilogueArgs& ep, int32_t* dbg, int sms,
+                           int64_t n_tiles, const EpilogueArgs& ep, int32_t* dbg, int dbg_row, int sms,
                            cudaStream_t stream);
 
 // Fused INT8 band Gram over the packed BED rows themselves (record r at
@@ -112,7 +116,7 @@ cudaError_t launch_gram_i8(const uint8_t* ops, uint64_t ld, int64_t m, const Til
 // operand rows exist in device memory.  Same tiles, epilogue and results as
 // launch_gram_i8; the per-record n / s / qinv come from a moments-only decode.
 cudaError_t launch_gram_i8_packed(const uint8_t* rows, uint64_t pitch, uint64_t n_indiv, int64_t m, const Tile* tiles,
-                                  int64_t n_tiles, const EpilogueArgs& ep, int32_t* dbg, int sms,
+                                  int64_t n_tiles, const EpilogueArgs& ep, int32_t* dbg, int dbg_row, int sms,
                                   cudaStream_t stream);
 
 // CountSketch, step 1 (once per panel, sketch dimension and individual set):
@@ -145,9 +149,9 @@ bool sketch_supported(uint64_t n_used, uint32_t d);
 
 // CountSketch band Gram on tcgen05 kind::tf32 over split rows (hi/lo
 // interleaved, `ld` floats per row, ld*4 a multiple of 128) + quadratic
-// bias-correction epilogue (TA = 64, TB = 128 records per tile).
+// bias-correction epilogue (128 x 128 records per tile).
 cudaError_t launch_gram_tf32(const float* ops, uint64_t ld, int64_t m, const Tile* tiles, int64_t n_tiles,
-                             const EpilogueArgs& ep, int maf_aware, int32_t* dbg, int sms, cudaStream_t stream);
+                             const EpilogueArgs& ep, int maf_aware, int sms, cudaStream_t stream);
 
 // FP32 band Gram of sketched rows + quadratic bias correction epilogue.
 cudaError_t launch_gram_f32(const float* x, uint64_t ld, uint64_t kdim, const Tile* tiles,

@@ -161,9 +161,8 @@ __global__ void __launch_bounds__(NT, 1)
             }
             __syncthreads();
         } else {
-            // K > 1: the masked r2u tile goes to global memory in f64 (row k of
-            // TB values) for the banded annotation contraction (contract.cu);
-            // the 16 lanes of a row store 128 contiguous bytes
+            // K > 1: the masked r2u tile goes to global memory in f64 (row j of
+            // TA values) for the banded annotation contraction (contract.cu)
             double* dst = ep.rtiles + (size_t)t * TA * TB;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -173,7 +172,7 @@ __global__ void __launch_bounds__(NT, 1)
                     const int64_t j = j0 + tx + 16 * l;
                     double r = 0.0;
                     if (pair_in_band(k, j, m, ep.left)) r = correct<MODE>((double)acc[i][l], k, j, ep);
-                    dst[(ty + 16 * i) * TB + tx + 16 * l] = r;
+                    dst[(tx + 16 * l) * TA + ty + 16 * i] = r;
                 }
             }
         }

@@ -92,7 +92,10 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     const uint64_t m = n_snp;
     const uint64_t ld = up(n_indiv, 128);
     std::vector<int64_t> lv(left, left + m);
-    const std::vector<Tile> tiles = band_tiles(lv, 64, 128);
+    const std::vector<Tile> tiles = band_tiles(lv, TILE_RECORDS, TILE_RECORDS);
+    // the documented limit counts 8 bytes per 64 x 128 records of the band (at
+    // least as many entries as the list above has)
+    const uint64_t tile_room = band_tiles(lv, 64, 128).size();
     uint64_t off = 0;
     auto take = [&](uint64_t bytes) {
         const uint64_t o = off;
@@ -101,7 +104,7 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     };
     const uint64_t o_ops = take(2 * m * ld), o_n = take(4 * m), o_s = take(4 * m), o_q = take(4 * m),
                    o_mean = take(8 * m), o_inv = take(8 * m), o_qinv = take(8 * m), o_aeff = take(8 * m),
-                   o_left = take(8 * m), o_tiles = take(sizeof(Tile) * (tiles.size() + 1)), o_err = take(16);
+                   o_left = take(8 * m), o_tiles = take(sizeof(Tile) * (tile_room + 1)), o_err = take(16);
     if (off > (uint64_t)LDSC_NOALLOC_SCRATCH_BYTES)
         return set_error(LDSC_E_INVALID, "ldsc_l2_int8_noalloc: n_snp=" + std::to_string(m) + ", n_indiv=" +
                                              std::to_string(n_indiv) + " needs " + std::to_string(off) +
@@ -158,7 +161,7 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     ep.err = reinterpret_cast<unsigned int*>(base + o_err);
     if (!tiles.empty() &&
         (rc = ck(launch_gram_i8(ops, ld, (int64_t)m, reinterpret_cast<Tile*>(base + o_tiles), (int64_t)tiles.size(),
-                                ep, nullptr, sms, s),
+                                ep, nullptr, 0, sms, s),
                  "gram")))
         return rc;
     unsigned int herr = 0;

@@ -476,6 +476,12 @@ int ldsc_noalloc_last_error(char *buf, size_t len);
 int ldsc_debug_gram_i8_tile(ldsc_ctx *ctx, const ldsc_panel *panel, uint64_t k0, uint64_t j0,
                             int32_t *out);
 
+/* The tcgen05 Gram's tile list for n_snp left limits (host only): up to `cap`
+ * rows of (left block, right block, first quarter, quarters) into out; returns
+ * the number of tiles, or LDSC_E_INVALID. */
+int64_t ldsc_debug_gram_tiles(const int64_t *left, uint64_t n_snp, int32_t trim, int32_t max_quarters,
+                              uint32_t *out, uint64_t cap);
+
 #ifdef __cplusplus
 }
 #endif

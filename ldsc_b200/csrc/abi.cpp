@@ -115,8 +115,9 @@ struct ldsc_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t copy = nullptr;  // host-to-device BED stream of ldsc_l2_from_bed
     cudaStream_t side = nullptr;  // low-priority stream of the decode that overlaps the Gram
+    cudaStream_t gram2 = nullptr;  // every other Gram launch of an overlapped run
     std::vector<cudaEvent_t> ovl_ev;  // per decoded record chunk
-    cudaEvent_t ovl_go = nullptr;
+    cudaEvent_t ovl_go = nullptr, ovl_plan = nullptr, ovl_done = nullptr;
     std::mutex mu;
     std::string last_error;
     uint64_t kernels = 0;
@@ -129,7 +130,7 @@ struct ldsc_ctx {
     uint64_t sk_panel = 0;
     GraphCache graphs;            // regression pipelines
     uint64_t graph_launches = 0;  // replays of cached graphs
-    DevBuf rtiles, cptr_r, cidx_r, cptr_l, cidx_l;  // K > 1 contraction: r2u tiles and CSR tile lists
+    DevBuf rtiles, roff, cptr_r, cidx_r, cptr_l, cidx_l;  // K > 1 contraction: r2u tiles and CSR tile lists
     DevBuf prow, pcol;                              // K = 1: per-tile row / column sums
     DevBuf rg_jobs, rg_states, rg_outs, rg_part, rg_tdel, rg_y, rg_y2, rg_n, rg_ld, rg_wld, rg_sel, rg_pairs, rg_res;
     DevBuf ts_seps, ts_n1, ts_cnt, ts_dv, ts_outs;  // --two-step
@@ -140,6 +141,7 @@ struct ldsc_ctx {
     LeftLimits plan_left;
     std::vector<Tile> plan_tiles;
     std::vector<int32_t> plan_ptr_r, plan_idx_r, plan_ptr_l, plan_idx_l;  // CSR tile lists
+    std::vector<uint32_t> plan_roff;
     // whole-file entry: staged file rows, the pitched panel, per-chunk events
     DevBuf bed_stage, bed_rows;
     std::vector<cudaEvent_t> feed_ev;
@@ -151,7 +153,7 @@ struct ldsc_ctx {
                       &pq, &err, &st_n, &st_s, &st_q, &st_q3,
                       &st_q4, &st_mean, &st_inv, &st_qinv, &st_kappa,
                       &packed, &tsum, &dbg,
-                      &rtiles, &cptr_r, &cidx_r, &cptr_l, &cidx_l, &prow, &pcol,
+                      &rtiles, &roff, &cptr_r, &cidx_r, &cptr_l, &cidx_l, &prow, &pcol,
                       &rg_jobs, &rg_states, &rg_outs, &rg_part, &rg_tdel,
                       &rg_y, &rg_y2, &rg_n, &rg_ld, &rg_wld, &rg_sel,
                       &rg_pairs, &rg_res, &bed_stage, &bed_rows, &ts_seps, &ts_n1, &ts_cnt, &ts_dv, &ts_outs,
@@ -256,15 +258,17 @@ int ldsc_ctx_destroy(ldsc_ctx* ctx) {
     std::vector<DevBuf*> bufs = ctx->workspace();
     cudaStreamSynchronize(ctx->copy);
     if (ctx->side) cudaStreamSynchronize(ctx->side);
+    if (ctx->gram2) cudaStreamSynchronize(ctx->gram2);
     for (DevBuf* b : bufs) b->release();
     ctx->sk.release();
     ctx->graphs.clear();
     cudaStreamSynchronize(ctx->stream);
     for (cudaEvent_t e : ctx->feed_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->ovl_ev) cudaEventDestroy(e);
-    for (cudaEvent_t e : {ctx->feed_t0, ctx->feed_t1, ctx->feed_go, ctx->up_ev, ctx->ovl_go})
+    for (cudaEvent_t e : {ctx->feed_t0, ctx->feed_t1, ctx->feed_go, ctx->up_ev, ctx->ovl_go, ctx->ovl_plan, ctx->ovl_done})
         if (e) cudaEventDestroy(e);
     if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->gram2) cudaStreamDestroy(ctx->gram2);
     if (ctx->copy) cudaStreamDestroy(ctx->copy);
     if (ctx->own) cudaStreamDestroy(ctx->own);
     delete ctx;
@@ -295,6 +299,8 @@ int ldsc_ctx_trim(ldsc_ctx* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     cudaStreamSynchronize(ctx->copy);
+    for (cudaStream_t x : {ctx->side, ctx->gram2})
+        if (x) cudaStreamSynchronize(x);
     ctx->graphs.clear();  // their kernels hold the buffers' addresses
     for (DevBuf* b : ctx->workspace()) b->release();
     ctx->sk.release();
@@ -447,14 +453,19 @@ int ldsc_l2_workspace_bytes(const ldsc_l2_args* a, uint64_t n_indiv, uint64_t* b
     const uint64_t K = a->annot ? a->n_annot : 1;
     const uint32_t d = a->sketch_d;
     const bool exact_i8 = !d && a->precision == LDSC_PRECISION_INT8;
-    const int ta = TILE_RECORDS, tb = TILE_RECORDS;
-    const uint64_t ntiles = band_tiles(L.left, ta, tb).size();
+    std::vector<Tile> tl;
+    gram_tiles(L.left, gram_trims(d ? 4 * round_up(d, 32) : round_up(n_used, 128)), 4, &tl);
+    uint64_t quarters = 0;
+    for (const Tile& t : tl) quarters += t.nq1 + 1u;
+    // a run with fewer tiles than SMs cuts them finer, up to one per SM
+    const uint64_t ntiles = K == 1 ? std::max<uint64_t>(tl.size(), std::min<uint64_t>(quarters, 160)) : tl.size();
     uint64_t b = m * (12 + 32 + 16 * K) + 8 * m + 8 * (ntiles + 1) + 64;  // stats, l2/aeff, left, tiles
     if (d && a->sketch_maf_aware) b += 16 * m;
     // f64 r2u tiles (K > 1) or per-tile row / column sums (K = 1), CSR tile lists
     const uint64_t nt_room = ntiles + ntiles / 8;  // the run's headroom on tile-count buffers
-    b += (K > 1 ? (uint64_t)8 * ta * tb * nt_room : (uint64_t)8 * (ta + tb) * nt_room) + 8 * nt_room +
-         4 * (2 * (m / 128) + 4);
+    b += (K > 1 ? (uint64_t)8 * TILE_RECORDS * TILE_QUARTER * (quarters + quarters / 8) + 4 * nt_room
+                : (uint64_t)8 * 2 * TILE_RECORDS * nt_room) +
+         8 * nt_room + 4 * (2 * (m / 128) + 4);
     if (a->annot && !a->annot_on_device) b += 8 * m * K;
     if (a->bed_idx) b += 8 * m;
     if (a->keep_iids) b += 8 * a->n_keep;
@@ -464,6 +475,19 @@ int ldsc_l2_workspace_bytes(const ldsc_l2_args* a, uint64_t n_indiv, uint64_t* b
     else b += 8 * m * round_up(n_used, 128);
     *bytes = b;
     return LDSC_OK;
+}
+
+int64_t ldsc_debug_gram_tiles(const int64_t* left, uint64_t n_snp, int32_t trim, int32_t max_quarters, uint32_t* out,
+                              uint64_t cap) {
+    if ((n_snp && !left) || (cap && !out) || max_quarters < 1 || max_quarters > 4) return LDSC_E_INVALID;
+    std::vector<Tile> tiles;
+    gram_tiles(std::vector<int64_t>(left, left + n_snp), trim != 0, max_quarters, &tiles);
+    for (size_t t = 0; t < tiles.size() && t < cap; t++) {
+        const Tile& x = tiles[t];
+        const uint32_t row[4] = {x.a_blk, x.b_blk, x.q0, x.nq1 + 1u};
+        std::memcpy(out + 4 * t, row, sizeof row);
+    }
+    return (int64_t)tiles.size();
 }
 
 int ldsc_l2_pair_count(const ldsc_l2_args* a, uint64_t* n_pairs) {
@@ -628,7 +652,9 @@ int ensure_overlap(ldsc_ctx* ctx, int n) {
         CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         CK(cudaStreamCreateWithPriority(&ctx->side, cudaStreamNonBlocking, least));
     }
-    if (!ctx->ovl_go) CK(cudaEventCreateWithFlags(&ctx->ovl_go, cudaEventDisableTiming));
+    if (!ctx->gram2) CK(cudaStreamCreateWithFlags(&ctx->gram2, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&ctx->ovl_go, &ctx->ovl_plan, &ctx->ovl_done})
+        if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     while ((int)ctx->ovl_ev.size() < n) {
         cudaEvent_t e;
         CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -876,7 +902,11 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         if (L.any_full && !a->yes_really)
             std::printf("WARNING: LD window spans the entire chromosome. Use --yes-really to silence this warning.\n");
         pf.n_pairs = L.n_pairs;
-        band_tiles(L.left, ta, tb, &tiles);
+        const bool trim = gram_trims(d ? 4 * round_up(d, 32) : round_up(n_used, 128));
+        if (K == 1 && (d || exact_i8))
+            gram_tiles_for(L.left, trim, ctx->sms, &tiles);
+        else
+            gram_tiles(L.left, trim, 4, &tiles);
         pf.n_tiles = tiles.size();
         CK(ctx->left.ensure(sizeof(int64_t) * nmom));
         // buffers sized by the tile count get an eighth more when they grow: a
@@ -910,7 +940,16 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                 idx_l[fl[tiles[t].a_blk]++] = t;
             }
             if (K > 1) {
-                CK(ctx->rtiles.ensure(sizeof(double) * (size_t)ta * tb * nt_room));
+                std::vector<uint32_t>& roff = ctx->plan_roff;
+                roff.resize(tiles.size());
+                uint32_t q = 0;
+                for (size_t t = 0; t < tiles.size(); t++) {
+                    roff[t] = q;
+                    q += tiles[t].nq1 + 1u;
+                }
+                CK(ctx->rtiles.ensure(sizeof(double) * (size_t)ta * TILE_QUARTER * (q + q / 8)));
+                CK(ctx->roff.ensure(4 * nt_room));
+                CK(cudaMemcpyAsync(ctx->roff.p, roff.data(), 4 * roff.size(), cudaMemcpyHostToDevice, up));
             } else {
                 CK(ctx->prow.ensure(sizeof(double) * (size_t)ta * nt_room));
                 CK(ctx->pcol.ensure(sizeof(double) * (size_t)tb * nt_room));
@@ -944,6 +983,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     ep.n_inv_sq_r2u_a = (1.0 / N) * (1.0 / N) * ep.r2u_a;
     ep.n_inv_sq = (1.0 / N) * (1.0 / N);
     ep.sketch_d = (double)d;
+    ep.n_used = N;
     ep.err = ctx->err.as<unsigned int>();
 
     // Whole-file INT8 runs with one annotation column overlap the band Gram
@@ -1113,6 +1153,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         if (rc != LDSC_OK) return rc;
         ep.left = ctx->left.as<int64_t>();
         ep.rtiles = (K > 1 && !tiles.empty()) ? ctx->rtiles.as<double>() : nullptr;
+        ep.roff = ctx->roff.as<uint32_t>();
         ep.prow = (K == 1 && !tiles.empty()) ? ctx->prow.as<double>() : nullptr;
         ep.pcol = (K == 1 && !tiles.empty()) ? ctx->pcol.as<double>() : nullptr;
     }
@@ -1123,21 +1164,29 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     if (!tiles.empty() && overlap) {
         // tiles are ordered by right block; chunk k's launch takes those whose
         // right block is complete once chunks [0, k] are decoded
+        // Launches alternate between two streams, so the next chunk's CTAs fill
+        // the SMs that a launch's last, partly filled wave leaves idle (the
+        // chunks' tiles are independent).
+        CK(cudaEventRecord(ctx->ovl_plan, s));
+        CK(cudaStreamWaitEvent(ctx->gram2, ctx->ovl_plan, 0));
         size_t t0 = 0;
         for (int k = 0; k < ov_n; k++) {
             const int64_t r1 = ov_b[k + 1];
+            cudaStream_t gs = k & 1 ? ctx->gram2 : s;
             size_t t1 = t0;
             while (t1 < tiles.size() && (r1 == m || (int64_t)(tiles[t1].b_blk + 1) * tb <= r1)) t1++;
             if (t1 == t0) continue;
-            CK(cudaStreamWaitEvent(s, ctx->ovl_ev[k], 0));
+            CK(cudaStreamWaitEvent(gs, ctx->ovl_ev[k], 0));
             EpilogueArgs ec = ep;  // this launch's tiles write their sums at their own tile indices
             ec.prow += t0 * ta;
             ec.pcol += t0 * tb;
             CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>() + t0, (int64_t)(t1 - t0), ec,
-                              nullptr, 0, ctx->sms, s));
+                              nullptr, 0, ctx->sms, gs));
             ctx->kernels++;
             t0 = t1;
         }
+        CK(cudaEventRecord(ctx->ovl_done, ctx->gram2));
+        CK(cudaStreamWaitEvent(s, ctx->ovl_done, 0));
     }
     // every record's statistics are final before the reduction reads them
     if (overlap) CK(cudaStreamWaitEvent(s, ctx->ovl_ev[ov_n - 1], 0));
@@ -1158,10 +1207,10 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         ctx->kernels++;
         e_c = ev.mark();
         if (K > 1) {
-            CK(launch_contract(ctx->rtiles.as<double>(), ta, tb, ctx->tiles.as<Tile>(), ctx->cptr_r.as<int32_t>(),
-                               ctx->cidx_r.as<int32_t>(), n_right, true, ep, s));
-            CK(launch_contract(ctx->rtiles.as<double>(), ta, tb, ctx->tiles.as<Tile>(), ctx->cptr_l.as<int32_t>(),
-                               ctx->cidx_l.as<int32_t>(), n_left, false, ep, s));
+            CK(launch_contract(ctx->tiles.as<Tile>(), ctx->cptr_r.as<int32_t>(), ctx->cidx_r.as<int32_t>(), n_right, true,
+                               ep, ctx->sms, s));
+            CK(launch_contract(ctx->tiles.as<Tile>(), ctx->cptr_l.as<int32_t>(), ctx->cidx_l.as<int32_t>(), n_left, false,
+                               ep, ctx->sms, s));
             ctx->kernels += 2;
         }
     }
@@ -1414,7 +1463,7 @@ int ldsc_debug_gram_i8_tile(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t k0,
     CK(launch_finalize_stats(m, n, st, nullptr, 1, 0, 0.0, ctx->aeff.as<double>(), ctx->l2.as<double>(), s));
     CK(cudaMemsetAsync(ctx->left.p, 0, 8 * (size_t)m, s));
     CK(cudaMemsetAsync(ctx->err.p, 0, 16, s));
-    Tile t{(uint32_t)(k0 / TILE_RECORDS), (uint32_t)(j0 / TILE_RECORDS)};
+    Tile t{(uint32_t)(k0 / TILE_RECORDS), (uint32_t)(j0 / TILE_RECORDS), 0, 3};
     const int dbg_row = (int)(k0 % TILE_RECORDS);
     CK(cudaMemcpyAsync(ctx->tiles.p, &t, sizeof(Tile), cudaMemcpyHostToDevice, s));
     EpilogueArgs ep{};
@@ -1428,6 +1477,7 @@ int ldsc_debug_gram_i8_tile(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t k0,
     ep.K = 1;
     ep.r2u_a = 1.0;
     ep.r2u_b = 0.0;
+    ep.n_used = (double)n;
     ep.err = ctx->err.as<unsigned int>();
     if (fused)
         CK(launch_gram_i8_packed(panel->rows, panel->pitch, n, m, ctx->tiles.as<Tile>(), 1, ep,

@@ -4,7 +4,7 @@
 // in both directions (src/l2/compute.rs:1869-1893, 2259-2314):
 //     l2[window] += R_ab * A_chunk,   l2[chunk] += R_ab^T * A_window (+ R_bb A_chunk).
 // Here the Gram kernels leave every band tile's masked r2u values in global
-// memory (f64, row j of the tile = TA values) and these passes do the two
+// memory (f64, row j of the tile = 128 values) and these passes do the two
 // products per block of rows: pass "by right block" owns l2 rows j of one
 // right block, pass "by left block" owns l2 rows k of one left block, so no
 // row is written by two CTAs of a pass and the summation order is fixed.
@@ -23,36 +23,38 @@ namespace {
 constexpr int NT = 256;  // threads of k_l2_reduce
 
 // The contraction on the FP64 tensor path (mma.sync m8n8k4 .f64):
-//   BY_RIGHT: out rows j of the right block, out[j][c] += sum_k R[k][j] A[k][c]
-//   BY_LEFT:  out rows k of the left block,  out[k][c] += sum_j R[k][j] A[j][c]
-// One CTA owns one output block and up to MK = 128 annotation columns (K > 128
-// runs column chunks).  The summed records of every tile of the block go by in
-// steps of JS_M = 32; a step's r2u values and the annotation values of its 32
-// records are staged by cp.async into one of two buffers while the MMAs run
-// on the other.  Warp (rg, cg) owns output rows 32 rg .. 32 rg + 31 and
-// columns 32 cg .. 32 cg + 31 of the chunk: 4 x 4 fragments of 8 x 8 f64
-// accumulators, eight k-steps of four records per staged step.  Fragment
-// layouts of m8n8k4 (row.col): A element (lane / 4, lane % 4), B element
-// (lane % 4, lane / 4), D elements (lane / 4, 2 (lane % 4) + {0, 1}).  Shared
-// rows are padded to a stride of 4 mod 16 doubles, so each half-warp's 16
-// 8-byte fragment loads hit 16 distinct bank pairs.
+//   BY_RIGHT: out rows j of the right block, out[j][c] += sum_k R[j][k] A[k][c]
+//   BY_LEFT:  out rows k of the left block,  out[k][c] += sum_j R[j][k] A[j][c]
+// One CTA owns one output block of 128 rows and up to MK = 128 annotation
+// columns (K > 128 runs column chunks).  The summed records of every tile of
+// the block go by in steps of JS = 32 (a quarter of the right block for
+// BY_LEFT, so quarters a tile leaves out cost nothing); a step's r2u values and
+// the annotation values of its 32 records are staged by cp.async into one of
+// two buffers while the MMAs run on the other.  Each of the 8 warps owns 16
+// output rows and all the chunk's columns: 2 x NF fragments of 8 x 8 f64
+// accumulators, eight k-steps of four records per staged step, so the 2 + NF
+// fragment loads of a k-step feed 2 NF MMAs and only about ceil(K / 8) fragments
+// are multiplied (a warp on 32 rows x 32 columns padded 97 columns to 128).  In a
+// BY_RIGHT step a warp whose rows the tile leaves out skips the MMAs.
+// The FP64 pipe bounds it (64 FMA per clock and SM):
+// 100,000 records x 97 columns, 2,892 tiles: 553 + 535 us against 574 + 567 us
+// with 32 x 32 warp tiles on the same tile list.
+// Fragment layouts of m8n8k4 (row.col): A element (lane / 4, lane % 4), B
+// element (lane % 4, lane / 4), D elements (lane / 4, 2 (lane % 4) + {0, 1}).
+// Shared rows are padded to a stride of 4 mod 16 doubles, so each half-warp's
+// 16 8-byte fragment loads hit 16 distinct bank pairs.
 constexpr int MK = 128;        // annotation columns per chunk
-constexpr int JS_M = 32;       // summed records per staged step
-constexpr int SLD = JS_M + 4;  // staged annotation stride (annotations are [column][record])
+constexpr int JS = 32;         // summed records per staged step
+constexpr int OB = TILE_RECORDS;
+constexpr int CTH = 256;       // threads
+constexpr int SLD = JS + 4;    // staged annotation stride (annotations are [column][record])
+constexpr int RLD_R = JS + 4;  // BY_RIGHT r2u stage [128 j][32 k]
+constexpr int RLD_L = OB + 4;  // BY_LEFT  r2u stage [32 j][128 k]
 
-template <int TA, int TB, bool BY_RIGHT>
-struct MmaShape {
-    static constexpr int OB = BY_RIGHT ? TB : TA;          // output rows per block
-    static constexpr int NS = BY_RIGHT ? TA : TB;          // summed records per tile
-    static constexpr int SPT = NS / JS_M;                  // staged steps per tile
-    static constexpr int WARPS = (OB / 32) * (MK / 32);
-    static constexpr int THREADS = 32 * WARPS;
-    // r2u stage: BY_RIGHT [TB j][JS_M k], BY_LEFT [JS_M j][TA k]
-    static constexpr int RLD = BY_RIGHT ? JS_M + 4 : TA + 4;
-    static constexpr int RROWS = BY_RIGHT ? TB : JS_M;
-    static constexpr int R_ELEMS = RROWS * RLD;
-    static constexpr int A_ELEMS = MK * SLD;
-    static constexpr int STAGE = R_ELEMS + A_ELEMS;          // doubles per buffer
+template <int NF, bool BY_RIGHT>
+struct ContractShape {
+    static constexpr int R_ELEMS = BY_RIGHT ? OB * RLD_R : JS * RLD_L;
+    static constexpr int STAGE = R_ELEMS + 8 * NF * SLD;   // doubles per buffer
     static constexpr size_t smem = sizeof(double) * 2 * (size_t)STAGE;
 };
 
@@ -77,16 +79,15 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-template <int TA, int TB, bool BY_RIGHT>
-__global__ void __launch_bounds__(MmaShape<TA, TB, BY_RIGHT>::THREADS)
-    k_contract_mma(const double* __restrict__ rtiles, const Tile* __restrict__ tiles,
-                   const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx, int32_t nblocks,
-                   EpilogueArgs ep) {
-    using S = MmaShape<TA, TB, BY_RIGHT>;
-    constexpr int NTH = S::THREADS, SPT = S::SPT, RLD = S::RLD, OB = S::OB;
+// NF: fragments of 8 columns per warp (the chunk has at most 8 NF columns;
+// results past it are not stored).
+template <int NF, bool BY_RIGHT>
+__global__ void __launch_bounds__(CTH)
+    k_contract_mma(const Tile* __restrict__ tiles, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+                   int32_t nblocks, EpilogueArgs ep) {
+    using S = ContractShape<NF, BY_RIGHT>;
     extern __shared__ __align__(16) double smm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rg = warp / (MK / 32), cg = warp % (MK / 32);
     const int K = ep.K;
     const int64_t m = ep.m;
     const int nchunks = (K + MK - 1) / MK;
@@ -95,90 +96,112 @@ __global__ void __launch_bounds__(MmaShape<TA, TB, BY_RIGHT>::THREADS)
     for (int64_t w = blockIdx.x; w < (int64_t)nblocks * nchunks; w += gridDim.x) {
         const int32_t blk = (int32_t)(w / nchunks);
         const int c0 = (int)(w % nchunks) * MK;
+        const int kc = K - c0 < MK ? K - c0 : MK;   // columns of this chunk
         const int32_t t0 = ptr[blk], t1 = ptr[blk + 1];
-        const int nsteps = (t1 - t0) * SPT;
-        if (nsteps == 0) continue;
-        const bool active = c0 + 32 * cg < K;  // warp-uniform: any of this warp's columns in range
+        if (t0 == t1) continue;
 
-        // stage step st into buffer b
-        auto issue = [&](int st, int b) {
-            const int32_t t = idx[t0 + st / SPT];
-            const int js = (st % SPT) * JS_M;
+        // the staged steps run over the block's tiles: cursor (tile entry, step in it)
+        struct Cursor {
+            int32_t e;
+            int st;
+        };
+        auto steps_of = [&](const Tile& tl) { return BY_RIGHT ? OB / JS : (int)tl.nq1 + 1; };
+        auto issue = [&](const Cursor& cu, int b) {
+            const int32_t t = idx[cu.e];
             const Tile tl = tiles[t];
-            const double* src = rtiles + (size_t)t * TA * TB;
+            const double* src = ep.rtiles + (size_t)ep.roff[t] * TILE_QUARTER * OB;
             double* Rs = smm + b * S::STAGE;
             double* As = Rs + S::R_ELEMS;
             if (BY_RIGHT) {
-                // all TB rows j, values k = js .. js + 31: 16-byte pieces
-#pragma unroll
-                for (int q = tid; q < TB * JS_M / 2; q += NTH) {
-                    const int r = q / (JS_M / 2), cc = 2 * (q % (JS_M / 2));
-                    cp_async16(Rs + r * RLD + cc, src + (size_t)r * TA + js + cc);
+                // the tile's rows j, values k = 32 st .. 32 st + 31: 16-byte pieces
+                const int n = ((int)tl.nq1 + 1) * TILE_QUARTER;
+                double* dst = Rs + (int)tl.q0 * TILE_QUARTER * RLD_R;
+                for (int q = tid; q < n * JS / 2; q += CTH) {
+                    const int r = q / (JS / 2), cc = 2 * (q % (JS / 2));
+                    cp_async16(dst + r * RLD_R + cc, src + (size_t)r * OB + cu.st * JS + cc);
                 }
             } else {
-                // rows j = js .. js + 31, all TA values
+                // 32 rows j of the tile's quarter st, all 128 values
+                const double* q0 = src + (size_t)cu.st * JS * OB;
 #pragma unroll
-                for (int q = tid; q < JS_M * TA / 2; q += NTH) {
-                    const int r = q / (TA / 2), cc = 2 * (q % (TA / 2));
-                    cp_async16(Rs + r * RLD + cc, src + (size_t)(js + r) * TA + cc);
+                for (int q = tid; q < JS * OB / 2; q += CTH) {
+                    const int r = q / (OB / 2), cc = 2 * (q % (OB / 2));
+                    cp_async16(Rs + r * RLD_L + cc, q0 + (size_t)r * OB + cc);
                 }
             }
             // annotation column c0 + c of summed record s at aeff[s + (c0 + c) m]; consecutive threads
             // take consecutive records (coalesced), zeros past m or K
-            const int64_t s0 = (BY_RIGHT ? (int64_t)tl.a_blk * TA : (int64_t)tl.b_blk * TB) + js;
-#pragma unroll
-            for (int e = tid; e < MK * JS_M; e += NTH) {
-                const int s = e & (JS_M - 1), c = e / JS_M;
-                const bool ok = s0 + s < m && c0 + c < K;
+            const int64_t s0 = BY_RIGHT ? (int64_t)tl.a_blk * OB + cu.st * JS
+                                        : (int64_t)tl.b_blk * OB + ((int)tl.q0 + cu.st) * TILE_QUARTER;
+            for (int e = tid; e < 8 * NF * JS; e += CTH) {
+                const int s = e & (JS - 1), c = e / JS;
+                const bool ok = s0 + s < m && c < kc;
                 cp_async8_zfill(As + c * SLD + s, ok ? ep.aeff + (s0 + s) + (int64_t)(c0 + c) * m : ep.aeff, ok);
             }
         };
+        auto advance = [&](Cursor& cu) {
+            if (++cu.st == steps_of(tiles[idx[cu.e]])) {
+                cu.st = 0;
+                cu.e++;
+            }
+        };
 
-        double acc[4][4][2];
+        double acc[2][NF][2];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < 2; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+            for (int j = 0; j < NF; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-        issue(0, 0);
+        Cursor cur{t0, 0}, nxt{t0, 0};
+        issue(nxt, 0);
+        advance(nxt);
         cp_async_commit();
-        for (int st = 0; st < nsteps; st++) {
-            if (st + 1 < nsteps) issue(st + 1, (st + 1) & 1);
+        for (int b = 0; cur.e < t1; b ^= 1) {
+            if (nxt.e < t1) {
+                issue(nxt, b ^ 1);
+                advance(nxt);
+            }
             cp_async_commit();
-            cp_async_wait1();  // step st's copies (this thread's) have landed
+            cp_async_wait1();  // the current step's copies (this thread's) have landed
             __syncthreads();   // ... and every thread's
+            bool active = true;   // warp-uniform
+            if (BY_RIGHT) {
+                const Tile tl = tiles[idx[cur.e]];
+                const int quarter = warp >> 1;
+                active = quarter >= (int)tl.q0 && quarter <= (int)(tl.q0 + tl.nq1);
+            }
             if (active) {
-                const double* Rs = smm + (st & 1) * S::STAGE;
+                const double* Rs = smm + b * S::STAGE;
                 const double* As = Rs + S::R_ELEMS;
+#pragma unroll 2
+                for (int kk = 0; kk < JS; kk += 4) {
+                    double a[2];
 #pragma unroll
-                for (int kk = 0; kk < JS_M; kk += 4) {
-                    double a[4], b[4];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int orow = 32 * rg + 8 * i + fr;  // output row of the fragment
-                        a[i] = BY_RIGHT ? Rs[orow * RLD + kk + fc] : Rs[(kk + fc) * RLD + orow];
+                    for (int i = 0; i < 2; i++) {
+                        const int orow = 16 * warp + 8 * i + fr;  // output row of the fragment
+                        a[i] = BY_RIGHT ? Rs[orow * RLD_R + kk + fc] : Rs[(kk + fc) * RLD_L + orow];
                     }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) b[j] = As[(32 * cg + 8 * j + fr) * SLD + kk + fc];
+                    for (int j = 0; j < NF; j++) {
+                        const double bj = As[(8 * j + fr) * SLD + kk + fc];
 #pragma unroll
-                    for (int i = 0; i < 4; i++)
-#pragma unroll
-                        for (int j = 0; j < 4; j++) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+                        for (int i = 0; i < 2; i++) dmma(acc[i][j][0], acc[i][j][1], a[i], bj);
+                    }
                 }
             }
-            __syncthreads();  // buffer st & 1 is refilled by the next iteration's issue
+            __syncthreads();  // this buffer is refilled by the next iteration's issue
+            advance(cur);
         }
-        if (!active) continue;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int64_t row = (int64_t)blk * OB + 32 * rg + 8 * i + fr;
+        for (int i = 0; i < 2; i++) {
+            const int64_t row = (int64_t)blk * OB + 16 * warp + 8 * i + fr;
             if (row >= m) continue;
 #pragma unroll
-            for (int j = 0; j < 4; j++)
+            for (int j = 0; j < NF; j++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const int c = c0 + 32 * cg + 8 * j + 2 * fc + h;
-                    if (c < K) ep.l2[row + (int64_t)c * m] += acc[i][j][h];
+                    const int c = 8 * j + 2 * fc + h;
+                    if (c < kc) ep.l2[row + (int64_t)(c0 + c) * m] += acc[i][j][h];
                 }
         }
     }
@@ -211,29 +234,51 @@ cudaError_t launch_l2_reduce(int64_t m, int ta, int tb, const int32_t* ptr_r, co
     return cudaGetLastError();
 }
 
-cudaError_t launch_contract(const double* rtiles, int ta, int tb, const Tile* tiles, const int32_t* ptr,
-                            const int32_t* idx, int32_t nblocks, bool by_right, const EpilogueArgs& ep,
-                            cudaStream_t stream) {
+template <int NF, bool BY_RIGHT>
+static cudaError_t run_contract(const Tile* tiles, const int32_t* ptr, const int32_t* idx, int32_t nblocks,
+                                const EpilogueArgs& ep, int sms, cudaStream_t stream) {
+    const size_t smem = ContractShape<NF, BY_RIGHT>::smem;
+    cudaError_t e =
+        cudaFuncSetAttribute(k_contract_mma<NF, BY_RIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int64_t work = (int64_t)nblocks * ((ep.K + MK - 1) / MK), cap = (int64_t)sms * (NF <= 7 ? 2 : 1);
+    k_contract_mma<NF, BY_RIGHT><<<(unsigned)(work < cap ? work : cap), CTH, smem, stream>>>(tiles, ptr, idx, nblocks, ep);
+    return cudaGetLastError();
+}
+
+// Fragments per warp by the columns of a chunk: every fragment is multiplied,
+// so the sizes are close together (K = 97 runs 13, a 53-annotation model 7).
+cudaError_t launch_contract(const Tile* tiles, const int32_t* ptr, const int32_t* idx, int32_t nblocks, bool by_right,
+                            const EpilogueArgs& ep, int sms, cudaStream_t stream) {
     if (nblocks <= 0) return cudaSuccess;
-    const int64_t work = (int64_t)nblocks * ((ep.K + MK - 1) / MK);
-    auto go = [&](auto kern, size_t smem, int threads) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        // 512-thread CTAs (141 - 147 KB): one per SM; 256-thread CTAs (111 KB): two
-        const int64_t cap = (int64_t)148 * (threads <= 256 ? 2 : 1);
-        kern<<<(unsigned)(work < cap ? work : cap), threads, smem, stream>>>(rtiles, tiles, ptr, idx, nblocks, ep);
-        return cudaGetLastError();
-    };
-#define LDSC_CONTRACT(TA_, TB_, BR_) \
-    go(k_contract_mma<TA_, TB_, BR_>, MmaShape<TA_, TB_, BR_>::smem, MmaShape<TA_, TB_, BR_>::THREADS)
-    if (ta == 128 && tb == 128) return by_right ? LDSC_CONTRACT(128, 128, true) : LDSC_CONTRACT(128, 128, false);
+#define LDSC_CONTRACT(NF_)                                                                        \
+    (by_right ? run_contract<NF_, true>(tiles, ptr, idx, nblocks, ep, sms, stream)               \
+              : run_contract<NF_, false>(tiles, ptr, idx, nblocks, ep, sms, stream))
+    if (ep.K <= 8) return LDSC_CONTRACT(1);
+    if (ep.K <= 16) return LDSC_CONTRACT(2);
+    if (ep.K <= 32) return LDSC_CONTRACT(4);
+    if (ep.K <= 56) return LDSC_CONTRACT(7);
+    if (ep.K <= 80) return LDSC_CONTRACT(10);
+    if (ep.K <= 104) return LDSC_CONTRACT(13);
+    return LDSC_CONTRACT(16);
 #undef LDSC_CONTRACT
-    return cudaErrorInvalidValue;
 }
 
 cudaError_t preload_contract() {
-    cudaError_t e = preload_kernel(k_contract_mma<128, 128, true>);
-    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<128, 128, false>);
+    cudaError_t e = preload_kernel(k_contract_mma<1, true>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<1, false>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<2, true>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<2, false>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<4, true>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<4, false>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<7, true>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<7, false>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<10, true>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<10, false>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<13, true>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<13, false>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<16, true>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_mma<16, false>);
     if (e == cudaSuccess) e = preload_kernel(k_l2_reduce);
     return e;
 }

@@ -260,7 +260,9 @@ cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st, cons
                                   int32_t K, int has_pq, double pq_exp, double* aeff,
                                   double* l2_init, cudaStream_t stream, uint64_t annot_ld) {
     if (m <= 0) return cudaSuccess;
-    k_finalize<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(m, n_indiv, st, annot,
+    // blocks of 64: in an overlapped run the SMs are held by the Gram, and a block
+    // of 256 does not find its registers there until a Gram CTA ends
+    k_finalize<<<(unsigned)((m + 63) / 64), 64, 0, stream>>>(m, n_indiv, st, annot,
                                                               annot_ld ? annot_ld : (uint64_t)m, K, has_pq,
                                                               pq_exp, aeff, l2_init);
     return cudaGetLastError();

@@ -42,10 +42,15 @@ struct RecStats {
 // Records per side of a band tile (left block x right block), every form.
 constexpr int TILE_RECORDS = 128;
 
-// Band tile: A block (k side, left SNPs) x B block (j side, right SNPs).
+constexpr int TILE_QUARTER = TILE_RECORDS / 4;
+
+// Band tile: the 128 left records of A block a_blk against the right records
+// of quarters [q0, q0 + nq1 + 1) (32 records each) of B block b_blk.
 struct Tile {
     uint32_t a_blk;
-    uint32_t b_blk;
+    uint32_t b_blk : 28;
+    uint32_t q0 : 2;
+    uint32_t nq1 : 2;
 };
 
 // Everything the Gram epilogues need.
@@ -64,8 +69,12 @@ struct EpilogueArgs {
     double n_inv_sq_r2u_a;    // r2u_a / N^2   (FP64 form)
     double n_inv_sq;          // 1 / N^2       (sketch form)
     double sketch_d;          // d as double   (sketch form)
+    double n_used;            // individuals
     unsigned int* err;        // device error word (non-zero = a bounded wait gave up)
-    double* rtiles;           // K > 1: tile t's masked r2u values, tb rows (j) x ta (k) f64 at t * ta * tb
+    // K > 1: tile t's masked r2u values, its right records (rows j) x 128 left
+    // records (k) in f64, from quarter roff[t] (32 x 128 values each) of rtiles
+    double* rtiles;
+    const uint32_t* roff;
     // K = 1: tile t's row sums (ta values at prow + t * ta: sum_j r2u a_j for
     // each left record k) and column sums (tb values at pcol + t * tb), added
     // to l2 in a fixed order by launch_l2_reduce; null = atomics into l2
@@ -101,6 +110,10 @@ cudaError_t launch_decode_f64(const PanelView& p, const uint64_t* rec_rows, int6
 cudaError_t launch_gram_f64(const double* x, uint64_t ld, uint64_t kdim, const Tile* tiles,
                             int64_t n_tiles, const EpilogueArgs& ep, int sms,
                             cudaStream_t stream);
+
+// Whether a tcgen05 Gram over operand rows of row_bytes gains from tiles
+// trimmed to the right records they need (gram_tiles, plan.h).
+bool gram_trims(uint64_t row_bytes);
 
 // INT8 tcgen05 band Gram + exact epilogue (128 x 128 records per tile).
 // ops: 2*m rows of `ld` bytes.  dbg (optional) receives the raw accumulators
@@ -159,13 +172,12 @@ cudaError_t launch_gram_f32(const float* x, uint64_t ld, uint64_t kdim, const Ti
                             cudaStream_t stream);
 
 // K > 1 annotation contraction from the R tiles a Gram wrote (no atomics, each
-// l2 row owned by one CTA per pass):
+// l2 row owned by one CTA per pass), ep.rtiles / ep.roff:
 //   by right block:  l2[j, C] += sum over tiles of block, sum_k R[k][j] a[k, C]
 //   by left block:   l2[k, C] += sum over tiles of block, sum_j R[k][j] a[j, C]
 // ptr/idx: CSR lists of tile indices per right block (by_right) or per left block.
-cudaError_t launch_contract(const double* rtiles, int ta, int tb, const Tile* tiles, const int32_t* ptr,
-                            const int32_t* idx, int32_t nblocks, bool by_right, const EpilogueArgs& ep,
-                            cudaStream_t stream);
+cudaError_t launch_contract(const Tile* tiles, const int32_t* ptr, const int32_t* idx, int32_t nblocks, bool by_right,
+                            const EpilogueArgs& ep, int sms, cudaStream_t stream);
 
 // Load a kernel's code on the current device now.  With lazy module loading
 // (the CUDA 12 default) a kernel is loaded at its first launch, which can

@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(NT, 1)
         } else {
             // K > 1: the masked r2u tile goes to global memory in f64 (row j of
             // TA values) for the banded annotation contraction (contract.cu)
-            double* dst = ep.rtiles + (size_t)t * TA * TB;
+            double* dst = ep.rtiles + (size_t)ep.roff[t] * TILE_QUARTER * TA;
+            const int q_lo = (int)tl.q0 * TILE_QUARTER, q_n = ((int)tl.nq1 + 1) * TILE_QUARTER;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int64_t k = k0 + ty + 16 * i;
@@ -172,7 +173,8 @@ __global__ void __launch_bounds__(NT, 1)
                     const int64_t j = j0 + tx + 16 * l;
                     double r = 0.0;
                     if (pair_in_band(k, j, m, ep.left)) r = correct<MODE>((double)acc[i][l], k, j, ep);
-                    dst[(tx + 16 * l) * TA + ty + 16 * i] = r;
+                    const int jr = tx + 16 * l - q_lo;
+                    if (jr >= 0 && jr < q_n) dst[jr * TA + ty + 16 * i] = r;
                 }
             }
         }

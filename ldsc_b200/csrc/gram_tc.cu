@@ -20,8 +20,8 @@
 // With n, s, q the per-record non-missing count, genotype sum and sum of
 // squares, the reference's standardised dot product (normalize.rs:71-110
 // followed by the A^T B GEMM, compute.rs:1897-2236) is recovered exactly:
-//     X   = n_k (n_j GG - s_j GM) - s_k (n_j MG - s_j MM)         (int64, exact)
-//     r   = X / sqrt(n_k V_k n_j V_j),  V = n q - s^2            (f64)
+//     X   = n_k (n_j GG - s_j GM) + s_k (s_j MM - n_j MG)         (int64, exact)
+//     r^2 = X^2 / (n_k V_k n_j V_j),  V = n q - s^2              (f64)
 //     r2u = r^2 (1 + 1/(N-2)) - 1/(N-2)                           (f64)
 // N cancels from r; a monomorphic record (V = 0) gives r = 0 and
 // r2u = -1/(N-2), as the reference's zero inv_std does.
@@ -46,14 +46,21 @@
 //              r; the right records' constants are read as broadcasts from
 //              shared memory, a row's sum stays in its thread, and a column's
 //              sum over the warp's 32 rows is a transposing butterfly (9 f64
-//              shuffles per 8 columns).  At sketch d = 200, where the
-//              epilogue outweighs the MMAs, 100,000 x 50,000 went from 715 to
-//              409 us against row / column pairs exchanged between lanes.
+//              shuffles per 8 columns).  f64 instructions and tcgen05.mma share
+//              one pipe of the SM (an f64 instruction beside running MMAs waits
+//              about 20 clocks), so they are kept few: five per pair in a block
+//              that lies inside the band (X to double, X^2, row and column
+//              terms, butterfly), with 1/(nV) of the row, the column and the
+//              constant -1/(N-2) applied to the sums: about 10,000
+//              clocks per tile (sketch: 19,000, f32 square root and division per
+//              pair), 13 f64 instructions per pair before.
 //              With K > 1 annotation columns the epilogue stores each tile's
 //              masked r2u values (f64, [j][k]) for the contraction of
 //              contract.cu.
 // The accumulators fill TMEM, so a tile's epilogue does not overlap the next
-// tile's MMAs (its loads do).
+// tile's MMAs (its loads do).  Half tiles (64 right records) with two
+// accumulator buffers were slower even at 7 K steps: the epilogue's f64
+// instructions then wait for the other buffer's MMAs.
 //
 // Fused INT8 form (the operand rows are never written to HBM): warp 0 stages
 // the packed 2-bit BED rows themselves by TMA -- 32 bytes per record per 128
@@ -70,6 +77,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "engine.h"
 #include "epilogue.cuh"
 #include "expand.cuh"
@@ -82,6 +91,7 @@ namespace {
 constexpr int TA = 128;            // left records per tile
 constexpr int TB = 128;            // right records per tile
 constexpr int HALF = 128 * 128;    // 128 operand rows (one kind) x 128 bytes
+constexpr int QROWS = TILE_QUARTER * 128;   // 32 operand rows x 128 bytes
 constexpr int A_BYTES = 2 * HALF;  // one stage of A: G rows, then M rows
 constexpr int B_BYTES = 2 * HALF;
 // fused form: packed ring of 2-bit rows, 128 individuals (32 bytes) per record per stage
@@ -91,9 +101,17 @@ constexpr int P_BYTES = (TA + TB) * 32;
 // operand stages, epilogue and converter warps of the two forms (576 threads
 // either way); the fused form's packed ring leaves room for two operand stages
 constexpr int STAGES_TMA = 3, EPI_TMA = 16;
+// Long rows (from LONG_STEPS K steps) run 8 epilogue warps: the epilogue is a
+// few percent there, and 320 threads leave the registers for three blocks of
+// the decode that runs beside the Gram (576 threads: one).  At 50,000 x
+// 100,000 with whole tiles a pass took 13.22 ms on the device, with 16 epilogue
+// warps 13.39 ms.
+constexpr int EPI_LONG = 8, LONG_STEPS = 200;
 constexpr int STAGES_FUSED = 2, EPI_FUSED = 8, CONV_FUSED = 8;
 // threads per CTA: TMA and MMA warps + ew epilogue warps + cw converter warps
 __host__ __device__ constexpr int gram_threads(int ew, int cw) { return 64 + 32 * ew + 32 * cw; }
+// every form is compiled for the 576 threads of the widest (112 registers at most)
+constexpr int GRAM_BOUND = 576;
 constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;  // 2 s per wait
 
 // Sums over the warp's 32 lanes of 8 values per lane: lane l ends with the sum
@@ -115,12 +133,29 @@ __device__ __forceinline__ double transpose_sum8(const double (&c)[8], int lane)
     return f;
 }
 
-// Right-record constants of the tile being finished.
-struct ColConst {
-    double2 qa[TB];     // (INT8: qinv | sketch: kappa), effective annotation (K = 1)
-    int2 ns[TB];        // INT8: non-missing count, genotype sum
-    int64_t left[TB];   // left limit (m past the last record)
+template <typename T>
+__device__ __forceinline__ T warp_sum(T v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    return v;
+}
+
+// Right-record constants and partial sums of the tile being finished
+// (double-buffered: a tile's sums leave while the next tile starts).
+struct EpiTile {
+    double2 qa[TB];        // (INT8: 1 / (n V) | sketch: kappa), effective annotation (K = 1)
+    double qw[TB];         // INT8: 1 / (n V) x effective annotation
+    int4 ns[TB];           // INT8: n, -s, s, -n (non-missing count, genotype sum)
+    int64_t left[TB];      // left limit (m past the last record)
+    double cpart[4][TB];   // column sums per TMEM lane quarter
+    double rpart[4][TA];   // row sums per column group
 };
+
+// 1.5 * 2^52: an integer |x| < 2^51 plus its bits, read as a double, is this
+// constant plus x exactly.
+constexpr uint64_t INT_MAGIC = 0x4338000000000000ull;
+// X fits that way while n^3 < 2^51 (|X| <= n_k V_k n_j V_j's root <= N^3)
+constexpr double MAGIC_MAX_N = 131072.0;
 
 // MODE 0: INT8 exact r^2; 1: TF32 sketch, quadratic correction; 2: same, MAF-aware.
 // kap: kappa_k + kappa_j (MAF-aware).
@@ -163,8 +198,8 @@ __device__ __forceinline__ float sketch_r2u_f32(float val, double kap2, const Sk
 // rows staged by TMA (the map covers the BED rows, boxes of 32 bytes x 128
 // rows) and expanded by CW converter warps; n_indiv masks the last stage.
 template <int STAGES, int MODE, int EW, int CW>
-__global__ void __launch_bounds__(gram_threads(EW, CW), 1)
-    k_gram_tc(const __grid_constant__ CUtensorMap tm, int num_kb, const Tile* __restrict__ tiles, int64_t n_tiles,
+__global__ void __launch_bounds__(GRAM_BOUND, 1)
+    k_gram_tc(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tmq, int num_kb, const Tile* __restrict__ tiles, int64_t n_tiles,
               EpilogueArgs ep, int32_t* __restrict__ dbg, int dbg_row, uint64_t n_indiv) {
     static_assert(CW == 0 || MODE == 0, "the fused form is INT8 only");
     // elements per 128-byte stage row: 128 (INT8) or 32 (TF32); TMA x is in elements
@@ -185,9 +220,7 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     // 16-byte aligned: the barriers above take an even number of 8-byte words
     static_assert((2 * STAGES + 2 * P_STAGES + 4) % 2 == 0, "alignment of the epilogue arrays");
-    ColConst& cc = *reinterpret_cast<ColConst*>(drain + 2);
-    double* cpart = reinterpret_cast<double*>(&cc + 1);    // [4][TB]: column sums per TMEM lane quarter
-    double* rpart = cpart + 4 * TB;                         // [4][TA]: row sums per group of 32 columns
+    EpiTile* epi = reinterpret_cast<EpiTile*>(drain + 2);   // [2]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -218,6 +251,7 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
         // ------------------------------------------------ TMA producer
         if (elect_one_sync()) {
             tma_prefetch_desc(&tm);
+            if (CW == 0) tma_prefetch_desc(&tmq);
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -229,7 +263,8 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
             uint64_t* rempty = CW > 0 ? pempty : empty;
             for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
                 const Tile tl = tiles[t];
-                const int32_t ra = (int32_t)tl.a_blk * TA, rb = (int32_t)tl.b_blk * TB;
+                const int nq = (int)tl.nq1 + 1;
+                const int32_t ra = (int32_t)tl.a_blk * TA, rb = (int32_t)(tl.b_blk * TB + tl.q0 * TILE_QUARTER);
                 for (int kb = 0; kb < num_kb; kb++) {
                     if (!mbar_wait(&rempty[stage], phase ^ 1, WAIT_LIMIT_NS)) {
                         ok = false;
@@ -240,13 +275,21 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
                         tma_load_2d(sP + stage * P_BYTES, &tm, &rfull[stage], kb * 32, ra);
                         tma_load_2d(sP + stage * P_BYTES + PA_BYTES, &tm, &rfull[stage], kb * 32, rb);
                     } else {
-                        mbar_arrive_expect_tx(&rfull[stage], A_BYTES + B_BYTES);
+                        mbar_arrive_expect_tx(&rfull[stage], A_BYTES + nq * 2 * QROWS);
                         uint8_t* da = sA + stage * A_BYTES;
                         uint8_t* db = sB + stage * B_BYTES;
                         tma_load_3d(da, &tm, &rfull[stage], kb * KSTEP, 0, ra);
                         tma_load_3d(da + HALF, &tm, &rfull[stage], kb * KSTEP, 1, ra);
-                        tma_load_3d(db, &tm, &rfull[stage], kb * KSTEP, 0, rb);
-                        tma_load_3d(db + HALF, &tm, &rfull[stage], kb * KSTEP, 1, rb);
+                        if (nq == 4) {
+                            tma_load_3d(db, &tm, &rfull[stage], kb * KSTEP, 0, rb);
+                            tma_load_3d(db + HALF, &tm, &rfull[stage], kb * KSTEP, 1, rb);
+                        } else {   // the tile's quarters of the right block only
+                            for (int q = 0; q < nq; q++) {
+                                tma_load_3d(db + q * QROWS, &tmq, &rfull[stage], kb * KSTEP, 0, rb + q * TILE_QUARTER);
+                                tma_load_3d(db + (nq + q) * QROWS, &tmq, &rfull[stage], kb * KSTEP, 1,
+                                            rb + q * TILE_QUARTER);
+                            }
+                        }
                     }
                     armed |= 1u << stage;
                     armed_par = (armed_par & ~(1u << stage)) | (phase << stage);
@@ -266,7 +309,6 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
     } else if (warp == 1) {
         // ------------------------------------------------ UMMA issuer
         if (elect_one_sync()) {
-            const uint32_t idesc = MODE == 0 ? idesc_i8(128, 256) : idesc_tf32(128, 256);
             int stage = 0;
             uint32_t phase = 0, aphase = 0;
             bool ok = true;
@@ -277,6 +319,8 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
                     break;
                 }
                 tc_fence_after();
+                const uint32_t n2 = 64u * (tiles[t].nq1 + 1);   // the tile's right G rows and M rows
+                const uint32_t idesc = MODE == 0 ? idesc_i8(128, n2) : idesc_tf32(128, n2);
                 for (int kb = 0; kb < num_kb; kb++) {
                     if (!mbar_wait(&full[stage], phase, WAIT_LIMIT_NS)) {
                         ok = false;
@@ -292,10 +336,11 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
                             const uint64_t da = sdesc_k_sw128(a_addr + h * HALF + kk * 32);
                             const uint64_t db = sdesc_k_sw128(b_addr + kk * 32);
                             const uint32_t acc = (kb | kk) != 0 ? 1u : 0u;
+                            const uint32_t d_tmem = tmem_base + h * 256u;
                             if (MODE == 0)
-                                umma_i8(tmem_base + h * 256u, da, db, idesc, acc);
+                                umma_i8(d_tmem, da, db, idesc, acc);
                             else
-                                umma_tf32(tmem_base + h * 256u, da, db, idesc, acc);
+                                umma_tf32(d_tmem, da, db, idesc, acc);
                         }
                     }
                     issued = true;
@@ -325,7 +370,7 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
         constexpr int RPP = 32 * (CW > 0 ? CW : 1) / 8;   // records per pass
         constexpr int NPASS = (TA + TB) / RPP;
         constexpr int APASS = TA / RPP;              // passes that fill the A tile
-        static_assert((TA + TB) % RPP == 0 && TA % RPP == 0, "converter passes");
+        static_assert(CW == 0 || (RPP == TILE_QUARTER && TA % RPP == 0), "converter passes");
         const int ct = threadIdx.x - (64 + 32 * EW);
         const int wd = ct & 7;
         uint32_t offP[NPASS], offG[NPASS];
@@ -341,11 +386,13 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
         for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
             // records past the last one read as missing (the map's zero fill would read as genotype 2)
             const Tile tl = tiles[t];
+            const int nq = (int)tl.nq1 + 1;   // the right block's quarters; pass APASS + q fills quarter q
             uint32_t live = 0;
 #pragma unroll
             for (int i = 0; i < NPASS; i++) {
                 const int rr = (ct >> 3) + RPP * i;
-                const int64_t rec = i < APASS ? (int64_t)tl.a_blk * TA + rr : (int64_t)tl.b_blk * TB + (rr - TA);
+                const int64_t rec = i < APASS ? (int64_t)tl.a_blk * TA + rr
+                                              : (int64_t)tl.b_blk * TB + tl.q0 * TILE_QUARTER + (rr - TA);
                 live |= (rec < ep.m ? 1u : 0u) << i;
             }
             for (int kb = 0; kb < num_kb; kb++) {
@@ -374,11 +421,12 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
                 }
 #pragma unroll
                 for (int i = 0; i < NPASS; i++) {
+                    if (i >= APASS + nq) break;
                     uint4 g, mk;
                     expand_chunk(w[i], g, mk);
                     uint8_t* base = i < APASS ? oa : ob;
                     *reinterpret_cast<uint4*>(base + offG[i]) = g;
-                    *reinterpret_cast<uint4*>(base + HALF + offG[i]) = mk;
+                    *reinterpret_cast<uint4*>(base + (i < APASS ? HALF : nq * QROWS) + offG[i]) = mk;
                 }
                 // the generic-proxy stores must be visible to the tensor core's async proxy
                 fence_proxy_async_smem();
@@ -400,7 +448,7 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
     } else {
         // ------------------------------------------------ epilogue
         constexpr int EPI_T = 32 * EW;           // epilogue threads
-        constexpr int NG = 16 / EW;              // groups of 32 columns per warp
+        constexpr int NG = 16 / EW;              // column groups (quarters of the tile's columns) per warp
         const int et = threadIdx.x - 64;         // 0..EPI_T-1
         const int ew = et >> 5;                  // epilogue warp
         const int quarter = warp & 3;            // TMEM lanes this warp may access
@@ -409,23 +457,35 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
         const int64_t m = ep.m;
         const SketchF cf{(float)ep.n_inv_sq, (float)ep.sketch_d, (float)ep.r2u_a, (float)ep.r2u_b};
         const bool f32_corr = MODE != 0 && ep.sketch_d >= 8.0;
-        uint32_t aphase = 0;
-        for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        const bool big = ep.n_used >= MAGIC_MAX_N;
+        const uint64_t magic = big ? 0ull : INT_MAGIC;
+        uint32_t aphase = 0, flip = 0;
+        for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, flip ^= 1) {
+            EpiTile& E = epi[flip];
             const Tile tl = tiles[t];
-            const int64_t k0 = (int64_t)tl.a_blk * TA, j0 = (int64_t)tl.b_blk * TB;
+            const int nq = (int)tl.nq1 + 1, ncol = nq * TILE_QUARTER;
+            const int64_t k0 = (int64_t)tl.a_blk * TA, j0 = (int64_t)tl.b_blk * TB + tl.q0 * TILE_QUARTER;
             const int64_t k = k0 + row;
             const bool kval = k < m;
             const uint32_t nk = (MODE == 0 && kval) ? (uint32_t)__ldg(ep.n + k) : 0u;
             const uint32_t sk = (MODE == 0 && kval) ? (uint32_t)__ldg(ep.s + k) : 0u;
-            const double qk = !kval ? 0.0 : (MODE == 0 ? __ldg(ep.qinv + k) : (MODE == 2 ? __ldg(ep.kappa + k) : 0.0));
+            // INT8: 1 / (n V) of the left record; MAF-aware sketch: its kappa
+            double qk = !kval ? 0.0 : (MODE == 0 ? __ldg(ep.qinv + k) : (MODE == 2 ? __ldg(ep.kappa + k) : 0.0));
+            if (MODE == 0) qk *= qk;
             const double ak = (kval && ep.K == 1) ? __ldg(ep.aeff + k) : 0.0;
             if (et < TB) {   // the right records' constants, while the tile's MMAs run
                 const int64_t j = j0 + et;
-                const bool jv = j < m;
-                const double qj = !jv ? 0.0 : (MODE == 0 ? __ldg(ep.qinv + j) : (MODE == 2 ? __ldg(ep.kappa + j) : 0.0));
-                cc.qa[et] = make_double2(qj, (jv && ep.K == 1) ? __ldg(ep.aeff + j) : 0.0);
-                if (MODE == 0) cc.ns[et] = jv ? make_int2(__ldg(ep.n + j), __ldg(ep.s + j)) : make_int2(0, 0);
-                cc.left[et] = jv ? __ldg(ep.left + j) : m;
+                const bool jv = et < ncol && j < m;
+                double qj = !jv ? 0.0 : (MODE == 0 ? __ldg(ep.qinv + j) : (MODE == 2 ? __ldg(ep.kappa + j) : 0.0));
+                if (MODE == 0) qj *= qj;
+                const double aj = (jv && ep.K == 1) ? __ldg(ep.aeff + j) : 0.0;
+                E.qa[et] = make_double2(qj, aj);
+                if (MODE == 0) E.qw[et] = qj * aj;
+                if (MODE == 0) {
+                    const int nj = jv ? __ldg(ep.n + j) : 0, sj = jv ? __ldg(ep.s + j) : 0;
+                    E.ns[et] = make_int4(nj, -sj, sj, -nj);
+                }
+                E.left[et] = jv ? __ldg(ep.left + j) : m;
             }
 
             // One thread does the bounded wait; the decision is made uniform for
@@ -438,107 +498,146 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
                 if (et == 0) atomicOr(ep.err, 4u);
                 break;
             }
-            aphase ^= 1;
             tc_fence_after();
+            aphase ^= 1;
+            const double a_rows = ep.K == 1 ? warp_sum(ak) : 0.0;   // annotation sum of the warp's rows
 #pragma unroll 1
             for (int g = 0; g < NG; g++) {
-                const int cg = (ew >> 2) * NG + g, c0 = cg * 32;   // columns [c0, c0 + 32) of the tile
-                // does the warp's 32 x 32 block hold any in-band pair, or only in-band pairs?
+                const int cg = (ew >> 2) * NG + g, c0 = cg * 8 * nq;   // columns [c0, c0 + 8 nq) of the tile
+                // does the warp's 32 x 8 nq block hold any in-band pair, or only in-band pairs?
                 const int64_t klo = k0 + quarter * 32;
-                const int64_t jl = j0 + c0 + lane, ll = cc.left[c0 + lane];
+                const int cl = c0 + (lane < 8 * nq ? lane : 0);
+                const int64_t jl = j0 + cl, ll = E.left[cl];
                 const int64_t lo = ll > klo ? ll : klo, hi = jl - 1 < klo + 31 ? jl - 1 : klo + 31;
                 const bool any = __any_sync(0xFFFFFFFFu, jl < m && lo <= hi) || dbg != nullptr;
                 const bool all = __all_sync(0xFFFFFFFFu, jl < m && ll <= klo && klo + 31 < jl);
-                double rsum = 0.0;
-                double* rt = ep.K == 1 ? nullptr : ep.rtiles + (size_t)t * TA * TB + (size_t)c0 * TA + row;
+                // K = 1, INT8, a block inside the band: sums of X^2 / (n V), scaled at the end
+                const bool raw = MODE == 0 && all && ep.K == 1 && dbg == nullptr;
+                double rs[2] = {0.0, 0.0};
+                double* rt = ep.K == 1 ? nullptr : ep.rtiles + ((size_t)ep.roff[t] * TILE_QUARTER + c0) * TA + row;
                 if (!any) {
                     if (g == NG - 1) {
                         tc_fence_before();
                         mbar_arrive(tempty);
                     }
                     if (ep.K == 1)
-                        cpart[quarter * TB + c0 + lane] = 0.0;
+                        E.cpart[quarter][cl] = 0.0;
                     else
-                        for (int c = 0; c < 32; c++) rt[(size_t)c * TA] = 0.0;
+                        for (int c = 0; c < 8 * nq; c++) rt[(size_t)c * TA] = 0.0;
                 } else {
+                    // WHAT 0: K = 1, raw; 1: K = 1; 2: K > 1
+                    auto finish = [&](auto what) {
+                        constexpr int WHAT = decltype(what)::value;
+                        const double ck = WHAT == 0 ? qk * ak : qk * ep.r2u_a;
 #pragma unroll 1
-                    for (int ch = 0; ch < 4; ch++) {
-                        const int cb = c0 + 8 * ch;
-                        uint32_t v[4][8];   // GG, GM, MG, MM (sketch: hh, hl, lh, ll) of 8 columns
+                        for (int ch = 0; ch < nq; ch++) {
+                            const int cb = c0 + 8 * ch;
+                            uint32_t v[4][8];   // GG, GM, MG, MM (sketch: hh, hl, lh, ll) of 8 columns
 #pragma unroll
-                        for (int x = 0; x < 4; x++) tmem_ld_32x32b_x8(t_row + (uint32_t)(x * 128 + cb), v[x]);
-                        tmem_ld_wait();
-                        if (g == NG - 1 && ch == 3) {
-                            // this thread's part of the accumulators is read: hand them back to the MMA warp
-                            tc_fence_before();
-                            mbar_arrive(tempty);
-                        }
-                        if (dbg != nullptr && t == 0 && row >= dbg_row && row < dbg_row + 64) {
-#pragma unroll
-                            for (int i = 0; i < 8; i++)
-#pragma unroll
-                                for (int x = 0; x < 4; x++)
-                                    dbg[(2 * (row - dbg_row) + (x >> 1)) * 256 + 2 * (cb + i) + (x & 1)] = (int32_t)v[x][i];
-                        }
-                        double cv[8];
-#pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const double2 qa = cc.qa[cb + i];
-                            double r2u;
-                            if (MODE == 0) {
-                                const int2 ns = cc.ns[cb + i];
-                                const int64_t pg = (int64_t)ns.x * (int32_t)v[0][i] - (int64_t)ns.y * (int32_t)v[1][i];
-                                const int64_t pm = (int64_t)ns.x * (int32_t)v[2][i] - (int64_t)ns.y * (int32_t)v[3][i];
-                                const int64_t X = (int64_t)((uint64_t)pg * nk - (uint64_t)pm * sk);
-                                const double r = (double)X * qk * qa.x;
-                                r2u = r * r * ep.r2u_a + ep.r2u_b;
-                            } else {
-                                const float val = (__uint_as_float(v[0][i]) + __uint_as_float(v[1][i])) +
-                                                  (__uint_as_float(v[2][i]) + __uint_as_float(v[3][i]));
-                                r2u = f32_corr ? (double)sketch_r2u_f32<MODE>(val, qk + qa.x, cf)
-                                               : sketch_r2u<MODE>(val, qk + qa.x, ep);
+                            for (int x = 0; x < 4; x++)
+                                tmem_ld_32x32b_x8(t_row + (uint32_t)((x >> 1) * 256 + (x & 1) * ncol + cb), v[x]);
+                            tmem_ld_wait();
+                            if (g == NG - 1 && ch == nq - 1) {
+                                // this thread's part of the accumulators is read: hand them back to the MMA warp
+                                tc_fence_before();
+                                mbar_arrive(tempty);
                             }
-                            if (!all) {
-                                const int64_t j = j0 + cb + i;
-                                if (!(j < m && k < j && cc.left[cb + i] <= k)) r2u = 0.0;
+                            if (WHAT == 1 && dbg != nullptr && row >= dbg_row && row < dbg_row + 64) {
+#pragma unroll
+                                for (int i = 0; i < 8; i++)
+#pragma unroll
+                                    for (int x = 0; x < 4; x++)
+                                        dbg[(2 * (row - dbg_row) + (x >> 1)) * 256 + 2 * (cb + i) + (x & 1)] =
+                                            (int32_t)v[x][i];
                             }
-                            if (ep.K == 1) {
-                                rsum += r2u * qa.y;
-                                cv[i] = r2u * ak;
-                            } else {
-                                // K > 1: the masked value goes to the tile's f64 slot (record j's row of
-                                // TA values) for the banded annotation contraction; a warp stores 256
-                                // contiguous bytes
-                                rt[(size_t)(8 * ch + i) * TA] = r2u;
+                            double cv[8];
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                double x2 = 0.0, r2u = 0.0;
+                                if (MODE == 0) {
+                                    const int4 ns = E.ns[cb + i];
+                                    const int64_t pg = (int64_t)ns.x * (int32_t)v[0][i] + (int64_t)ns.y * (int32_t)v[1][i];
+                                    const int64_t pm = (int64_t)ns.z * (int32_t)v[3][i] + (int64_t)ns.w * (int32_t)v[2][i];
+                                    const uint64_t xb = (uint64_t)pg * nk + ((uint64_t)pm * sk + magic);
+                                    const double X = big ? (double)(int64_t)xb
+                                                         : __longlong_as_double((long long)xb) -
+                                                               __longlong_as_double((long long)INT_MAGIC);
+                                    x2 = X * X;
+                                    if (WHAT != 0) r2u = fma(x2 * ck, E.qa[cb + i].x, ep.r2u_b);
+                                } else {
+                                    const float val = (__uint_as_float(v[0][i]) + __uint_as_float(v[1][i])) +
+                                                      (__uint_as_float(v[2][i]) + __uint_as_float(v[3][i]));
+                                    const double kap = MODE == 2 ? qk + E.qa[cb + i].x : 0.0;
+                                    r2u = f32_corr ? (double)sketch_r2u_f32<MODE>(val, kap, cf)
+                                                   : sketch_r2u<MODE>(val, kap, ep);
+                                }
+                                if (WHAT == 0) {
+                                    rs[i & 1] = fma(x2, E.qw[cb + i], rs[i & 1]);
+                                    cv[i] = x2 * ck;
+                                    continue;
+                                }
+                                if (!all) {
+                                    const int64_t j = j0 + cb + i;
+                                    if (!(j < m && k < j && E.left[cb + i] <= k)) r2u = 0.0;
+                                }
+                                if (WHAT == 1) {
+                                    rs[i & 1] = fma(r2u, E.qa[cb + i].y, rs[i & 1]);
+                                    cv[i] = r2u * ak;
+                                } else {
+                                    // K > 1: the masked value goes to the tile's f64 slot (record j's row of
+                                    // TA values) for the banded annotation contraction; a warp stores 256
+                                    // contiguous bytes
+                                    rt[(size_t)(8 * ch + i) * TA] = r2u;
+                                }
+                            }
+                            if (WHAT != 2) {
+                                double cs = transpose_sum8(cv, lane);
+                                const int c = cb + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+                                if (WHAT == 0) cs = fma(cs * ep.r2u_a, E.qa[c].x, ep.r2u_b * a_rows);
+                                if ((lane & 3) == 0) E.cpart[quarter][c] = cs;
                             }
                         }
-                        if (ep.K == 1) {
-                            const double cs = transpose_sum8(cv, lane);
-                            if ((lane & 3) == 0)
-                                cpart[quarter * TB + cb + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 +
-                                      ((lane >> 2) & 1)] = cs;
-                        }
-                    }
+                    };
+                    if (ep.K != 1)
+                        finish(std::integral_constant<int, 2>{});
+                    else if (MODE == 0 && raw)
+                        finish(std::integral_constant<int, 0>{});
+                    else
+                        finish(std::integral_constant<int, 1>{});
                 }
-                if (ep.K == 1) rpart[cg * TA + row] = rsum;
+                if (ep.K == 1) {
+                    double rsum = rs[0] + rs[1];
+                    if (raw) {
+                        const double a_cols = warp_sum(lane < 8 * nq ? E.qa[cl].y : 0.0);
+                        rsum = fma(rsum * ep.r2u_a, qk, ep.r2u_b * a_cols);
+                    }
+                    E.rpart[cg][row] = rsum;
+                }
             }
             if (ep.K == 1) {
                 named_bar_sync(1, EPI_T);
-                if (et < TB) {
-                    // per-tile sums in fixed order; launch_l2_reduce adds them to l2
-                    const double rs = rpart[et] + rpart[TA + et] + rpart[2 * TA + et] + rpart[3 * TA + et];
-                    const double cs = cpart[et] + cpart[TB + et] + cpart[2 * TB + et] + cpart[3 * TB + et];
-                    if (ep.prow) {
-                        ep.prow[(size_t)t * TA + et] = rs;
-                        ep.pcol[(size_t)t * TB + et] = cs;
-                    } else {
-                        if (k0 + et < m && rs != 0.0) atomicAdd(ep.l2 + k0 + et, rs);
-                        if (j0 + et < m && cs != 0.0) atomicAdd(ep.l2 + j0 + et, cs);
-                    }
+                // per-tile sums in fixed order; launch_l2_reduce adds them to l2 (columns of the
+                // right block that the tile leaves out are 0).  The next tile writes the other
+                // buffer, and the one after it only past the barriers of the next.
+                if (et < TA) {
+                    const double rsum = E.rpart[0][et] + E.rpart[1][et] + E.rpart[2][et] + E.rpart[3][et];
+                    if (ep.prow)
+                        ep.prow[(size_t)t * TA + et] = rsum;
+                    else if (k0 + et < m && rsum != 0.0)
+                        atomicAdd(ep.l2 + k0 + et, rsum);
+                } else if (et < TA + TB) {
+                    const int cj = et - TA, c = cj - (int)tl.q0 * TILE_QUARTER;
+                    const bool in = c >= 0 && c < ncol;
+                    const double cs = in ? E.cpart[0][c] + E.cpart[1][c] + E.cpart[2][c] + E.cpart[3][c] : 0.0;
+                    if (ep.prow)
+                        ep.pcol[(size_t)t * TB + cj] = cs;
+                    else if (in && j0 + c < m && cs != 0.0)
+                        atomicAdd(ep.l2 + j0 + c, cs);
                 }
+            } else {
+                // every thread has read this tile's wait decision before the next one is written
+                named_bar_sync(1, EPI_T);
             }
-            // every thread has read this tile's wait decision and constants before the next ones are written
-            named_bar_sync(1, EPI_T);
         }
     }
 
@@ -549,6 +648,16 @@ __global__ void __launch_bounds__(gram_threads(EW, CW), 1)
 }
 
 }  // namespace
+
+// Long rows keep whole tiles: the CTAs of a wave then walk K in step, and what
+// one reads the others find in L2.  Trimmed tiles end early, the CTAs drift
+// apart, and the wave's rows (about 25 blocks x 128 records x 2 rows) have to
+// fit: 320 MB at 50,000 individuals, where a tile took 270 us among trimmed
+// ones and 208 us among whole ones; 130 MB at sketch d = 5,000 (157 steps:
+// 1,480 against 1,401 us per launch); 65 MB at 10,000 individuals (79 steps:
+// 1,038 against 1,051 us).
+constexpr uint64_t TRIM_STEPS = 100;
+bool gram_trims(uint64_t row_bytes) { return row_bytes / 128 < TRIM_STEPS; }
 
 using PFN_encodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                      const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -568,14 +677,14 @@ static PFN_encodeTiled get_encode() {
 }
 
 // Map of the operand rows as (byte column, parity, record): row 2 r + p is
-// (., p, r), so a box of 128 records holds rows of one kind.
+// (., p, r), so a box of records holds rows of one kind.
 static bool make_map(CUtensorMap* map, const void* base, CUtensorMapDataType dt, uint64_t ld_elems,
-                     uint64_t elem_bytes, uint64_t m) {
+                     uint64_t elem_bytes, uint64_t m, uint32_t box_records) {
     PFN_encodeTiled enc = get_encode();
     if (!enc) return false;
     cuuint64_t dims[3] = {ld_elems, 2, m};
     cuuint64_t strides[2] = {ld_elems * elem_bytes, 2 * ld_elems * elem_bytes};
-    cuuint32_t box[3] = {(cuuint32_t)(128 / elem_bytes), 1, 128};  // 128-byte rows
+    cuuint32_t box[3] = {(cuuint32_t)(128 / elem_bytes), 1, box_records};  // 128-byte rows
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(map, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -584,18 +693,18 @@ static bool make_map(CUtensorMap* map, const void* base, CUtensorMapDataType dt,
 }
 
 template <int STAGES, int MODE, int EW, int CW>
-static cudaError_t run_tc(const CUtensorMap& tm, int num_kb, const Tile* tiles, int64_t n_tiles,
+static cudaError_t run_tc(const CUtensorMap& tm, const CUtensorMap& tmq, int num_kb, const Tile* tiles, int64_t n_tiles,
                           const EpilogueArgs& ep, int32_t* dbg, int dbg_row, int sms, cudaStream_t stream,
                           uint64_t n_indiv = 0) {
     // alignment slack, operand (and packed) ring, barriers + TMEM slot words, epilogue arrays
     const size_t smem = 1024 + STAGES * (size_t)(A_BYTES + B_BYTES) + (CW > 0 ? (size_t)P_STAGES * P_BYTES : 0) +
-                        8 * (2 * STAGES + 2 * P_STAGES + 4) + sizeof(ColConst) + sizeof(double) * 4 * (TB + TA);
+                        8 * (2 * STAGES + 2 * P_STAGES + 4) + 2 * sizeof(EpiTile);
     cudaError_t e = cudaFuncSetAttribute(k_gram_tc<STAGES, MODE, EW, CW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t grid = dbg ? 1 : (n_tiles < sms ? n_tiles : sms);
     k_gram_tc<STAGES, MODE, EW, CW><<<(unsigned)grid, gram_threads(EW, CW), smem, stream>>>(
-        tm, num_kb, tiles, dbg ? 1 : n_tiles, ep, dbg, dbg_row, n_indiv);
+        tm, tmq, num_kb, tiles, dbg ? 1 : n_tiles, ep, dbg, dbg_row, n_indiv);
     return cudaGetLastError();
 }
 
@@ -606,14 +715,19 @@ static cudaError_t launch_tc(const void* ops, CUtensorMapDataType dt, uint64_t e
     if (n_tiles <= 0) return cudaSuccess;
     if ((ld_elems * elem_bytes) % 128 != 0 || (reinterpret_cast<uintptr_t>(ops) & 15) != 0)
         return cudaErrorInvalidValue;
-    CUtensorMap tm;
-    if (!make_map(&tm, ops, dt, ld_elems, elem_bytes, (uint64_t)m)) return cudaErrorInvalidValue;
-    return run_tc<STAGES_TMA, MODE, EPI_TMA, 0>(tm, (int)(ld_elems * elem_bytes / 128), tiles, n_tiles, ep, dbg,
-                                                dbg_row, sms, stream);
+    CUtensorMap tm, tmq;   // boxes of 128 records, and of 32 for a tile's quarters
+    if (!make_map(&tm, ops, dt, ld_elems, elem_bytes, (uint64_t)m, 128) ||
+        !make_map(&tmq, ops, dt, ld_elems, elem_bytes, (uint64_t)m, TILE_QUARTER))
+        return cudaErrorInvalidValue;
+    const int steps = (int)(ld_elems * elem_bytes / 128);
+    if (MODE == 0 && steps >= LONG_STEPS)
+        return run_tc<STAGES_TMA, 0, EPI_LONG, 0>(tm, tmq, steps, tiles, n_tiles, ep, dbg, dbg_row, sms, stream);
+    return run_tc<STAGES_TMA, MODE, EPI_TMA, 0>(tm, tmq, steps, tiles, n_tiles, ep, dbg, dbg_row, sms, stream);
 }
 
 cudaError_t launch_gram_i8(const uint8_t* ops, uint64_t ld, int64_t m, const Tile* tiles, int64_t n_tiles,
-                           const EpilogueArgs& ep, int32_t* dbg, int dbg_row, int sms, cudaStream_t stream) {
+                           const EpilogueArgs& ep, int32_t* dbg, int dbg_row, int sms,
+                           cudaStream_t stream) {
     return launch_tc<0>(ops, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, ld, m, tiles, n_tiles, ep, dbg, dbg_row, sms, stream);
 }
 
@@ -634,27 +748,30 @@ static bool make_packed_map(CUtensorMap* map, const uint8_t* rows, uint64_t pitc
 }
 
 cudaError_t launch_gram_i8_packed(const uint8_t* rows, uint64_t pitch, uint64_t n_indiv, int64_t m, const Tile* tiles,
-                                  int64_t n_tiles, const EpilogueArgs& ep, int32_t* dbg, int dbg_row, int sms,
-                                  cudaStream_t stream) {
+                                  int64_t n_tiles, const EpilogueArgs& ep, int32_t* dbg, int dbg_row,
+                                  int sms, cudaStream_t stream) {
     if (n_tiles <= 0) return cudaSuccess;
     if (pitch % 16 != 0 || pitch < (n_indiv + 3) / 4 || n_indiv == 0 ||
         (reinterpret_cast<uintptr_t>(rows) & 15) != 0)
         return cudaErrorInvalidValue;
     CUtensorMap tm;
     if (!make_packed_map(&tm, rows, pitch, (uint64_t)m)) return cudaErrorInvalidValue;
-    return run_tc<STAGES_FUSED, 0, EPI_FUSED, CONV_FUSED>(tm, (int)((n_indiv + 127) / 128), tiles, n_tiles, ep, dbg,
+    return run_tc<STAGES_FUSED, 0, EPI_FUSED, CONV_FUSED>(tm, tm, (int)((n_indiv + 127) / 128), tiles, n_tiles, ep, dbg,
                                                           dbg_row, sms, stream, n_indiv);
 }
 
 cudaError_t launch_gram_tf32(const float* ops, uint64_t ld, int64_t m, const Tile* tiles, int64_t n_tiles,
                              const EpilogueArgs& ep, int maf_aware, int sms, cudaStream_t stream) {
     if (maf_aware)
-        return launch_tc<2>(ops, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ld, m, tiles, n_tiles, ep, nullptr, 0, sms, stream);
-    return launch_tc<1>(ops, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ld, m, tiles, n_tiles, ep, nullptr, 0, sms, stream);
+        return launch_tc<2>(ops, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ld, m, tiles, n_tiles, ep, nullptr, 0,
+                            sms, stream);
+    return launch_tc<1>(ops, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ld, m, tiles, n_tiles, ep, nullptr, 0,
+                            sms, stream);
 }
 
 cudaError_t preload_gram_tc() {
     cudaError_t e = preload_kernel(k_gram_tc<STAGES_TMA, 0, EPI_TMA, 0>);
+    if (e == cudaSuccess) e = preload_kernel(k_gram_tc<STAGES_TMA, 0, EPI_LONG, 0>);
     if (e == cudaSuccess) e = preload_kernel(k_gram_tc<STAGES_TMA, 1, EPI_TMA, 0>);
     if (e == cudaSuccess) e = preload_kernel(k_gram_tc<STAGES_TMA, 2, EPI_TMA, 0>);
     if (e == cudaSuccess) e = preload_kernel(k_gram_tc<STAGES_FUSED, 0, EPI_FUSED, CONV_FUSED>);

@@ -92,9 +92,10 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     const uint64_t m = n_snp;
     const uint64_t ld = up(n_indiv, 128);
     std::vector<int64_t> lv(left, left + m);
-    const std::vector<Tile> tiles = band_tiles(lv, TILE_RECORDS, TILE_RECORDS);
-    // the documented limit counts 8 bytes per 64 x 128 records of the band (at
-    // least as many entries as the list above has)
+    std::vector<Tile> tiles;
+    gram_tiles(lv, gram_trims(ld), 4, &tiles);
+    // the documented limit counts 8 bytes per 64 x 128 records of the band, at
+    // least as many as there are whole tiles
     const uint64_t tile_room = band_tiles(lv, 64, 128).size();
     uint64_t off = 0;
     auto take = [&](uint64_t bytes) {
@@ -158,6 +159,7 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     const double denom = n_indiv > 2 ? N - 2.0 : N;
     ep.r2u_a = 1.0 + 1.0 / denom;
     ep.r2u_b = -1.0 / denom;
+    ep.n_used = N;
     ep.err = reinterpret_cast<unsigned int*>(base + o_err);
     if (!tiles.empty() &&
         (rc = ck(launch_gram_i8(ops, ld, (int64_t)m, reinterpret_cast<Tile*>(base + o_tiles), (int64_t)tiles.size(),

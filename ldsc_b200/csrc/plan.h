@@ -38,6 +38,14 @@ bool left_limits(int64_t m, const uint8_t* chr, const double* cm, const uint32_t
 // Band tiles of ta x tb records covering every pair left[j] <= k < j; the
 // second form refills *out, keeping its storage.
 std::vector<Tile> band_tiles(const std::vector<int64_t>& left, int ta, int tb);
+// Gram tiles of the band (Tile, engine.h): per right block of 128 records the
+// left blocks it pairs with.  With trim, each is cut to the quarters of the
+// right block that hold in-band pairs, and then into pieces of at most
+// max_quarters.  Ordered by right block, then left block.
+void gram_tiles(const std::vector<int64_t>& left, bool trim, int max_quarters, std::vector<Tile>* tiles);
+// The same for a run on `sms` SMs: whole right blocks, or finer pieces where
+// that still leaves at most one tile per SM.
+void gram_tiles_for(const std::vector<int64_t>& left, bool trim, int sms, std::vector<Tile>* tiles);
 void band_tiles(const std::vector<int64_t>& left, int ta, int tb, std::vector<Tile>* out);
 
 // fastrand 2.3.0 WyRand stream as used by CountSketchProj::new

@@ -1659,14 +1659,14 @@ extern "C" int ldsc_h2_batch(ldsc_ctx* ctx, const ldsc_h2_args* a, ldsc_h2_resul
                                      (uint64_t)d_ld, (uint64_t)d_wld, (uint64_t)ctx->rg_jobs.p,
                                      (uint64_t)ctx->rg_states.p, (uint64_t)ctx->rg_outs.p, (uint64_t)ctx->rg_part.p,
                                      (uint64_t)ctx->rg_sel.p, (uint64_t)two, (uint64_t)ctx->ts_seps.p,
-                                     (uint64_t)ctx->ts_dv.p, (uint64_t)ctx->ts_outs.p};
+                                     (uint64_t)ctx->ts_dv.p, (uint64_t)ctx->ts_outs.p, (uint64_t)(d_n != nullptr)};
     CK(graph_launch(ctx, gkey, s, [&](cudaStream_t gs) -> cudaError_t {
         RegJob* dj = ctx->rg_jobs.as<RegJob>();
         RegState* dst = ctx->rg_states.as<RegState>();
         cudaError_t e2;
         if (!two) {
             e2 = launch_regressions(dj, dst, ctx->rg_outs.as<RegOut>(), nullptr, ctx->rg_part.as<double>(), nullptr,
-                                    d_ld, d_wld, n, nb, a->m_snps, T, gs);
+                                    d_ld, d_wld, n, nb, a->m_snps, T, gs, nullptr, REG_FORM_HSQ_DIRECT, !d_n);
         } else {
             RegOut* o12 = ctx->ts_outs.as<RegOut>();
             double* dv = ctx->ts_dv.as<double>();
@@ -1991,11 +1991,11 @@ extern "C" int ldsc_rg_batch(ldsc_ctx* ctx, const ldsc_rg_args* a, ldsc_rg_resul
                                      (uint64_t)ctx->rg_res.p};
     CK(graph_launch(ctx, gkey, s, [&](cudaStream_t gs) -> cudaError_t {
         cudaError_t e2 = launch_regressions(dj, dst, dout, nullptr, ctx->rg_part.as<double>(), dtd, d_ld, d_wld, n,
-                                            nb, a->m_snps, 2 * P, gs, nullptr, REG_FORM_HSQ_SQUARE);
+                                            nb, a->m_snps, 2 * P, gs, nullptr, REG_FORM_HSQ_SQUARE, true);
         if (e2 != cudaSuccess) return e2;
         e2 = launch_regressions(dj + 2 * P, dst + 2 * P, dout + 2 * P, dout,
                                 ctx->rg_part.as<double>() + (size_t)2 * P * nb * 5, dtd + (size_t)2 * P * nb, d_ld,
-                                d_wld, n, nb, a->m_snps, P, gs, nullptr, REG_FORM_GENCOV_PRODUCT);
+                                d_wld, n, nb, a->m_snps, P, gs, nullptr, REG_FORM_GENCOV_PRODUCT, true);
         if (e2 != cudaSuccess) return e2;
         return launch_rg_finish(ctx->rg_pairs.as<RgPairIdx>(), dout, dtd, nb, ctx->rg_res.as<RgOut>(), P, gs);
     }));

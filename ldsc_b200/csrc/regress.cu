@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "engine.h"
 #include "regress.h"
@@ -185,6 +186,247 @@ __global__ void __launch_bounds__(RJ * 32, form_kind(FORM) == REG_HSQ ? 3 : 1)
         double* out = part + ((size_t)j * nb + b) * 5;
 #pragma unroll
         for (int q = 0; q < NQ; q++) out[q] = s[q];
+    }
+}
+
+// 1 / d for positive d from the hardware's approximation of the upper word
+// (about 20 bits) by one step of Halley's iteration, which triples the bits:
+// with e = 1 - d r, 1/d = r / (1 - e) = r (1 + e + e^2 + ...), so r + r (e + e^2)
+// leaves e^3.  Without the division's own range checks the chains of a step
+// interleave.  Values outside the normal range's middle take the division.
+__device__ __forceinline__ bool recip_plain(double d) {
+    const uint32_t e = ((uint32_t)__double2hiint(d) >> 20);   // sign and exponent: 0x3FF at 1
+    return e - 2u < 2042u;
+}
+__device__ __forceinline__ double recip_halley(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+// The same sums for plain jobs: scalar sample sizes, the blocks of sep(), no
+// mask (every job of a launch; --two-step and per-SNP sample sizes take
+// k_reg_sums).  A warp sums one block of J jobs, two SNPs per lane at a time:
+// 2 J independent chains, and the LD scores, their clamps and the loop are
+// shared.  The regressor's scale c = Nx / nbar is a constant of the job and
+// multiplies the finished sums (l in place of x0 = c l), so a term costs 12 f64
+// instructions, 3 of them the reciprocal.  A lane takes SNPs lane, lane + 32,
+// ... of the block whatever J is, so a job's sums do not depend on the other
+// jobs of the call.  Bound by the f64 pipe (half busy) and the LSU (70%) in the
+// weighted pass, by DRAM (6 TB/s) in the aggregate pass.  1,000 traits x 200,000
+// SNPs: weighted pass 385 us, aggregate pass 269 us (k_reg_sums: 650 and 331 us).
+// Variants of the weighted pass, same sizes: loads in registers, four jobs per
+// warp, two SNPs in flight 414 us (one prefetched two steps ahead 465 us); y in
+// the ring and the LD scores in registers 435 us.
+constexpr int PLAIN_DEPTH = 4;   // steps of 64 SNPs in a warp's ring
+// streams of a warp's ring: y of each job (two factors in the product form), ld, wld
+template <int FORM, int J>
+constexpr int plain_streams() { return J * (form_ymode(FORM) == REG_Y_PRODUCT ? 2 : 1) + 2; }
+template <int MODE, int FORM, int J>
+constexpr int plain_smem() { return MODE == 0 ? 0 : RJ * PLAIN_DEPTH * plain_streams<FORM, J>() * 64 * (int)sizeof(double); }
+
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+
+template <int MODE, int FORM, int J>
+__global__ void __launch_bounds__(RJ * 32, 3)
+    k_reg_plain(const RegJob* __restrict__ jobs, const RegState* __restrict__ states, const double* __restrict__ ld,
+                const double* __restrict__ wld, uint64_t n, int nb, double m, int njobs, double* __restrict__ part) {
+    constexpr int KIND = form_kind(FORM), YM = form_ymode(FORM);
+    constexpr int U = J == 1 ? 4 : 2;   // aggregate pass: SNPs per lane whose loads are issued together
+    constexpr int S = plain_streams<FORM, J>();
+    const int lane = threadIdx.x & 31;
+    const int b = blockIdx.x, j0 = (blockIdx.y * RJ + (threadIdx.x >> 5)) * J;
+    if (j0 >= njobs) return;
+    const uint64_t lo = sep(n, nb, b);
+    const int32_t cnt = (int32_t)(sep(n, nb, b + 1) - lo);   // n < 2^31 (checked by the launcher)
+    const double* __restrict__ lb = ld + lo;
+    const double* __restrict__ wb = wld + lo;
+    const double* ya[J];
+    const double* yb[J];
+    double ka[J], kb[J], kc[J], ia[J], ib[J], ic[J];   // weight: coefficients of max(l, 1) and constants
+    double s[J][5], sl = 0.0;
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+        const int q = j0 + j < njobs ? j0 + j : j0;   // past the end: the first job again, not stored
+        const RegJob& jb = jobs[q];
+        ya[j] = jb.ya + lo;
+        yb[j] = YM == REG_Y_PRODUCT ? jb.yb + lo : nullptr;
+        if (MODE == 1) {
+            const RegState& st = states[q];
+            const WeightConsts k = weight_consts(st, m);
+            if (KIND == REG_HSQ) {
+                kc[j] = k.hm * jb.n1s;
+                ic[j] = st.intercept;
+            } else {
+                ka[j] = jb.n1s * k.h1m;
+                ia[j] = st.int_h1;
+                kb[j] = jb.n2s * k.h2m;
+                ib[j] = st.int_h2;
+                kc[j] = sqrt(jb.n1s * jb.n2s) * k.sm;
+                ic[j] = st.intercept;
+            }
+        }
+#pragma unroll
+        for (int q5 = 0; q5 < 5; q5++) s[j][q5] = 0.0;
+    }
+    // V SNPs at once: V J independent chains
+    auto step = [&](auto v_c, const double (&y)[2][J], const double (&l)[2], const double (&wl)[2]) {
+        constexpr int V = decltype(v_c)::value;
+        double d[V][J], w[V][J];
+        bool plain_range = true;
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+            const double ocd = fmax(wl[v], 1.0) * (KIND == REG_HSQ ? 2.0 : 1.0), l1 = fmax(l[v], 1.0);
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const double c = fma(kc[j], l1, ic[j]);
+                double t = c * c;
+                if (KIND == REG_GENCOV) t = fma(fma(ka[j], l1, ia[j]), fma(kb[j], l1, ib[j]), t);
+                d[v][j] = t * ocd;
+                plain_range &= recip_plain(d[v][j]);
+            }
+        }
+        if (plain_range) {
+#pragma unroll
+            for (int v = 0; v < V; v++)
+#pragma unroll
+                for (int j = 0; j < J; j++) w[v][j] = recip_halley(d[v][j]);
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; v++)
+#pragma unroll
+                for (int j = 0; j < J; j++) w[v][j] = 1.0 / d[v][j];
+        }
+#pragma unroll
+        for (int v = 0; v < V; v++)
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const double wx = w[v][j] * l[v];
+                s[j][0] = fma(wx, l[v], s[j][0]);
+                s[j][1] += wx;
+                s[j][2] += w[v][j];
+                s[j][3] = fma(wx, y[v][j], s[j][3]);
+                s[j][4] = fma(w[v][j], y[v][j], s[j][4]);
+            }
+    };
+    auto make_y = [&](double a, double a2) {
+        if (YM == REG_Y_SQUARE) {
+            a = a * a;
+            a = isnan(a) ? 0.0 : a;   // fmax(a^2, 0)
+        }
+        return YM == REG_Y_PRODUCT ? a * a2 : a;
+    };
+    if (MODE == 0) {
+        // no arithmetic to hide the loads behind: U of them per stream in flight
+        int32_t k0 = lane;
+        for (; k0 - lane + 32 * U <= cnt; k0 += 32 * U) {
+            double y[U][J], l[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int32_t q = k0 + 32 * u;
+#pragma unroll
+                for (int j = 0; j < J; j++) y[u][j] = make_y(ya[j][q], YM == REG_Y_PRODUCT ? yb[j][q] : 0.0);
+                l[u] = lb[q];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                sl += l[u];
+#pragma unroll
+                for (int j = 0; j < J; j++) s[j][0] += y[u][j];
+            }
+        }
+        for (; k0 < cnt; k0 += 32) {
+            sl += lb[k0];
+#pragma unroll
+            for (int j = 0; j < J; j++) s[j][0] += make_y(ya[j][k0], YM == REG_Y_PRODUCT ? yb[j][k0] : 0.0);
+        }
+    } else {
+        // each lane copies its own SNPs of every stream into a ring of
+        // PLAIN_DEPTH steps of 64 SNPs (no other lane reads them, so there is no
+        // barrier): the loads in flight cost no registers
+        extern __shared__ double ring[];
+        double* mine = ring + (size_t)(threadIdx.x >> 5) * PLAIN_DEPTH * S * 64 + lane;
+        auto issue = [&](int32_t t, int slot) {
+            double* dst = mine + slot * S * 64;
+#pragma unroll
+            for (int v = 0; v < 2; v++) {
+                const int32_t q = 64 * t + 32 * v + lane;
+                if (q >= cnt) break;
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    cp_async8(dst + 64 * j + 32 * v, ya[j] + q);
+                    if (YM == REG_Y_PRODUCT) cp_async8(dst + 64 * (J + 2 + j) + 32 * v, yb[j] + q);
+                }
+                cp_async8(dst + 64 * J + 32 * v, lb + q);
+                cp_async8(dst + 64 * (J + 1) + 32 * v, wb + q);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        const int32_t steps = (cnt + 63) / 64;
+#pragma unroll
+        for (int t = 0; t < PLAIN_DEPTH - 1; t++) issue(t, t);
+        for (int32_t t0 = 0; t0 < steps; t0 += PLAIN_DEPTH) {
+#pragma unroll
+            for (int slot = 0; slot < PLAIN_DEPTH; slot++) {
+                const int32_t t = t0 + slot;
+                if (t >= steps) break;
+                issue(t + PLAIN_DEPTH - 1, (slot + PLAIN_DEPTH - 1) % PLAIN_DEPTH);
+                asm volatile("cp.async.wait_group %0;" ::"n"(PLAIN_DEPTH - 1) : "memory");
+                const double* src = mine + slot * S * 64;
+                const int32_t q = 64 * t + lane;
+                double y[2][J], l[2], wl[2];
+#pragma unroll
+                for (int v = 0; v < 2; v++) {
+#pragma unroll
+                    for (int j = 0; j < J; j++)
+                        y[v][j] =
+                            make_y(src[64 * j + 32 * v], YM == REG_Y_PRODUCT ? src[64 * (J + 2 + j) + 32 * v] : 0.0);
+                    l[v] = src[64 * J + 32 * v];
+                    wl[v] = src[64 * (J + 1) + 32 * v];
+                }
+                if (q + 32 < cnt)
+                    step(std::integral_constant<int, 2>{}, y, l, wl);
+                else if (q < cnt)
+                    step(std::integral_constant<int, 1>{}, y, l, wl);
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    constexpr int NQ = MODE == 0 ? 1 : 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (MODE == 0) sl += __shfl_xor_sync(0xFFFFFFFFu, sl, o);
+#pragma unroll
+        for (int j = 0; j < J; j++)
+#pragma unroll
+            for (int q = 0; q < NQ; q++) s[j][q] += __shfl_xor_sync(0xFFFFFFFFu, s[j][q], o);
+    }
+    if (lane != 0) return;
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+        if (j0 + j >= njobs) break;
+        const RegJob& jb = jobs[j0 + j];
+        const double nx = KIND == REG_HSQ ? jb.n1s : sqrt(jb.n1s * jb.n2s);
+        double* out = part + ((size_t)(j0 + j) * nb + b) * 5;
+        if (MODE == 0) {
+            out[0] = s[j][0];
+            out[1] = nx * sl;
+            out[2] = nx * (double)cnt;
+        } else {
+            const double c = nx * (1.0 / states[j0 + j].nbar);
+            out[0] = s[j][0] * c * c;
+            out[1] = s[j][1] * c;
+            out[2] = s[j][2];
+            out[3] = s[j][3] * c;
+            out[4] = s[j][4];
+        }
+        if (jb.kind != KIND || jb.ymode != YM)   // a job of another form
+#pragma unroll
+            for (int q = 0; q < 5; q++) out[q] = NAN;
     }
 }
 
@@ -387,20 +629,31 @@ __global__ void __launch_bounds__(NT) k_rg_finish(const RgPairIdx* __restrict__ 
     }
 }
 
-// The two middle order statistics of each job's y (ranks ra <= rb, rb - ra
-// <= 1), exactly: a radix select over the order-preserving 64-bit keys of the
-// doubles, 11 bits per digit, one CTA per job.  Each digit is one sweep over
-// the job's y; the sweep histograms the keys that share the prefix fixed so
-// far.  Once that prefix holds at most SEL_CAP keys, one more sweep gathers
-// them into shared memory and they are ranked there.  If the two ranks fall
-// in different buckets of a digit, ra is the largest key of its bucket and rb
-// the smallest of its own, found by one more sweep.  On LD-score chi2 values
-// two digits (sign and exponent, then the mantissa's top bits) usually leave
-// about a hundred keys, so the select reads each y three times.
+// The two middle order statistics of each job's ya (ranks ra <= rb, rb - ra
+// <= 1), exactly, over the order-preserving 64-bit keys of the doubles; one CTA
+// per job, bound by the sweeps over the job's y.
+//
+// Two sweeps (n >= SEL_SAMPLE_MIN): 1,024 evenly spaced keys are sorted, and
+// the keys 80 places either side of the ranks' places (five standard
+// deviations of a sampled rank) bracket them.  The first sweep counts the keys
+// below the bracket and histograms those inside it (about a sixth) into 2,048
+// equal bins of the keys' upper words; the second gathers the one or two bins that hold the
+// ranks, and the gathered keys are ranked in shared memory.  A bracket that
+// misses, or a bin of more than SEL_CAP keys (ties), falls back to the
+// radix select.  1,000 traits x 200,000: 638 us (radix select alone 1,689 us).
+//
+// Radix select: 11 bits per digit, one sweep per digit; the sweep histograms
+// the keys that share the prefix fixed so far.  Once that prefix holds at most
+// SEL_CAP keys, one more sweep gathers them into shared memory and they are
+// ranked there.  If the two ranks fall in different buckets of a digit, ra is
+// the largest key of its bucket and rb the smallest of its own, found by one
+// more sweep.
 __device__ __forceinline__ uint64_t okey(double v) {
     const uint64_t b = (uint64_t)__double_as_longlong(v);
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
+// upper word of okey from the upper word of the double
+__device__ __forceinline__ uint32_t okey_hi(uint32_t h) { return h ^ ((uint32_t)((int32_t)h >> 31) | 0x80000000u); }
 __device__ __forceinline__ double okey_value(uint64_t k) {
     const uint64_t b = (k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k;
     return __longlong_as_double((long long)b);
@@ -410,88 +663,55 @@ constexpr int SEL_T = 256;
 constexpr int SEL_W = SEL_T / 32;
 constexpr int SEL_BITS = 11;
 constexpr int SEL_BINS = 1 << SEL_BITS;
-constexpr int SEL_CAP = 2048;  // keys ranked in shared memory
-constexpr int SEL_U = 8;       // loads in flight per thread
+constexpr int SEL_CAP = 1024;  // keys ranked in shared memory
+constexpr int SEL_DEPTH = 6;   // ring of the sweeps
+constexpr int SEL_SAMPLE = 1024, SEL_HALF = 80;   // (the sample is sorted in the candidates' place)
+constexpr uint64_t SEL_SAMPLE_MIN = 16384;   // below, three sweeps of a cached y cost less than the sort
 
-// Calls f(key, valid) for every y of the job; the trip count is the same in
-// every lane of a warp, so f may use warp-collective operations.
+// Calls f(value, valid) for every ya of the job; the trip count is the same in
+// every lane of a warp, so f may use warp-collective operations.  Each thread
+// copies its own values through a ring in shared memory (SEL_DEPTH loads in
+// flight without registers; seven CTAs of a job each per SM).
 template <class F>
-__device__ __forceinline__ void sel_sweep(const RegJob& jb, uint64_t n, F f) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint64_t i0 = (uint64_t)warp * 32 * SEL_U; i0 < n; i0 += (uint64_t)SEL_T * SEL_U) {
-        uint64_t k[SEL_U];
-        bool v[SEL_U];
+__device__ __forceinline__ void sel_sweep(const double* __restrict__ y, uint64_t n, double (*ring)[SEL_T], F f) {
+    const int32_t steps = (int32_t)((n + SEL_T - 1) / SEL_T);   // n < 2^31
+    auto issue = [&](int32_t t, int slot) {
+        const uint64_t i = (uint64_t)t * SEL_T + threadIdx.x;
+        if (i < n) cp_async8(&ring[slot][threadIdx.x], y + i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-        for (int u = 0; u < SEL_U; u++) {
-            const uint64_t i = i0 + (uint64_t)u * 32 + lane;
-            v[u] = i < n;
-            k[u] = v[u] ? okey(job_y(jb, i)) : 0ull;
+    for (int t = 0; t < SEL_DEPTH - 1; t++) issue(t, t);
+    for (int32_t t0 = 0; t0 < steps; t0 += SEL_DEPTH) {
+#pragma unroll
+        for (int slot = 0; slot < SEL_DEPTH; slot++) {
+            const int32_t t = t0 + slot;
+            if (t >= steps) break;
+            issue(t + SEL_DEPTH - 1, (slot + SEL_DEPTH - 1) % SEL_DEPTH);
+            asm volatile("cp.async.wait_group %0;" ::"n"(SEL_DEPTH - 1) : "memory");
+            const bool v = (uint64_t)t * SEL_T + threadIdx.x < n;
+            f(ring[slot][threadIdx.x], v);   // (nothing valid where !v)
         }
-#pragma unroll
-        for (int u = 0; u < SEL_U; u++) f(k[u], v[u]);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(SEL_T, 8) k_select_mid(const RegJob* __restrict__ jobs, uint64_t n, uint64_t ra,
+__global__ void __launch_bounds__(SEL_T, 7) k_select_mid(const RegJob* __restrict__ jobs, uint64_t n, uint64_t ra,
                                                       uint64_t rb, double* __restrict__ out_a,
                                                       double* __restrict__ out_b) {
     __shared__ uint32_t hist[SEL_BINS];
     __shared__ uint64_t cand[SEL_CAP];
+    __shared__ double ring[SEL_DEPTH][SEL_T];
     __shared__ uint32_t wsum[SEL_W];
     __shared__ uint32_t s_da, s_db, s_acc_a, s_acc_b, s_cnt;
     __shared__ unsigned long long s_ka, s_kb;
-    const RegJob jb = jobs[blockIdx.x];
+    const double* __restrict__ y = jobs[blockIdx.x].ya;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint64_t prefix = 0, pmask = 0, cnt = n;
-    uint64_t qa = ra, qb = rb;  // ranks among the keys that match the prefix
-    int top = 64;               // bits below the prefix
-    for (;;) {
-        if (cnt <= SEL_CAP) {
-            // gather the prefix's keys and rank them in shared memory
-            if (threadIdx.x == 0) s_cnt = 0;
-            __syncthreads();
-            sel_sweep(jb, n, [&](uint64_t k, bool v) {
-                const bool take = v && (k & pmask) == prefix;
-                const unsigned m = __ballot_sync(0xFFFFFFFFu, take);
-                uint32_t base = 0;
-                if (lane == 0 && m) base = atomicAdd(&s_cnt, (uint32_t)__popc(m));
-                base = __shfl_sync(0xFFFFFFFFu, base, 0);
-                if (take) cand[base + __popc(m & ((1u << lane) - 1u))] = k;
-            });
-            __syncthreads();
-            const uint32_t c = s_cnt;
-            for (uint32_t i = threadIdx.x; i < c; i += SEL_T) {
-                const uint64_t ki = cand[i];
-                uint32_t r = 0;
-                for (uint32_t j = 0; j < c; j++) {
-                    const uint64_t kj = cand[j];
-                    r += (kj < ki || (kj == ki && j < i)) ? 1u : 0u;
-                }
-                if (r == qa) s_ka = ki;
-                if (r == qb) s_kb = ki;
-            }
-            __syncthreads();
-            break;
-        }
-        if (top == 0) {  // every key left equals the prefix
-            if (threadIdx.x == 0) s_ka = s_kb = prefix;
-            __syncthreads();
-            break;
-        }
-        const int width = top < SEL_BITS ? top : SEL_BITS;
-        const int shift = top - width;
-        const uint32_t dmask = (1u << width) - 1u;
-        for (int i = threadIdx.x; i < SEL_BINS; i += SEL_T) hist[i] = 0;
-        __syncthreads();
-        sel_sweep(jb, n, [&](uint64_t k, bool v) {
-            const bool take = v && (k & pmask) == prefix;
-            const uint32_t bin = take ? (uint32_t)(k >> shift) & dmask : 0xFFFFFFFFu;
-            const unsigned peers = __match_any_sync(0xFFFFFFFFu, bin);
-            if (take && lane == __ffs(peers) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
-        });
-        __syncthreads();
-        // bins of this thread: [PER t, PER t + PER); exclusive block scan of their sums
-        constexpr int PER = SEL_BINS / SEL_T;
+    // exclusive block scan of the histogram; sets s_da / s_acc_a to the bin of
+    // rank qa and the keys before it (same for qb) where the ranks lie in it,
+    // and returns the number of keys in it (hist must be complete)
+    constexpr int PER = SEL_BINS / SEL_T;   // bins of this thread: [PER t, PER t + PER)
+    auto find_bins = [&](uint64_t qa, uint64_t qb) {
         uint32_t c[PER], tsum = 0;
 #pragma unroll
         for (int q = 0; q < PER; q++) {
@@ -506,8 +726,11 @@ __global__ void __launch_bounds__(SEL_T, 8) k_select_mid(const RegJob* __restric
         }
         if (lane == 31) wsum[warp] = incl;
         __syncthreads();
-        uint32_t acc = incl - tsum;
-        for (int w = 0; w < warp; w++) acc += wsum[w];
+        uint32_t acc = incl - tsum, total = 0;
+        for (int w = 0; w < SEL_W; w++) {
+            if (w < warp) acc += wsum[w];
+            total += wsum[w];
+        }
 #pragma unroll
         for (int q = 0; q < PER; q++) {
             if (qa >= acc && qa < acc + c[q]) {
@@ -521,6 +744,115 @@ __global__ void __launch_bounds__(SEL_T, 8) k_select_mid(const RegJob* __restric
             acc += c[q];
         }
         __syncthreads();
+        return total;
+    };
+    // keys of ranks qa and qb among the c gathered ones, into s_ka and s_kb
+    auto rank_gathered = [&](uint32_t c, uint64_t qa, uint64_t qb) {
+        for (uint32_t i = threadIdx.x; i < c; i += SEL_T) {
+            const uint64_t ki = cand[i];
+            uint32_t r = 0;
+            for (uint32_t j = 0; j < c; j++) {
+                const uint64_t kj = cand[j];
+                r += (kj < ki || (kj == ki && j < i)) ? 1u : 0u;
+            }
+            if (r == qa) s_ka = ki;
+            if (r == qb) s_kb = ki;
+        }
+        __syncthreads();
+    };
+    bool done = false;
+    if (n >= SEL_SAMPLE_MIN) {
+        for (int i = threadIdx.x; i < SEL_SAMPLE; i += SEL_T) cand[i] = okey(y[(uint64_t)i * n / SEL_SAMPLE]);
+        for (int i = threadIdx.x; i < SEL_BINS; i += SEL_T) hist[i] = 0;
+        if (threadIdx.x == 0) s_cnt = 0;
+        for (int k = 2; k <= SEL_SAMPLE; k <<= 1)   // bitonic sort
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                __syncthreads();
+                for (int t = threadIdx.x; t < SEL_SAMPLE / 2; t += SEL_T) {
+                    const int i = 2 * t - (t & (j - 1)), l = i + j;   // t's pair at distance j
+                    const uint64_t a = cand[i], b = cand[l];
+                    if ((a > b) == ((i & k) == 0)) {
+                        cand[i] = b;
+                        cand[l] = a;
+                    }
+                }
+            }
+        __syncthreads();
+        // the bracket in upper words of the keys: [klo, klo + range]
+        const int64_t pa = (int64_t)(ra * SEL_SAMPLE / n) - SEL_HALF, pb = (int64_t)(rb * SEL_SAMPLE / n) + SEL_HALF;
+        const uint32_t klo = pa >= 0 ? (uint32_t)(cand[pa] >> 32) : 0u;
+        const uint32_t range = (pb < SEL_SAMPLE ? (uint32_t)(cand[pb] >> 32) : 0xFFFFFFFFu) - klo;
+        const int shift = max(0, 32 - __clz((int)(range | 1u)) - SEL_BITS);   // range >> shift < SEL_BINS
+        uint32_t below = 0;
+        sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+            const uint32_t k = okey_hi((uint32_t)__double2hiint(yv)), t = k - klo;
+            below += v && k < klo;
+            if (v && t <= range) atomicAdd(&hist[t >> shift], 1u);
+        });
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xFFFFFFFFu, below, o);
+        if (lane == 0) atomicAdd(&s_cnt, below);
+        __syncthreads();   // histogram and s_cnt complete; the sample is no longer read
+        const uint64_t nbelow = s_cnt;
+        const uint64_t inside = find_bins(ra - nbelow, rb - nbelow);   // (a rank below the bracket wraps: in no bin)
+        if (ra >= nbelow && rb - nbelow < inside) {
+            const uint32_t da = s_da, db = s_db, acc_a = s_acc_a;
+            if (hist[da] + (db != da ? hist[db] : 0u) <= (uint32_t)SEL_CAP) {   // bins between the two are empty
+                // upper words of bins da .. db: [g0, g0 + gr]
+                const uint32_t g0 = klo + (da << shift), gr = ((db - da + 1) << shift) - 1u;
+                const uint32_t cut = min(gr, range - (da << shift));
+                if (threadIdx.x == 0) s_cnt = 0;
+                __syncthreads();
+                sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+                    if (v && okey_hi((uint32_t)__double2hiint(yv)) - g0 <= cut) cand[atomicAdd(&s_cnt, 1u)] = okey(yv);
+                });
+                __syncthreads();
+                rank_gathered(s_cnt, ra - nbelow - acc_a, rb - nbelow - acc_a);
+                done = true;
+            }
+        }
+        __syncthreads();
+    }
+    uint64_t prefix = 0, pmask = 0, cnt = n;
+    uint64_t qa = ra, qb = rb;  // ranks among the keys that match the prefix
+    int top = 64;               // bits below the prefix
+    while (!done) {
+        if (cnt <= SEL_CAP) {
+            // gather the prefix's keys and rank them in shared memory
+            if (threadIdx.x == 0) s_cnt = 0;
+            __syncthreads();
+            sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+                const uint64_t k = okey(yv);
+                const bool take = v && (k & pmask) == prefix;
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, take);
+                uint32_t base = 0;
+                if (lane == 0 && m) base = atomicAdd(&s_cnt, (uint32_t)__popc(m));
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                if (take) cand[base + __popc(m & ((1u << lane) - 1u))] = k;
+            });
+            __syncthreads();
+            rank_gathered(s_cnt, qa, qb);
+            break;
+        }
+        if (top == 0) {  // every key left equals the prefix
+            if (threadIdx.x == 0) s_ka = s_kb = prefix;
+            __syncthreads();
+            break;
+        }
+        const int width = top < SEL_BITS ? top : SEL_BITS;
+        const int shift = top - width;
+        const uint32_t dmask = (1u << width) - 1u;
+        for (int i = threadIdx.x; i < SEL_BINS; i += SEL_T) hist[i] = 0;
+        __syncthreads();
+        sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+            const uint64_t k = okey(yv);
+            const bool take = v && (k & pmask) == prefix;
+            const uint32_t bin = take ? (uint32_t)(k >> shift) & dmask : 0xFFFFFFFFu;
+            const unsigned peers = __match_any_sync(0xFFFFFFFFu, bin);
+            if (take && lane == __ffs(peers) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
+        });
+        __syncthreads();
+        find_bins(qa, qb);
         const uint32_t da = s_da, db = s_db;
         const uint64_t dm = (uint64_t)dmask << shift;
         if (da == db) {
@@ -541,7 +873,8 @@ __global__ void __launch_bounds__(SEL_T, 8) k_select_mid(const RegJob* __restric
             s_kb = ~0ull;
         }
         __syncthreads();
-        sel_sweep(jb, n, [&](uint64_t k, bool v) {
+        sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+            const uint64_t k = okey(yv);
             if (v && (k & nm) == pa) atomicMax(&s_ka, (unsigned long long)k);
             if (v && (k & nm) == pb) atomicMin(&s_kb, (unsigned long long)k);
         });
@@ -693,6 +1026,33 @@ __global__ void __launch_bounds__(NT) k_ts_combine(const RegOut* __restrict__ ou
 
 }  // namespace
 
+// Jobs per warp of the plain kernel's many-job form.
+static constexpr int plain_jobs(int form) { return form == REG_FORM_GENCOV_PRODUCT ? 1 : 2; }
+
+// Loads the plain kernels of a form and sets their shared-memory limit, which
+// stays with the device's context.
+template <int F, int J>
+static cudaError_t preload_plain() {
+    cudaError_t e = preload_kernel(k_reg_plain<0, F, 1>);
+    if (e == cudaSuccess) e = preload_kernel(k_reg_plain<0, F, 2 * J>);
+    if (e == cudaSuccess) e = preload_kernel(k_reg_plain<1, F, J>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_reg_plain<1, F, J>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 plain_smem<1, F, J>());
+    return e;
+}
+
+// f called with the form as a compile-time constant.
+template <typename F>
+static void for_form(int form, F&& f) {
+    if (form == REG_FORM_HSQ_DIRECT)
+        f(std::integral_constant<int, REG_FORM_HSQ_DIRECT>{});
+    else if (form == REG_FORM_HSQ_SQUARE)
+        f(std::integral_constant<int, REG_FORM_HSQ_SQUARE>{});
+    else
+        f(std::integral_constant<int, REG_FORM_GENCOV_PRODUCT>{});
+}
+
 cudaError_t launch_twostep_seps(const RegJob* jobs, uint64_t n, int nb, int32_t* seps, int32_t* n1, int32_t* cnt,
                                 int njobs, cudaStream_t s) {
     if (njobs <= 0 || n == 0) return cudaSuccess;
@@ -711,23 +1071,34 @@ cudaError_t launch_twostep_combine(const RegOut* out1, const RegOut* out2, const
 
 cudaError_t launch_regressions(const RegJob* jobs, RegState* states, RegOut* outs, const RegOut* ref_outs,
                                double* part, double* tot_delete, const double* ld, const double* wld, uint64_t n,
-                               int nb, double m, int njobs, cudaStream_t s, double* dv, int form) {
+                               int nb, double m, int njobs, cudaStream_t s, double* dv, int form, bool plain) {
     if (njobs <= 0) return cudaSuccess;
     if (form < REG_FORM_HSQ_DIRECT || form > REG_FORM_GENCOV_PRODUCT || n >= (1ull << 31))
         return cudaErrorInvalidValue;
-    const dim3 grid(nb, (njobs + RJ - 1) / RJ);
     const int ub = (njobs + 3) / 4;  // k_reg_update: four warps (jobs) per CTA
+    // Plain jobs: two to a warp (one of the covariance form, which has two y
+    // streams; twice as many in the aggregate pass, which only reads) once that
+    // still leaves the device full (148 SMs x 16 warps), else one.
+    const int many = plain_jobs(form);
+    const bool full = plain && (int64_t)nb * (njobs / many) >= 148 * 16;
+    auto grid_of = [&](int per) { return dim3(nb, (njobs + RJ * per - 1) / (RJ * per)); };
+    auto go = [&](auto mode_c, auto form_c) {
+        constexpr int M = decltype(mode_c)::value, F = decltype(form_c)::value;
+        constexpr int J = plain_jobs(F) * (M == 0 ? 2 : 1);
+        if (!plain)
+            k_reg_sums<M, F><<<grid_of(1), RJ * 32, 0, s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
+        else if (full)
+            k_reg_plain<M, F, J><<<grid_of(J), RJ * 32, plain_smem<M, F, J>(), s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
+        else
+            k_reg_plain<M, F, 1><<<grid_of(1), RJ * 32, plain_smem<M, F, 1>(), s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
+    };
     auto sums = [&](int mode) {
-        if (form == REG_FORM_HSQ_DIRECT) {
-            if (mode == 0) k_reg_sums<0, REG_FORM_HSQ_DIRECT><<<grid, RJ * 32, 0, s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
-            else k_reg_sums<1, REG_FORM_HSQ_DIRECT><<<grid, RJ * 32, 0, s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
-        } else if (form == REG_FORM_HSQ_SQUARE) {
-            if (mode == 0) k_reg_sums<0, REG_FORM_HSQ_SQUARE><<<grid, RJ * 32, 0, s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
-            else k_reg_sums<1, REG_FORM_HSQ_SQUARE><<<grid, RJ * 32, 0, s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
-        } else {
-            if (mode == 0) k_reg_sums<0, REG_FORM_GENCOV_PRODUCT><<<grid, RJ * 32, 0, s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
-            else k_reg_sums<1, REG_FORM_GENCOV_PRODUCT><<<grid, RJ * 32, 0, s>>>(jobs, states, ld, wld, n, nb, m, njobs, part);
-        }
+        for_form(form, [&](auto f) {
+            if (mode == 0)
+                go(std::integral_constant<int, 0>{}, f);
+            else
+                go(std::integral_constant<int, 1>{}, f);
+        });
     };
     sums(0);
     k_reg_update<0><<<ub, 128, 0, s>>>(jobs, states, ref_outs, part, n, nb, m, njobs);
@@ -749,18 +1120,22 @@ cudaError_t launch_rg_finish(const RgPairIdx* pairs, const RegOut* outs, const d
 
 cudaError_t launch_select_mid(const RegJob* jobs, uint64_t n, uint64_t ra, uint64_t rb, double* out_a, double* out_b,
                               int njobs, cudaStream_t s) {
-    if (njobs <= 0 || n == 0 || ra > rb || rb - ra > 1 || rb >= n) return cudaErrorInvalidValue;
+    if (njobs <= 0 || n == 0 || n >= (1ull << 31) || ra > rb || rb - ra > 1 || rb >= n) return cudaErrorInvalidValue;
     k_select_mid<<<njobs, SEL_T, 0, s>>>(jobs, n, ra, rb, out_a, out_b);
     return cudaGetLastError();
 }
 
 cudaError_t preload_regress() {
-    cudaError_t e = preload_kernel(k_reg_sums<0, REG_FORM_HSQ_DIRECT>);
-    if (e == cudaSuccess) e = preload_kernel(k_reg_sums<1, REG_FORM_HSQ_DIRECT>);
-    if (e == cudaSuccess) e = preload_kernel(k_reg_sums<0, REG_FORM_HSQ_SQUARE>);
-    if (e == cudaSuccess) e = preload_kernel(k_reg_sums<1, REG_FORM_HSQ_SQUARE>);
-    if (e == cudaSuccess) e = preload_kernel(k_reg_sums<0, REG_FORM_GENCOV_PRODUCT>);
-    if (e == cudaSuccess) e = preload_kernel(k_reg_sums<1, REG_FORM_GENCOV_PRODUCT>);
+    cudaError_t e = cudaSuccess;
+    for (int form = REG_FORM_HSQ_DIRECT; form <= REG_FORM_GENCOV_PRODUCT; form++)
+        for_form(form, [&](auto f) {
+            constexpr int F = decltype(f)::value;
+            if (e == cudaSuccess) e = preload_kernel(k_reg_sums<0, F>);
+            if (e == cudaSuccess) e = preload_kernel(k_reg_sums<1, F>);
+            constexpr int J = plain_jobs(F);
+            if (e == cudaSuccess) e = preload_plain<F, 1>();
+            if (e == cudaSuccess) e = preload_plain<F, J>();
+        });
     if (e == cudaSuccess) e = preload_kernel(k_reg_update<0>);
     if (e == cudaSuccess) e = preload_kernel(k_reg_update<1>);
     if (e == cudaSuccess) e = preload_kernel(k_reg_jackknife);

@@ -66,11 +66,12 @@ struct RgOut {
 // outs[j] receives job j's result; ref_outs holds the h2 results that
 // REG_GENCOV jobs refer to by index.  part: njobs * nb * 5 doubles of
 // scratch; tot_delete (optional): njobs * nb; dv (optional): njobs * nb * 2
-// delete values.
+// delete values.  plain: every job has scalar sample sizes, no block starts of
+// its own and no mask.
 cudaError_t launch_regressions(const RegJob* jobs, RegState* states, RegOut* outs, const RegOut* ref_outs,
                                double* part, double* tot_delete, const double* ld, const double* wld, uint64_t n,
                                int nb, double m, int njobs, cudaStream_t s, double* dv = nullptr,
-                               int form = REG_FORM_HSQ_DIRECT);
+                               int form = REG_FORM_HSQ_DIRECT, bool plain = false);
 
 // --two-step block starts: for each job, mask = y < mask_max, n1 = its size,
 // and seps[b] = index of the kept SNP of rank floor(b n1 / nb) (0 and n at
@@ -89,7 +90,7 @@ cudaError_t launch_twostep_combine(const RegOut* out1, const RegOut* out2, const
 cudaError_t launch_rg_finish(const RgPairIdx* pairs, const RegOut* outs, const double* tot_delete, int nb,
                              RgOut* res, int npairs, cudaStream_t s);
 
-// The ra-th and rb-th smallest y of each job (exact; ra <= rb <= ra + 1),
+// The ra-th and rb-th smallest ya of each job (exact; ra <= rb <= ra + 1; n < 2^31),
 // out_a[job] and out_b[job].
 cudaError_t launch_select_mid(const RegJob* jobs, uint64_t n, uint64_t ra, uint64_t rb, double* out_a, double* out_b,
                               int njobs, cudaStream_t s);

@@ -468,7 +468,7 @@ int ldsc_l2_workspace_bytes(const ldsc_l2_args* a, uint64_t n_indiv, uint64_t* b
          8 * nt_room + 4 * (2 * (m / 128) + 4);
     if (a->annot && !a->annot_on_device) b += 8 * m * K;
     if (a->bed_idx) b += 8 * m;
-    if (a->keep_iids) b += 8 * a->n_keep;
+    if (a->keep_iids) b += 8 * a->n_keep + (d ? 0 : m * round_up((n_used + 3) / 4, 16));  // indices, compacted rows
     // INT8 operand rows (the default two-pass form; an upper bound for the fused one)
     if (exact_i8) b += 2 * m * round_up(n_used, 128);
     else if (d) b += 8 * m * round_up(d, 32);
@@ -808,8 +808,25 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         pv.rows += a->row_begin * panel->pitch;
         pv.n_snp -= a->row_begin;
     }
-    IndivSel sel{a->keep_iids ? ctx->keep.as<int64_t>() : nullptr, n_used};
     const uint64_t* rr = a->bed_idx ? ctx->recrows.as<uint64_t>() : nullptr;
+    // --keep (exact forms): the kept individuals' rows are compacted first, and
+    // everything after reads those
+    const bool compact = a->keep_iids && !d;
+    const uint64_t kp = round_up((n_used + 3) / 4, 16);
+    if (compact) CK(ctx->packed.ensure((size_t)kp * nmom));
+    // rows of records [r0, r1) as the decode kernels read them (row list, or null for rows in order)
+    auto rows_of = [&](int64_t r0, int64_t r1, cudaStream_t on, PanelView* v, const uint64_t** list) -> cudaError_t {
+        *v = pv;
+        if (!rr) v->rows = pv.rows + (uint64_t)r0 * pv.pitch;
+        *list = rr ? rr + r0 : nullptr;
+        if (!compact) return cudaSuccess;
+        uint8_t* dst = ctx->packed.as<uint8_t>() + (size_t)r0 * kp;
+        const cudaError_t e = launch_compact(*v, *list, r1 - r0, ctx->keep.as<int64_t>(), n_used, dst, kp, on);
+        *v = PanelView{dst, (uint64_t)(r1 - r0), n_used, (n_used + 3) / 4, kp};
+        *list = nullptr;
+        ctx->kernels++;
+        return e;
+    };
     RecStats st{};
     st.n = ctx->st_n.as<int32_t>();
     st.s = ctx->st_s.as<int32_t>();
@@ -1053,14 +1070,15 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             int rc = feed->issue_until(k + 1, s);
             if (rc != LDSC_OK) return rc;
             if (r1 > r0) {
-                PanelView pc = pv;
-                if (!rr) pc.rows = pv.rows + (uint64_t)r0 * pv.pitch;
+                PanelView pc;
+                const uint64_t* list;
+                CK(rows_of(r0, r1, s, &pc, &list));
                 RecStats sc = st;
                 sc.n += r0;
                 sc.s += r0;
                 sc.q += r0;
                 uint8_t* oc = staged_i8 ? ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8 : nullptr;
-                CK(launch_decode_i8(pc, rr ? rr + r0 : nullptr, r1 - r0, sel, oc, staged_i8 ? ld_i8 : 0, sc, 0, s));
+                CK(launch_decode_i8(pc, list, r1 - r0, oc, staged_i8 ? ld_i8 : 0, sc, 0, s));
                 ctx->kernels++;
                 if (stream_gram) {
                     sc.maf += r0;
@@ -1102,8 +1120,9 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         CK(cudaStreamWaitEvent(ctx->side, ctx->ovl_go, 0));
         for (int k = 0; k < ov_n; k++) {
             const int64_t r0 = ov_b[k], r1 = ov_b[k + 1];
-            PanelView pc = pv;
-            if (!rr) pc.rows = pv.rows + (uint64_t)r0 * pv.pitch;
+            PanelView pc;
+            const uint64_t* list;
+            CK(rows_of(r0, r1, ctx->side, &pc, &list));
             RecStats sc = st;
             sc.n += r0;
             sc.s += r0;
@@ -1112,8 +1131,8 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             sc.mean += r0;
             sc.inv_std += r0;
             sc.qinv += r0;
-            CK(launch_decode_i8(pc, rr ? rr + r0 : nullptr, r1 - r0, sel, ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8,
-                                ld_i8, sc, 0, ctx->side));
+            CK(launch_decode_i8(pc, list, r1 - r0, ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8, ld_i8, sc, 0,
+                                ctx->side));
             CK(launch_finalize_stats(r1 - r0, n_used, sc, annot_dev ? annot_dev + r0 : nullptr, 1, a->has_pq_exp,
                                      a->pq_exp, ctx->aeff.as<double>() + r0, ctx->l2.as<double>() + r0, ctx->side,
                                      annot_ld_dev));
@@ -1122,16 +1141,17 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         }
         e_side = ev.mark_on(ctx->side);
         ctx->kernels--;  // counted once below
-    } else if (staged_i8) {
-        CK(launch_decode_i8(pv, rr, m, sel, ctx->ops.as<uint8_t>(), ld_i8, st, 0, s));
-    } else if (d) {
+    } else if (!d) {
+        PanelView pc;
+        const uint64_t* list;
+        CK(rows_of(0, m, s, &pc, &list));
+        CK(launch_decode_i8(pc, list, m, staged_i8 ? ctx->ops.as<uint8_t>() : nullptr, staged_i8 ? ld_i8 : 0, st, 0, s));
+    } else {
         // fused: moments + CountSketch rows in one pass over the permuted panel
         CK(launch_sketch_seg(skc->pp.as<uint32_t>() + (rr ? 0 : a->row_begin * skc->pitch_words), skc->pitch_words,
                              rr, m, n_used, skc->segt.as<int32_t>(), d, st, maf_aware ? 1 : 0, 1,
                              ctx->xsk.as<float>(), ld_sk, s));
         e_sk = ev.mark();
-    } else {
-        CK(launch_decode_i8(pv, rr, m, sel, nullptr, 0, st, 0, s));
     }
     ctx->kernels++;
     if (!stream_gram && !overlap) {
@@ -1142,7 +1162,8 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     const uint64_t ld_f64 = round_up(n_used, 128);
     if (!d && !exact_i8) {
         CK(ctx->xf64.ensure((size_t)8 * nmom * ld_f64));
-        CK(launch_decode_f64(pv, rr, m, sel, st, ctx->xf64.as<double>(), ld_f64, s));
+        const PanelView pk{ctx->packed.as<uint8_t>(), nmom, n_used, (n_used + 3) / 4, kp};
+        CK(launch_decode_f64(compact ? pk : pv, compact ? nullptr : rr, m, st, ctx->xf64.as<double>(), ld_f64, s));
         ctx->kernels++;
     }
     const int e1 = ev.mark();
@@ -1298,12 +1319,20 @@ int ldsc_snp_stats(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a
         pv.rows += a->row_begin * panel->pitch;
         pv.n_snp -= a->row_begin;
     }
-    IndivSel sel{a->keep_iids ? ctx->keep.as<int64_t>() : nullptr, n_used};
+    const uint64_t* rr = a->bed_idx ? ctx->recrows.as<uint64_t>() : nullptr;
+    if (a->keep_iids) {
+        const uint64_t kp = round_up((n_used + 3) / 4, 16);
+        CK(ctx->packed.ensure((size_t)kp * m));
+        CK(launch_compact(pv, rr, m, ctx->keep.as<int64_t>(), n_used, ctx->packed.as<uint8_t>(), kp, s));
+        ctx->kernels++;
+        pv = PanelView{ctx->packed.as<uint8_t>(), (uint64_t)m, n_used, (n_used + 3) / 4, kp};
+        rr = nullptr;
+    }
     RecStats st{};
     st.n = ctx->st_n.as<int32_t>();
     st.s = ctx->st_s.as<int32_t>();
     st.q = ctx->st_q.as<int32_t>();
-    CK(launch_decode_i8(pv, a->bed_idx ? ctx->recrows.as<uint64_t>() : nullptr, m, sel, nullptr, 0, st, 0, s));
+    CK(launch_decode_i8(pv, rr, m, nullptr, 0, st, 0, s));
     ctx->kernels++;
     std::vector<int32_t> hn((size_t)m), hs((size_t)m), hq((size_t)m);
     CK(cudaMemcpyAsync(hn.data(), st.n, 4 * (size_t)m, cudaMemcpyDeviceToHost, s));
@@ -1450,7 +1479,6 @@ int ldsc_debug_gram_i8_tile(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t k0,
     CK(ctx->err.ensure(16));
     CK(ctx->dbg.ensure(4 * 128 * 256));
     PanelView pv{panel->rows, panel->n_snp, panel->n_indiv, panel->bpr, panel->pitch};
-    IndivSel sel{nullptr, n};
     RecStats st{};
     st.n = ctx->st_n.as<int32_t>();
     st.s = ctx->st_s.as<int32_t>();
@@ -1459,7 +1487,7 @@ int ldsc_debug_gram_i8_tile(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t k0,
     st.mean = ctx->st_mean.as<double>();
     st.inv_std = ctx->st_inv.as<double>();
     st.qinv = ctx->st_qinv.as<double>();
-    CK(launch_decode_i8(pv, nullptr, m, sel, fused ? nullptr : ctx->ops.as<uint8_t>(), fused ? 0 : ld, st, 0, s));
+    CK(launch_decode_i8(pv, nullptr, m, fused ? nullptr : ctx->ops.as<uint8_t>(), fused ? 0 : ld, st, 0, s));
     CK(launch_finalize_stats(m, n, st, nullptr, 1, 0, 0.0, ctx->aeff.as<double>(), ctx->l2.as<double>(), s));
     CK(cudaMemsetAsync(ctx->left.p, 0, 8 * (size_t)m, s));
     CK(cudaMemsetAsync(ctx->err.p, 0, 16, s));

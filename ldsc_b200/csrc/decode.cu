@@ -19,31 +19,14 @@ namespace {
 
 constexpr uint32_t kEven = 0x55555555u;
 
-// Code word of individuals [i0, i0 + 16); slots past sel.n read as missing.
-__device__ __forceinline__ uint32_t codes16(const uint8_t* __restrict__ row, IndivSel sel,
-                                            uint64_t i0) {
-    if (i0 >= sel.n) return 0x55555555u;  // all missing: padding columns
-    uint32_t w;
-    if (sel.keep == nullptr) {
-        // i0 is a multiple of 16, rows are 16-byte aligned and padded to a
-        // multiple of 16 bytes, so the word load stays inside the row pitch.
-        w = __ldg(reinterpret_cast<const uint32_t*>(row + (i0 >> 2)));
-    } else {
-        w = 0;
-#pragma unroll
-        for (int t = 0; t < 16; t++) {
-            uint64_t i = i0 + t;
-            uint32_t code = 1u;
-            if (i < sel.n) {
-                int64_t iid = __ldg(sel.keep + i);
-                code = (__ldg(row + (iid >> 2)) >> ((iid & 3) * 2)) & 3u;
-            }
-            w |= code << (2 * t);
-        }
-    }
-    if (i0 + 16 > sel.n) {
-        uint32_t valid = sel.n > i0 ? static_cast<uint32_t>(sel.n - i0) : 0u;
-        uint32_t keepm = valid >= 16 ? 0xFFFFFFFFu : ((1u << (2 * valid)) - 1u);
+// Code word of individuals [i0, i0 + 16); slots past n read as missing.
+__device__ __forceinline__ uint32_t codes16(const uint8_t* __restrict__ row, uint64_t n, uint64_t i0) {
+    if (i0 >= n) return 0x55555555u;  // all missing: padding columns
+    // i0 is a multiple of 16, rows are 16-byte aligned and padded to a
+    // multiple of 16 bytes, so the word load stays inside the row pitch.
+    uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(row + (i0 >> 2)));
+    if (i0 + 16 > n) {
+        const uint32_t keepm = (1u << (2 * static_cast<uint32_t>(n - i0))) - 1u;   // n - i0 < 16
         w = (w & keepm) | (0x55555555u & ~keepm);
     }
     return w;
@@ -93,11 +76,11 @@ __device__ __forceinline__ void expand16(uint32_t w, uint8_t* grow, uint8_t* mro
 // A warp decodes 2,048 individuals per step: lane l takes words l, l+32,
 // l+64, l+96 of the step (loads issued together, stores coalesced).
 __global__ void __launch_bounds__(256) k_decode_i8(PanelView p, const uint64_t* __restrict__ rec_rows,
-                                                   int64_t m, IndivSel sel, uint8_t* __restrict__ ops,
-                                                   uint64_t ld, RecStats st, int want_moments) {
+                                                   int64_t m, uint8_t* __restrict__ ops, uint64_t ld,
+                                                   RecStats st, int want_moments) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const uint64_t span = ops ? ld : ((sel.n + 15) & ~uint64_t(15));
+    const uint64_t span = ops ? ld : ((p.n_indiv + 15) & ~uint64_t(15));
     for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < m; r += warps) {
         const uint64_t brow = rec_rows ? rec_rows[r] : (uint64_t)r;
         const uint8_t* row = p.rows + brow * p.pitch;
@@ -107,7 +90,7 @@ __global__ void __launch_bounds__(256) k_decode_i8(PanelView p, const uint64_t* 
         for (uint64_t s0 = 0; s0 < span; s0 += 2048) {
             uint32_t w[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) w[u] = codes16(row, sel, s0 + 512 * u + 16 * lane);
+            for (int u = 0; u < 4; u++) w[u] = codes16(row, p.n_indiv, s0 + 512 * u + 16 * lane);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const uint64_t i0 = s0 + 512 * u + 16 * lane;
@@ -182,8 +165,8 @@ __global__ void k_finalize(int64_t m, uint64_t n_indiv, RecStats st, const doubl
 // Standardised f64 columns (normalize_col_f64_with_stats,
 // src/l2/normalize.rs:71-110): x = (g - mean) * inv_std, missing -> 0.
 __global__ void __launch_bounds__(256) k_decode_f64(PanelView p, const uint64_t* __restrict__ rec_rows,
-                                                    int64_t m, IndivSel sel, RecStats st,
-                                                    double* __restrict__ x, uint64_t ld) {
+                                                    int64_t m, RecStats st, double* __restrict__ x,
+                                                    uint64_t ld) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < m; r += warps) {
@@ -194,7 +177,7 @@ __global__ void __launch_bounds__(256) k_decode_f64(PanelView p, const uint64_t*
         const double v2 = (2.0 - mean) * inv, v1 = (1.0 - mean) * inv, v0 = (0.0 - mean) * inv;
         double* xr = x + (uint64_t)r * ld;
         for (uint64_t i0 = (uint64_t)lane * 16; i0 < ld; i0 += 512) {
-            const uint32_t w = codes16(row, sel, i0);
+            const uint32_t w = codes16(row, p.n_indiv, i0);
             double v[16];
 #pragma unroll
             for (int t = 0; t < 16; t++) {
@@ -229,6 +212,66 @@ __global__ void __launch_bounds__(256) k_repitch(const uint8_t* __restrict__ src
     }
 }
 
+// --keep: rows of the kept individuals alone, in the panel's own packed form
+// (individual i of the output = FAM index keep[i], any order), so that every
+// pass after this one reads whole words.  A thread owns one output word: its
+// sixteen indices stay in registers over the CTA's rows, which are staged in
+// shared memory (double-buffered by cp.async) when two fit; the sixteen byte
+// reads of neighbouring lanes then fall in neighbouring banks.  Bound by the
+// issue of those reads (about five instructions per genotype).  50,021 records
+// x 15,003 of 20,011 individuals: 480 us; decoding through the index list took
+// 3.3 ms, sixteen dependent global loads per word and record.
+constexpr int CROWS = 16;   // rows per CTA
+constexpr size_t COMPACT_SMEM = 96 * 1024;   // two staged rows up to here (196,000 individuals), two CTAs per SM
+constexpr int CT = 256;
+
+template <bool STAGED>
+__global__ void __launch_bounds__(CT) k_compact(PanelView p, const uint64_t* __restrict__ rec_rows, int64_t m,
+                                                const int64_t* __restrict__ keep, uint64_t n_keep,
+                                                uint8_t* __restrict__ out, uint64_t out_pitch) {
+    extern __shared__ __align__(16) uint8_t rows_s[];
+    const uint64_t w = (uint64_t)blockIdx.y * CT + threadIdx.x;   // output word
+    const bool live = w < out_pitch / 4;
+    uint32_t iid[16], valid = 0;
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+        const bool v = live && 16 * w + t < n_keep;
+        iid[t] = v ? (uint32_t)__ldg(keep + 16 * w + t) : 0u;   // n_indiv < 2^32 (checked by the launcher)
+        valid |= (v ? 3u : 0u) << (2 * t);
+    }
+    const int64_t r0 = (int64_t)blockIdx.x * CROWS, r1 = r0 + CROWS < m ? r0 + CROWS : m;
+    auto src_row = [&](int64_t r) { return p.rows + (rec_rows ? rec_rows[r] : (uint64_t)r) * p.pitch; };
+    auto stage = [&](int64_t r) {
+        if (r < r1) {
+            const uint8_t* src = src_row(r);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(rows_s + ((r - r0) & 1) * p.pitch);
+            for (uint64_t q = 16ull * threadIdx.x; q < p.pitch; q += 16ull * CT)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)q), "l"(src + q) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (STAGED) stage(r0);
+    for (int64_t r = r0; r < r1; r++) {
+        const uint8_t* row;
+        if (STAGED) {
+            stage(r + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+            row = rows_s + ((r - r0) & 1) * p.pitch;
+        } else {
+            row = src_row(r);
+        }
+        uint32_t word = 0;
+#pragma unroll
+        for (int t = 0; t < 16; t++) {
+            const uint32_t code = ((uint32_t)row[iid[t] >> 2] >> ((iid[t] & 3u) * 2u)) & 3u;
+            word |= code << (2 * t);
+        }
+        if (live) *reinterpret_cast<uint32_t*>(out + (uint64_t)r * out_pitch + 4 * w) = word & valid;
+        if (STAGED) __syncthreads();   // this buffer is refilled next
+    }
+}
+
 int decode_grid(int64_t m) {
     int64_t blocks = (m + 7) / 8;
     if (blocks > 148 * 16) blocks = 148 * 16;
@@ -238,11 +281,23 @@ int decode_grid(int64_t m) {
 
 }  // namespace
 
-cudaError_t launch_decode_i8(const PanelView& p, const uint64_t* rec_rows, int64_t m, IndivSel sel,
-                             uint8_t* ops, uint64_t ld, RecStats st, int want_moments,
-                             cudaStream_t stream) {
+cudaError_t launch_compact(const PanelView& p, const uint64_t* rec_rows, int64_t m, const int64_t* keep,
+                           uint64_t n_keep, uint8_t* out, uint64_t out_pitch, cudaStream_t stream) {
+    if (m <= 0 || n_keep == 0) return cudaSuccess;
+    if (p.n_indiv >= (1ull << 32) || out_pitch % 16 != 0 || out_pitch < (n_keep + 3) / 4) return cudaErrorInvalidValue;
+    const dim3 grid((unsigned)((m + CROWS - 1) / CROWS), (unsigned)((out_pitch / 4 + CT - 1) / CT));
+    const size_t smem = 2 * p.pitch;
+    if (smem <= COMPACT_SMEM)
+        k_compact<true><<<grid, CT, smem, stream>>>(p, rec_rows, m, keep, n_keep, out, out_pitch);
+    else
+        k_compact<false><<<grid, CT, 0, stream>>>(p, rec_rows, m, keep, n_keep, out, out_pitch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_decode_i8(const PanelView& p, const uint64_t* rec_rows, int64_t m, uint8_t* ops, uint64_t ld,
+                             RecStats st, int want_moments, cudaStream_t stream) {
     if (m <= 0) return cudaSuccess;
-    k_decode_i8<<<decode_grid(m), 256, 0, stream>>>(p, rec_rows, m, sel, ops, ld, st, want_moments);
+    k_decode_i8<<<decode_grid(m), 256, 0, stream>>>(p, rec_rows, m, ops, ld, st, want_moments);
     return cudaGetLastError();
 }
 
@@ -268,16 +323,20 @@ cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st, cons
     return cudaGetLastError();
 }
 
-cudaError_t launch_decode_f64(const PanelView& p, const uint64_t* rec_rows, int64_t m, IndivSel sel,
-                              RecStats st, double* x, uint64_t ld, cudaStream_t stream) {
+cudaError_t launch_decode_f64(const PanelView& p, const uint64_t* rec_rows, int64_t m, RecStats st,
+                              double* x, uint64_t ld, cudaStream_t stream) {
     if (m <= 0) return cudaSuccess;
-    k_decode_f64<<<decode_grid(m), 256, 0, stream>>>(p, rec_rows, m, sel, st, x, ld);
+    k_decode_f64<<<decode_grid(m), 256, 0, stream>>>(p, rec_rows, m, st, x, ld);
     return cudaGetLastError();
 }
 
 cudaError_t preload_decode() {
     cudaError_t e = preload_kernel(k_decode_i8);
     if (e == cudaSuccess) e = preload_kernel(k_finalize);
+    if (e == cudaSuccess) e = preload_kernel(k_compact<false>);
+    if (e == cudaSuccess) e = preload_kernel(k_compact<true>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_compact<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMPACT_SMEM);
     if (e == cudaSuccess) e = preload_kernel(k_decode_f64);
     if (e == cudaSuccess) e = preload_kernel(k_repitch);
     return e;

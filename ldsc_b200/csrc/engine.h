@@ -18,12 +18,6 @@ struct PanelView {
     uint64_t pitch;
 };
 
-// Which individuals a run uses: all (keep == nullptr) or FAM indices keep[i].
-struct IndivSel {
-    const int64_t* keep;  // device pointer or nullptr
-    uint64_t n;           // individuals used
-};
-
 // Per-record statistics produced by the decode kernels (device SoA arrays).
 struct RecStats {
     int32_t* n;        // non-missing count
@@ -84,11 +78,17 @@ struct EpilogueArgs {
 
 // ---- kernels (launchers return cudaError_t of the launch) ----
 
-// Decode + stats (+ optional INT8 genotype/mask operand rows, interleaved:
-// row 2r = genotype, row 2r+1 = non-missing mask, `ld` bytes per row).
-cudaError_t launch_decode_i8(const PanelView& p, const uint64_t* rec_rows, int64_t m,
-                             IndivSel sel, uint8_t* ops, uint64_t ld, RecStats st,
-                             int want_moments, cudaStream_t stream);
+// Packed rows of the kept individuals: output row r, individual i = the code of
+// FAM index keep[i] (device) in record r's panel row; bits past n_keep are 0.
+// out_pitch: a multiple of 16, at least ceil(n_keep / 4).
+cudaError_t launch_compact(const PanelView& p, const uint64_t* rec_rows, int64_t m, const int64_t* keep,
+                           uint64_t n_keep, uint8_t* out, uint64_t out_pitch, cudaStream_t stream);
+
+// Decode + stats over all p.n_indiv individuals (+ optional INT8 genotype/mask
+// operand rows, interleaved: row 2r = genotype, row 2r+1 = non-missing mask,
+// `ld` bytes per row).
+cudaError_t launch_decode_i8(const PanelView& p, const uint64_t* rec_rows, int64_t m, uint8_t* ops, uint64_t ld,
+                             RecStats st, int want_moments, cudaStream_t stream);
 
 // Finalise per-record stats: maf, mean, inv_std, qinv, pq, kappa, aeff.
 cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st,
@@ -102,9 +102,8 @@ cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st,
 cudaError_t launch_repitch(const uint8_t* src, uint64_t bpr, uint8_t* dst, uint64_t pitch, uint64_t r0,
                            uint64_t r1, cudaStream_t stream);
 
-cudaError_t launch_decode_f64(const PanelView& p, const uint64_t* rec_rows, int64_t m,
-                              IndivSel sel, RecStats st, double* x, uint64_t ld,
-                              cudaStream_t stream);
+cudaError_t launch_decode_f64(const PanelView& p, const uint64_t* rec_rows, int64_t m, RecStats st, double* x,
+                              uint64_t ld, cudaStream_t stream);
 
 // FP64 band Gram + unbiased-r^2 epilogue (TA = TB = 128 records per tile).
 cudaError_t launch_gram_f64(const double* x, uint64_t ld, uint64_t kdim, const Tile* tiles,

@@ -131,7 +131,6 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     if ((rc = ck(cudaMemsetAsync(base + o_err, 0, 16, s), "clear error word"))) return rc;
 
     PanelView pv{d_rows, m, n_indiv, (n_indiv + 3) / 4, pitch};
-    IndivSel sel{nullptr, n_indiv};
     RecStats st{};
     st.n = reinterpret_cast<int32_t*>(base + o_n);
     st.s = reinterpret_cast<int32_t*>(base + o_s);
@@ -141,7 +140,7 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     st.inv_std = reinterpret_cast<double*>(base + o_inv);
     st.qinv = reinterpret_cast<double*>(base + o_qinv);
     uint8_t* ops = base + o_ops;
-    if ((rc = ck(launch_decode_i8(pv, nullptr, (int64_t)m, sel, ops, ld, st, 0, s), "decode"))) return rc;
+    if ((rc = ck(launch_decode_i8(pv, nullptr, (int64_t)m, ops, ld, st, 0, s), "decode"))) return rc;
     if ((rc = ck(launch_finalize_stats((int64_t)m, n_indiv, st, nullptr, 1, 0, 0.0,
                                        reinterpret_cast<double*>(base + o_aeff), d_l2, s),
                  "finalize")))

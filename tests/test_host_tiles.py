@@ -1,7 +1,5 @@
 """The Gram's tile list (host plan) against its definition: every in-band pair
 lies in exactly one tile, whole or trimmed, for windows of every width."""
-import ctypes as C
-
 import numpy as np
 import pytest
 
@@ -11,7 +9,6 @@ import pytest
 def test_every_pair_lies_in_one_tile(m, trim, max_quarters):
     from ldsc_b200 import _lib
     lib = _lib.load()
-    lib.ldsc_debug_gram_tiles.restype = C.c_int64
     rng = np.random.default_rng(m)
     for width in (0, 1, 17, 130, 10 ** 6):
         # non-decreasing limits with jumps (chromosome starts), and one list that is not monotone
@@ -19,8 +16,7 @@ def test_every_pair_lies_in_one_tile(m, trim, max_quarters):
         for lim in (left, np.maximum(np.arange(m) - rng.integers(0, width + 1, m), 0)):
             lim = np.ascontiguousarray(lim, dtype=np.int64)
             out = np.zeros((4 * (m // 128 + 1) ** 2 + 4, 4), dtype=np.uint32)
-            n = lib.ldsc_debug_gram_tiles(lim.ctypes.data_as(C.c_void_p), C.c_uint64(m), trim, max_quarters,
-                                          out.ctypes.data_as(C.c_void_p), C.c_uint64(len(out)))
+            n = lib.ldsc_debug_gram_tiles(lim.ctypes.data, m, trim, max_quarters, out.ctypes.data, len(out))
             assert 0 <= n <= len(out)
             seen = np.zeros((m + 128, m + 128), dtype=np.int32)
             for a, b, q0, nq in out[:n]:

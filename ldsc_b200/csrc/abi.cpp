@@ -122,7 +122,7 @@ struct ldsc_ctx {
     std::string last_error;
     uint64_t kernels = 0;
     // workspace (grow-only)
-    DevBuf ops, xf64, xsk, recrows, keep, left, tiles, annot, aeff, l2, maf, pq, err;
+    DevBuf ops, blocks, xsk, recrows, keep, left, tiles, annot, aeff, l2, maf, pq, err;
     DevBuf st_n, st_s, st_q, st_q3, st_q4, st_mean, st_inv, st_qinv, st_kappa, packed, tsum, dbg;
     // private CountSketch layout (explicit bucket/sign arrays, or a panel
     // whose shared layout is in use under another key)
@@ -142,13 +142,14 @@ struct ldsc_ctx {
     std::vector<Tile> plan_tiles;
     std::vector<int32_t> plan_ptr_r, plan_idx_r, plan_ptr_l, plan_idx_l;  // CSR tile lists
     std::vector<uint32_t> plan_roff;
+    std::vector<GramBlock> plan_blocks;
     // whole-file entry: staged file rows, the pitched panel, per-chunk events
     DevBuf bed_stage, bed_rows;
     std::vector<cudaEvent_t> feed_ev;
     cudaEvent_t feed_t0 = nullptr, feed_t1 = nullptr, feed_go = nullptr, up_ev = nullptr;
 
     std::vector<DevBuf*> workspace() {
-        return {&ops, &xf64, &xsk, &recrows, &keep, &left,
+        return {&ops, &blocks, &xsk, &recrows, &keep, &left,
                       &tiles, &annot, &aeff, &l2, &maf,
                       &pq, &err, &st_n, &st_s, &st_q, &st_q3,
                       &st_q4, &st_mean, &st_inv, &st_qinv, &st_kappa,
@@ -218,7 +219,7 @@ int ldsc_ctx_create(int device, uint32_t flags, ldsc_ctx** out) {
         static std::vector<int> preloaded;
         std::lock_guard<std::mutex> g(preload_mu);
         if (std::find(preloaded.begin(), preloaded.end(), device) == preloaded.end()) {
-            for (cudaError_t (*f)() : {preload_gram_tc, preload_gram_simt, preload_decode, preload_sketch,
+            for (cudaError_t (*f)() : {preload_gram_tc, preload_gram_f64, preload_decode, preload_sketch,
                                        preload_contract, preload_synth, preload_regress, preload_partitioned})
                 if (f() != cudaSuccess) {
                     cudaGetLastError();
@@ -453,8 +454,9 @@ int ldsc_l2_workspace_bytes(const ldsc_l2_args* a, uint64_t n_indiv, uint64_t* b
     const uint64_t K = a->annot ? a->n_annot : 1;
     const uint32_t d = a->sketch_d;
     const bool exact_i8 = !d && a->precision == LDSC_PRECISION_INT8;
+    const bool f64 = !d && !exact_i8;
     std::vector<Tile> tl;
-    gram_tiles(L.left, gram_trims(d ? 4 * round_up(d, 32) : round_up(n_used, 128)), 4, &tl);
+    gram_tiles(L.left, f64 || gram_trims(d ? 4 * round_up(d, 32) : round_up(n_used, 128)), 4, &tl);
     uint64_t quarters = 0;
     for (const Tile& t : tl) quarters += t.nq1 + 1u;
     // a run with fewer tiles than SMs cuts them finer, up to one per SM
@@ -466,13 +468,14 @@ int ldsc_l2_workspace_bytes(const ldsc_l2_args* a, uint64_t n_indiv, uint64_t* b
     b += (K > 1 ? (uint64_t)8 * TILE_RECORDS * TILE_QUARTER * (quarters + quarters / 8) + 4 * nt_room
                 : (uint64_t)8 * 2 * TILE_RECORDS * nt_room) +
          8 * nt_room + 4 * (2 * (m / 128) + 4);
+    // FP64: up to sixteen 32 x 32 blocks per tile (list, and with K = 1 their sums and CSR entries)
+    if (f64) b += 16 * nt_room * (sizeof(GramBlock) + (K == 1 ? 8 * 64 + 16 : 0)) + (K == 1 ? 4 * (2 * (m / 32) + 4) : 0);
     if (a->annot && !a->annot_on_device) b += 8 * m * K;
     if (a->bed_idx) b += 8 * m;
     if (a->keep_iids) b += 8 * a->n_keep + (d ? 0 : m * round_up((n_used + 3) / 4, 16));  // indices, compacted rows
     // INT8 operand rows (the default two-pass form; an upper bound for the fused one)
     if (exact_i8) b += 2 * m * round_up(n_used, 128);
     else if (d) b += 8 * m * round_up(d, 32);
-    else b += 8 * m * round_up(n_used, 128);
     *bytes = b;
     return LDSC_OK;
 }
@@ -748,7 +751,9 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     // place when the records are the panel rows in order and every individual
     // is used
     const bool fused_i8 = exact_i8 && !a->bed_idx && !a->keep_iids && (ctx->flags & LDSC_CTX_FUSED_OPERANDS);
-    const int ta = TILE_RECORDS, tb = TILE_RECORDS;
+    const bool f64 = !d && !exact_i8;
+    // records per side of the tiles behind the K = 1 sums (FP64: a warp's 32 x 32 blocks)
+    const int ta = f64 && K == 1 ? 32 : TILE_RECORDS, tb = ta;
     pf.gram_kind = d ? 2u : (exact_i8 ? 1u : 0u);
 
     cudaStream_t s = ctx->stream;
@@ -919,8 +924,10 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         if (L.any_full && !a->yes_really)
             std::printf("WARNING: LD window spans the entire chromosome. Use --yes-really to silence this warning.\n");
         pf.n_pairs = L.n_pairs;
-        const bool trim = gram_trims(d ? 4 * round_up(d, 32) : round_up(n_used, 128));
-        if (K == 1 && (d || exact_i8))
+        const bool trim = f64 || gram_trims(d ? 4 * round_up(d, 32) : round_up(n_used, 128));
+        if (f64 && K == 1)
+            gram_blocks(L.left, &tiles, &ctx->plan_blocks);
+        else if (K == 1)
             gram_tiles_for(L.left, trim, ctx->sms, &tiles);
         else
             gram_tiles(L.left, trim, 4, &tiles);
@@ -970,6 +977,13 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             } else {
                 CK(ctx->prow.ensure(sizeof(double) * (size_t)ta * nt_room));
                 CK(ctx->pcol.ensure(sizeof(double) * (size_t)tb * nt_room));
+            }
+            if (f64) {
+                if (K > 1) gram_blocks_of(tiles, ctx->plan_roff, &ctx->plan_blocks);
+                const size_t nb = ctx->plan_blocks.size();
+                CK(ctx->blocks.ensure(sizeof(GramBlock) * (nb + nb / 8)));
+                CK(cudaMemcpyAsync(ctx->blocks.p, ctx->plan_blocks.data(), sizeof(GramBlock) * nb, cudaMemcpyHostToDevice,
+                                   up));
             }
             CK(ctx->cptr_r.ensure(4 * ptr_r.size()));
             CK(ctx->cidx_r.ensure(4 * nt_room));
@@ -1159,13 +1173,6 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                                  ctx->l2.as<double>(), s, annot_ld_dev));
         ctx->kernels++;
     }
-    const uint64_t ld_f64 = round_up(n_used, 128);
-    if (!d && !exact_i8) {
-        CK(ctx->xf64.ensure((size_t)8 * nmom * ld_f64));
-        const PanelView pk{ctx->packed.as<uint8_t>(), nmom, n_used, (n_used + 3) / 4, kp};
-        CK(launch_decode_f64(compact ? pk : pv, compact ? nullptr : rr, m, st, ctx->xf64.as<double>(), ld_f64, s));
-        ctx->kernels++;
-    }
     const int e1 = ev.mark();
 
     if (!stream_gram) {
@@ -1222,8 +1229,9 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>(), (int64_t)tiles.size(), ep,
                               nullptr, 0, ctx->sms, s));
         } else {
-            CK(launch_gram_f64(ctx->xf64.as<double>(), ld_f64, ld_f64, ctx->tiles.as<Tile>(), (int64_t)tiles.size(),
-                               ep, ctx->sms, s));
+            const PanelView pk{ctx->packed.as<uint8_t>(), nmom, n_used, (n_used + 3) / 4, kp};
+            CK(launch_gram_f64(compact ? pk : pv, compact ? nullptr : rr, st, ctx->blocks.as<GramBlock>(),
+                               (uint32_t)ctx->plan_blocks.size(), ctx->err.as<unsigned int>() + 1, ep, ctx->sms, s));
         }
         ctx->kernels++;
         e_c = ev.mark();

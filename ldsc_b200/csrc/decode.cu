@@ -162,36 +162,6 @@ __global__ void k_finalize(int64_t m, uint64_t n_indiv, RecStats st, const doubl
     }
 }
 
-// Standardised f64 columns (normalize_col_f64_with_stats,
-// src/l2/normalize.rs:71-110): x = (g - mean) * inv_std, missing -> 0.
-__global__ void __launch_bounds__(256) k_decode_f64(PanelView p, const uint64_t* __restrict__ rec_rows,
-                                                    int64_t m, RecStats st, double* __restrict__ x,
-                                                    uint64_t ld) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < m; r += warps) {
-        const uint64_t brow = rec_rows ? rec_rows[r] : (uint64_t)r;
-        const uint8_t* row = p.rows + brow * p.pitch;
-        const double mean = st.mean[r];
-        const double inv = st.inv_std[r];
-        const double v2 = (2.0 - mean) * inv, v1 = (1.0 - mean) * inv, v0 = (0.0 - mean) * inv;
-        double* xr = x + (uint64_t)r * ld;
-        for (uint64_t i0 = (uint64_t)lane * 16; i0 < ld; i0 += 512) {
-            const uint32_t w = codes16(row, p.n_indiv, i0);
-            double v[16];
-#pragma unroll
-            for (int t = 0; t < 16; t++) {
-                const uint32_t c = (w >> (2 * t)) & 3u;
-                v[t] = c == 0 ? v2 : (c == 2 ? v1 : (c == 3 ? v0 : 0.0));
-            }
-#pragma unroll
-            for (int t = 0; t < 16; t += 2) {
-                *reinterpret_cast<double2*>(xr + i0 + t) = make_double2(v[t], v[t + 1]);
-            }
-        }
-    }
-}
-
 // One thread per 4-byte word of the pitched rows; the source is the file's
 // unpadded rows, read byte-wise (their starts are not word aligned).
 __global__ void __launch_bounds__(256) k_repitch(const uint8_t* __restrict__ src, uint64_t bpr,
@@ -323,13 +293,6 @@ cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st, cons
     return cudaGetLastError();
 }
 
-cudaError_t launch_decode_f64(const PanelView& p, const uint64_t* rec_rows, int64_t m, RecStats st,
-                              double* x, uint64_t ld, cudaStream_t stream) {
-    if (m <= 0) return cudaSuccess;
-    k_decode_f64<<<decode_grid(m), 256, 0, stream>>>(p, rec_rows, m, st, x, ld);
-    return cudaGetLastError();
-}
-
 cudaError_t preload_decode() {
     cudaError_t e = preload_kernel(k_decode_i8);
     if (e == cudaSuccess) e = preload_kernel(k_finalize);
@@ -337,7 +300,6 @@ cudaError_t preload_decode() {
     if (e == cudaSuccess) e = preload_kernel(k_compact<true>);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_compact<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMPACT_SMEM);
-    if (e == cudaSuccess) e = preload_kernel(k_decode_f64);
     if (e == cudaSuccess) e = preload_kernel(k_repitch);
     return e;
 }

@@ -33,7 +33,7 @@ struct RecStats {
     double* pq;        // (maf (1 - maf))^pq_exp, may be null
 };
 
-// Records per side of a band tile (left block x right block), every form.
+// Records per side of a band tile (left block x right block).
 constexpr int TILE_RECORDS = 128;
 
 constexpr int TILE_QUARTER = TILE_RECORDS / 4;
@@ -96,18 +96,22 @@ cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st,
                                   double* aeff, double* l2_init,
                                   cudaStream_t stream, uint64_t annot_ld = 0);
 
-// Standardised f64 columns, row r of `x` = record r, `ld` doubles per row.
 // Rows [r0, r1) of a packed BED body (bpr bytes per row, as in the file) to
 // the pitched panel layout; pad bytes are zeroed.
 cudaError_t launch_repitch(const uint8_t* src, uint64_t bpr, uint8_t* dst, uint64_t pitch, uint64_t r0,
                            uint64_t r1, cudaStream_t stream);
 
-cudaError_t launch_decode_f64(const PanelView& p, const uint64_t* rec_rows, int64_t m, RecStats st, double* x,
-                              uint64_t ld, cudaStream_t stream);
+// 32 x 32 records of the FP64 form: left records 32 a .., right records 32 b ..;
+// slot: K = 1, the block's place in prow / pcol (32 sums each); K > 1, the
+// quarter of rtiles that holds its right records.
+struct GramBlock {
+    uint32_t a, b, slot;
+};
 
-// FP64 band Gram + unbiased-r^2 epilogue (TA = TB = 128 records per tile).
-cudaError_t launch_gram_f64(const double* x, uint64_t ld, uint64_t kdim, const Tile* tiles,
-                            int64_t n_tiles, const EpilogueArgs& ep, int sms,
+// FP64 band Gram over the packed rows of all p.n_indiv individuals +
+// unbiased-r^2 epilogue.  next: a zeroed device word (block counter).
+cudaError_t launch_gram_f64(const PanelView& p, const uint64_t* rec_rows, RecStats st, const GramBlock* blocks,
+                            uint32_t n_blocks, unsigned int* next, const EpilogueArgs& ep, int sms,
                             cudaStream_t stream);
 
 // Whether a tcgen05 Gram over operand rows of row_bytes gains from tiles
@@ -165,11 +169,6 @@ bool sketch_supported(uint64_t n_used, uint32_t d);
 cudaError_t launch_gram_tf32(const float* ops, uint64_t ld, int64_t m, const Tile* tiles, int64_t n_tiles,
                              const EpilogueArgs& ep, int maf_aware, int sms, cudaStream_t stream);
 
-// FP32 band Gram of sketched rows + quadratic bias correction epilogue.
-cudaError_t launch_gram_f32(const float* x, uint64_t ld, uint64_t kdim, const Tile* tiles,
-                            int64_t n_tiles, const EpilogueArgs& ep, int maf_aware, int sms,
-                            cudaStream_t stream);
-
 // K > 1 annotation contraction from the R tiles a Gram wrote (no atomics, each
 // l2 row owned by one CTA per pass), ep.rtiles / ep.roff:
 //   by right block:  l2[j, C] += sum over tiles of block, sum_k R[k][j] a[k, C]
@@ -188,7 +187,7 @@ cudaError_t preload_kernel(F* kernel) {
     return cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(kernel));
 }
 cudaError_t preload_gram_tc();
-cudaError_t preload_gram_simt();
+cudaError_t preload_gram_f64();
 cudaError_t preload_decode();
 cudaError_t preload_sketch();
 cudaError_t preload_contract();

@@ -234,6 +234,21 @@ void gram_tiles_for(const std::vector<int64_t>& left, bool trim, int sms, std::v
     }
 }
 
+void gram_blocks(const std::vector<int64_t>& left, std::vector<Tile>* scratch, std::vector<GramBlock>* blocks) {
+    band_tiles(left, 32, 32, scratch);
+    blocks->resize(scratch->size());
+    for (size_t i = 0; i < scratch->size(); i++)
+        (*blocks)[i] = GramBlock{(*scratch)[i].a_blk, (*scratch)[i].b_blk, (uint32_t)i};
+}
+
+void gram_blocks_of(const std::vector<Tile>& tiles, const std::vector<uint32_t>& roff, std::vector<GramBlock>* blocks) {
+    blocks->clear();
+    for (size_t t = 0; t < tiles.size(); t++)
+        for (uint32_t q = 0; q <= tiles[t].nq1; q++)
+            for (uint32_t a = 0; a < 4; a++)
+                blocks->push_back(GramBlock{4 * tiles[t].a_blk + a, 4 * tiles[t].b_blk + tiles[t].q0 + q, roff[t] + q});
+}
+
 // ---- fastrand 2.3.0 WyRand (independent restatement of the published
 // algorithm; the crate is not vendored with the reference) ----
 namespace {

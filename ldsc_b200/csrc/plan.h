@@ -35,6 +35,12 @@ bool left_limits(int64_t m, const uint8_t* chr, const double* cm, const uint32_t
                  double wind, uint64_t half, uint32_t chunk, bool masking, bool global_pass,
                  LeftLimits* out, std::string* err);
 
+// The FP64 form's blocks: K = 1, the 32 x 32 blocks that hold in-band pairs,
+// by right block, then left block, numbered in order; K > 1, every block of the
+// tiles' quarters, numbered by quarter (tile t's first is roff[t]).
+void gram_blocks(const std::vector<int64_t>& left, std::vector<Tile>* scratch, std::vector<GramBlock>* blocks);
+void gram_blocks_of(const std::vector<Tile>& tiles, const std::vector<uint32_t>& roff, std::vector<GramBlock>* blocks);
+
 // Band tiles of ta x tb records covering every pair left[j] <= k < j; the
 // second form refills *out, keeping its storage.
 std::vector<Tile> band_tiles(const std::vector<int64_t>& left, int ta, int tb);

@@ -62,3 +62,26 @@ def test_sketch_tiles_match_the_oracle(ctx, m, per_cm, maf_aware):
                                  masking=True, use_f32=True, sketch_d=d, sketch_maf_aware=maf_aware))[0]
     panel.close()
     assert np.max(np.abs(got - ref)) < SKETCH_TOL
+
+
+@pytest.mark.parametrize("K", [1, 3])
+@pytest.mark.parametrize("m,per_cm,n", [(1, 10, 5), (2, 10, 16), (31, 60, 17), (32, 20, 130), (33, 300, 15),
+                                        (129, 45, 64), (300, 90, 133), (300, 2000, 31)])
+def test_fp64_blocks_match_the_definition(ctx, m, per_cm, n, K):
+    """The FP64 form's 32 x 32 blocks at their edges, words of sixteen individuals
+    that end in the row, and a record list."""
+    from conftest import brute_force_l2
+    from ldsc_b200.api import WindowMode, left_limits, run_l2
+    body, snps = _panel(m, n, per_cm, seed=m + per_cm + n)
+    pick = np.arange(0, m, 2) if m > 32 else np.arange(m)
+    for idx in (np.arange(m), pick):
+        sub = BimTable(snps.chr[idx], [f"rs{i}" for i in idx], snps.cm[idx], snps.bp[idx], idx.astype(np.int64))
+        A = None if K == 1 else np.random.default_rng(m).standard_normal((len(idx), K))
+        panel = ctx.upload(body, n)
+        for masking in (True, False):
+            l2, _, _ = run_l2(ctx, sub, panel, WindowMode.Cm(1.0), 40, annot=A, snp_level_masking=masking,
+                              precision="fp64", yes_really=True)
+            left = left_limits(sub, WindowMode.Cm(1.0), 40, snp_level_masking=masking)
+            ref, _ = brute_force_l2(body[idx], n, sub.chr, sub.cm, sub.bp, left, annot=A)
+            assert np.max(np.abs(l2 - ref) / np.maximum(np.abs(ref), 1.0)) < EXACT_TOL
+        panel.close()

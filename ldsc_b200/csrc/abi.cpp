@@ -1902,7 +1902,7 @@ extern "C" int ldsc_h2_partitioned(ldsc_ctx* ctx, const ldsc_h2p_args* a, ldsc_h
                                   fixed, d_w, n, gb, m_tot, ctx->p_m.as<double>(), ctx->p_xtot.as<double>(), first,
                                   ctx->p_part.as<double>(), ctx->p_gram.as<double>(), ctx->p_tot.as<double>(),
                                   ctx->p_sol.as<double>(), ctx->p_res.as<double>() + ro, nj, s));
-            ctx->kernels += first ? 7 : 6;
+            ctx->kernels += first ? 8 : 7;
             first = false;
             ro += (size_t)nj * part_result_len(gb, K, P);
         }

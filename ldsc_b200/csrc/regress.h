@@ -118,8 +118,6 @@ __host__ __device__ inline int part_params(int k, bool fixed) { return k + (fixe
 // nb x p, h2 per annotation k, then h2_total, h2_total_se, intercept,
 // intercept_se, nbar, mean_chi2, n_obs.
 __host__ __device__ inline size_t part_result_len(int nb, int k, int p) { return (size_t)p * (1 + p + nb) + k + 7; }
-// Shared memory of one delete-value solve (p x (p + 1) doubles) is capped here.
-constexpr int PART_SOLVE_SMEM = 210 * 1024;
 // Traits per launch: the block Grams of a launch (traits x nb x q^2 doubles)
 // stay within 1 GiB.
 inline int part_trait_chunk(int traits, int nb, int q) {

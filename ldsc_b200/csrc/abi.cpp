@@ -93,7 +93,7 @@ struct GraphCache {
 struct SketchCache {
     DevBuf perm, seg, segt, pp;
     uint64_t n = 0, key = 0, pitch_words = 0;
-    uint32_t d = 0;
+    uint32_t d = 0, max_run = 0;   // max_run: the longest (bucket, sign) run
     bool valid = false;
     bool matches(uint64_t n_, uint32_t d_, uint64_t key_) const { return valid && n == n_ && d == d_ && key == key_; }
     void release() {
@@ -549,13 +549,17 @@ int sketch_prepare(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t n_used, uint
     CK(cudaMemcpyAsync(c.seg.p, o.seg_off.data(), 4 * o.seg_off.size(), cudaMemcpyHostToDevice, s));
     PanelView pv{panel->rows, panel->n_snp, panel->n_indiv, panel->bpr, panel->pitch};
     CK(launch_sketch_permute(pv, c.perm.as<int32_t>(), n_used, c.pp.as<uint32_t>(), pitch_words, s));
-    CK(c.segt.ensure(4 * (size_t)sketch_segt_count(n_used, d)));
-    CK(launch_sketch_segt(c.seg.as<int32_t>(), n_used, d, c.segt.as<int32_t>(), s));
+    uint32_t max_run = 0;
+    for (size_t i = 1; i < o.seg_off.size(); i++)
+        max_run = std::max(max_run, (uint32_t)(o.seg_off[i] - o.seg_off[i - 1]));
+    CK(c.segt.ensure(4 * (size_t)sketch_segt_count(n_used, d, max_run)));
+    CK(launch_sketch_segt(c.seg.as<int32_t>(), n_used, d, max_run, c.segt.as<int32_t>(), s));
     ctx->kernels += 2;
     // host vectors go out of scope, and other streams may read the layout next
     CK(cudaStreamSynchronize(s));
     c.n = n_used;
     c.d = d;
+    c.max_run = max_run;
     c.key = key;
     c.pitch_words = pitch_words;
     c.valid = true;
@@ -1163,7 +1167,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     } else {
         // fused: moments + CountSketch rows in one pass over the permuted panel
         CK(launch_sketch_seg(skc->pp.as<uint32_t>() + (rr ? 0 : a->row_begin * skc->pitch_words), skc->pitch_words,
-                             rr, m, n_used, skc->segt.as<int32_t>(), d, st, maf_aware ? 1 : 0, 1,
+                             rr, m, n_used, skc->segt.as<int32_t>(), d, skc->max_run, st, maf_aware ? 1 : 0, 1,
                              ctx->xsk.as<float>(), ld_sk, s));
         e_sk = ev.mark();
     }
@@ -1454,7 +1458,7 @@ int ldsc_sketch_project(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t b, uint
     st.s = ctx->st_s.as<int32_t>();
     st.q = ctx->st_q.as<int32_t>();
     CK(launch_sketch_seg(ctx->sk.pp.as<uint32_t>(), ctx->sk.pitch_words, ctx->recrows.as<uint64_t>(), m, n_used,
-                         ctx->sk.segt.as<int32_t>(), d, st, 0, 0, ctx->xsk.as<float>(), d, s));
+                         ctx->sk.segt.as<int32_t>(), d, ctx->sk.max_run, st, 0, 0, ctx->xsk.as<float>(), d, s));
     ctx->kernels += 1;
     CK(cudaMemcpyAsync(out, ctx->xsk.p, 4 * (size_t)m * d, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));

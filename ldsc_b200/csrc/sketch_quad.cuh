@@ -37,32 +37,12 @@ __host__ __device__ __forceinline__ void quad_counts(uint4 v, int32_t& bits, int
     miss = popc32(v.x & ~v.y) + popc32(v.z & ~v.w);
 }
 
-// The same, with the bits and missing positions of the first half (0..31).
-__host__ __device__ __forceinline__ void quad_counts(uint4 v, int32_t& bits, int32_t& miss, int32_t& high,
-                                                     int32_t& bits0, int32_t& miss0) {
-    const int32_t cy = popc32(v.y), cw = popc32(v.w);
-    bits0 = popc32(v.x) + cy;
-    miss0 = popc32(v.x & ~v.y);
-    high = cy + cw;
-    bits = bits0 + popc32(v.z) + cw;
-    miss = miss0 + popc32(v.z & ~v.w);
-}
-
 // Bits and missing positions at quad positions [0, j), 0 <= j < 64.
 __host__ __device__ __forceinline__ void quad_head(uint4 v, uint32_t j, int32_t& bits, int32_t& miss) {
     const uint32_t m0 = j >= 32 ? 0xFFFFFFFFu : (j ? 0xFFFFFFFFu >> (32 - j) : 0u);
     const uint32_t m1 = j > 32 ? 0xFFFFFFFFu >> (64 - j) : 0u;
     bits = popc32(v.x & m0) + popc32(v.y & m0) + popc32(v.z & m1) + popc32(v.w & m1);
     miss = popc32(v.x & ~v.y & m0) + popc32(v.z & ~v.w & m1);
-}
-
-// Bits and missing positions at half positions [0, j), 0 <= j < 32, from the
-// half's (low, high) plane words.
-__host__ __device__ __forceinline__ void half_head(uint32_t lo, uint32_t hi, uint32_t j, int32_t& bits,
-                                                   int32_t& miss) {
-    const uint32_t m = j ? 0xFFFFFFFFu >> (32 - j) : 0u;
-    bits = popc32(lo & m) + popc32(hi & m);
-    miss = popc32(lo & ~hi & m);
 }
 
 }  // namespace ldsc

@@ -195,11 +195,10 @@ __host__ __device__ constexpr uint32_t idesc_tf32(uint32_t M, uint32_t N) {
            | ((M >> 4) << 24);    // m_dim
 }
 
-// Round an f32 to TF32 (round to nearest, ties away), low 13 bits cleared.
+// Round a finite f32 to TF32 (round to nearest, ties away), low 13 bits cleared:
+// half of the last kept place added to the magnitude, the rest cut off.
 __device__ __forceinline__ float to_tf32(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return __uint_as_float(r);
+    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
 }
 
 // 32 lanes x 32 bits, 8 consecutive columns per thread.

@@ -52,8 +52,10 @@
 //              that lies inside the band (X to double, X^2, row and column
 //              terms, butterfly), with 1/(nV) of the row, the column and the
 //              constant -1/(N-2) applied to the sums: about 10,000
-//              clocks per tile (sketch: 19,000, f32 square root and division per
-//              pair), 13 f64 instructions per pair before.
+//              clocks per tile, 13 f64 instructions per pair before (sketch: 12,000
+//              with the f32 root and quotient of sqrt_nr and div_nr, 19,000 with
+//              the IEEE ones and their branches; 50,000 records, d = 200: 378 -> 315
+//              us per launch).
 //              With K > 1 annotation columns the epilogue stores each tile's
 //              masked r2u values (f64, [j][k]) for the contraction of
 //              contract.cu.
@@ -170,6 +172,24 @@ __device__ __forceinline__ double sketch_r2u(float val, double kap, const Epilog
     return r2 * ep.r2u_a + ep.r2u_b;
 }
 
+// Square root and quotient of normal f32 numbers well inside the range: the
+// hardware's approximation and one correction from the exact remainder
+// (Newton's step for the root, Markstein's final correction for the quotient),
+// with no branch for special cases.  Against the IEEE operations: all 226
+// million x in [8, 2^30) equal; 1 of 3 billion quotients differs, by one place.
+__device__ __forceinline__ float sqrt_nr(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float s = x * y;
+    return fmaf(fmaf(-s, s, x), 0.5f * y, s);
+}
+__device__ __forceinline__ float div_nr(float a, float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    const float q = a * y;
+    return fmaf(fmaf(-q, b, a), y, q);
+}
+
 // Sketch constants in f32 for sketch_r2u_f32.
 struct SketchF {
     float n_inv_sq, d, r2u_a, r2u_b;
@@ -191,7 +211,11 @@ __device__ __forceinline__ float sketch_r2u_f32(float val, double kap2, const Sk
     const float dm3 = cf.d - 3.f - 2.f * kap;
     const float q = fmaf(cf.d, tilde, -1.f);
     const float disc = fmaf(dm3, dm3, 8.f * q);
-    const float r2 = disc >= 0.f ? 2.f * q / (sqrtf(disc) + dm3) : 0.f;
+    float r2;
+    if (MODE == 1 || dm3 >= 4.f)   // disc >= dm3^2 - 8 >= 8 (not MAF-aware: dm3 >= 5)
+        r2 = div_nr(2.f * q, sqrt_nr(disc) + dm3);
+    else
+        r2 = disc >= 0.f ? 2.f * q / (sqrtf(disc) + dm3) : 0.f;
     return fmaf(r2, cf.r2u_a, cf.r2u_b);
 }
 
@@ -526,9 +550,10 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                     else
                         for (int c = 0; c < 8 * nq; c++) rt[(size_t)c * TA] = 0.0;
                 } else {
-                    // WHAT 0: K = 1, raw; 1: K = 1; 2: K > 1
-                    auto finish = [&](auto what) {
+                    // WHAT 0: K = 1, raw; 1: K = 1; 2: K > 1.  F32: sketch, the f32 form of r2u
+                    auto finish = [&](auto what, auto f32) {
                         constexpr int WHAT = decltype(what)::value;
+                        constexpr bool F32 = decltype(f32)::value;
                         const double ck = WHAT == 0 ? qk * ak : qk * ep.r2u_a;
 #pragma unroll 1
                         for (int ch = 0; ch < nq; ch++) {
@@ -569,8 +594,8 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                                     const float val = (__uint_as_float(v[0][i]) + __uint_as_float(v[1][i])) +
                                                       (__uint_as_float(v[2][i]) + __uint_as_float(v[3][i]));
                                     const double kap = MODE == 2 ? qk + E.qa[cb + i].x : 0.0;
-                                    r2u = f32_corr ? (double)sketch_r2u_f32<MODE>(val, kap, cf)
-                                                   : sketch_r2u<MODE>(val, kap, ep);
+                                    r2u = F32 ? (double)sketch_r2u_f32<MODE>(val, kap, cf)
+                                              : sketch_r2u<MODE>(val, kap, ep);
                                 }
                                 if (WHAT == 0) {
                                     rs[i & 1] = fma(x2, E.qw[cb + i], rs[i & 1]);
@@ -599,12 +624,18 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                             }
                         }
                     };
-                    if (ep.K != 1)
-                        finish(std::integral_constant<int, 2>{});
-                    else if (MODE == 0 && raw)
-                        finish(std::integral_constant<int, 0>{});
+                    auto finish_k = [&](auto f32) {
+                        if (ep.K != 1)
+                            finish(std::integral_constant<int, 2>{}, f32);
+                        else if (MODE == 0 && raw)
+                            finish(std::integral_constant<int, 0>{}, f32);
+                        else
+                            finish(std::integral_constant<int, 1>{}, f32);
+                    };
+                    if (MODE != 0 && f32_corr)
+                        finish_k(std::true_type{});
                     else
-                        finish(std::integral_constant<int, 1>{});
+                        finish_k(std::false_type{});
                 }
                 if (ep.K == 1) {
                     double rsum = rs[0] + rs[1];

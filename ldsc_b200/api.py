@@ -453,6 +453,12 @@ def _f64(a):
     return np.ascontiguousarray(a, dtype=np.float64)
 
 
+def result_array(out) -> np.ndarray:
+    """A ctypes array of result structures (all doubles) as a structured array of its own."""
+    dtype = np.dtype([(f, np.float64) for f, _ in out._type_._fields_])
+    return np.ndarray(len(out), dtype=dtype, buffer=out).copy()
+
+
 def h2_batch(ctx: Context, chi2, n, ref_l2, w_l2, m_snps: float, n_blocks: int = 200,
              intercept: Optional[float] = None, lambda_gc: bool = True,
              two_step: Optional[float] = None) -> np.ndarray:
@@ -473,9 +479,7 @@ def h2_batch(ctx: Context, chi2, n, ref_l2, w_l2, m_snps: float, n_blocks: int =
                     two_step_cutoff=float(two_step or 0.0))
     out = (L.H2Result * T)()
     ctx.check(ctx.lib.ldsc_h2_batch(ctx.h, C.byref(args), C.cast(out, C.c_void_p)))
-    names = [f for f, _ in L.H2Result._fields_]
-    return np.array([tuple(getattr(r, f) for f in names) for r in out],
-                    dtype=[(f, np.float64) for f in names])
+    return result_array(out)
 
 
 def rg_batch(ctx: Context, z1, z2, n1, n2, ref_l2, w_l2, m_snps: float,
@@ -490,9 +494,7 @@ def rg_batch(ctx: Context, z1, z2, n1, n2, ref_l2, w_l2, m_snps: float,
                     w_l2=w_l2.ctypes.data, m_snps=float(m_snps), device_pointers=0)
     out = (L.RgResult * P)()
     ctx.check(ctx.lib.ldsc_rg_batch(ctx.h, C.byref(args), C.cast(out, C.c_void_p)))
-    names = [f for f, _ in L.RgResult._fields_]
-    return np.array([tuple(getattr(r, f) for f in names) for r in out],
-                    dtype=[(f, np.float64) for f in names])
+    return result_array(out)
 
 
 def snp_stats(ctx: Context, snps: BimTable, panel: Panel, iid_indices=None):

@@ -17,6 +17,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <algorithm>
 #include <atomic>
@@ -66,6 +67,36 @@ struct DevBuf {
     template <typename T>
     T* as() const {
         return reinterpret_cast<T*>(p);
+    }
+};
+
+// Host end of a call's copies, kept by the context (grow-only, given back by a
+// trim): page-locked up to PINNED_MAX, so a copy neither blocks the host nor goes
+// through the driver's staging buffer; larger, or where none can be locked,
+// ordinary memory.  One pageable copy of each result left the device idle
+// for 25 to 50 us before the next could start.
+struct HostBuf {
+    static constexpr size_t PINNED_MAX = 64ull << 20;
+    uint8_t* p = nullptr;
+    size_t cap = 0;
+    bool pinned = false;
+    uint8_t* ensure(size_t bytes) {   // null: out of memory
+        if (bytes <= cap && p) return p;
+        release();
+        bytes += bytes / 8 + 4096;
+        pinned = bytes <= PINNED_MAX && cudaHostAlloc(reinterpret_cast<void**>(&p), bytes, cudaHostAllocDefault) == cudaSuccess;
+        if (!pinned) {
+            cudaGetLastError();
+            p = static_cast<uint8_t*>(std::malloc(bytes));
+        }
+        cap = p ? bytes : 0;
+        return p;
+    }
+    void release() {
+        if (p && pinned) cudaFreeHost(p);
+        if (p && !pinned) std::free(p);
+        p = nullptr;
+        cap = 0;
     }
 };
 
@@ -121,8 +152,11 @@ struct ldsc_ctx {
     std::mutex mu;
     std::string last_error;
     uint64_t kernels = 0;
+    HostBuf host_up, host_out;    // the plan's upload and the results
+    bool up_pending = false;      // host_up may still be read by a copy
+    cudaEvent_t run_ev[8] = {};   // timing marks of an l2 run
     // workspace (grow-only)
-    DevBuf ops, blocks, xsk, recrows, keep, left, tiles, annot, aeff, l2, maf, pq, err;
+    DevBuf ops, plan_dev, xsk, recrows, keep, left, tiles, annot, aeff, l2, maf, pq, err;
     DevBuf st_n, st_s, st_q, st_q3, st_q4, st_mean, st_inv, st_qinv, st_kappa, packed, tsum, dbg;
     // private CountSketch layout (explicit bucket/sign arrays, or a panel
     // whose shared layout is in use under another key)
@@ -130,7 +164,7 @@ struct ldsc_ctx {
     uint64_t sk_panel = 0;
     GraphCache graphs;            // regression pipelines
     uint64_t graph_launches = 0;  // replays of cached graphs
-    DevBuf rtiles, roff, cptr_r, cidx_r, cptr_l, cidx_l;  // K > 1 contraction: r2u tiles and CSR tile lists
+    DevBuf rtiles;                                  // K > 1 contraction: r2u tiles
     DevBuf prow, pcol;                              // K = 1: per-tile row / column sums
     DevBuf rg_jobs, rg_states, rg_outs, rg_part, rg_tdel, rg_y, rg_y2, rg_n, rg_ld, rg_wld, rg_sel, rg_pairs, rg_res;
     DevBuf ts_seps, ts_n1, ts_cnt, ts_dv, ts_outs;  // --two-step
@@ -149,12 +183,12 @@ struct ldsc_ctx {
     cudaEvent_t feed_t0 = nullptr, feed_t1 = nullptr, feed_go = nullptr, up_ev = nullptr;
 
     std::vector<DevBuf*> workspace() {
-        return {&ops, &blocks, &xsk, &recrows, &keep, &left,
+        return {&ops, &plan_dev, &xsk, &recrows, &keep, &left,
                       &tiles, &annot, &aeff, &l2, &maf,
                       &pq, &err, &st_n, &st_s, &st_q, &st_q3,
                       &st_q4, &st_mean, &st_inv, &st_qinv, &st_kappa,
                       &packed, &tsum, &dbg,
-                      &rtiles, &roff, &cptr_r, &cidx_r, &cptr_l, &cidx_l, &prow, &pcol,
+                      &rtiles, &prow, &pcol,
                       &rg_jobs, &rg_states, &rg_outs, &rg_part, &rg_tdel,
                       &rg_y, &rg_y2, &rg_n, &rg_ld, &rg_wld, &rg_sel,
                       &rg_pairs, &rg_res, &bed_stage, &bed_rows, &ts_seps, &ts_n1, &ts_cnt, &ts_dv, &ts_outs,
@@ -266,6 +300,10 @@ int ldsc_ctx_destroy(ldsc_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     for (cudaEvent_t e : ctx->feed_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->ovl_ev) cudaEventDestroy(e);
+    for (cudaEvent_t e : ctx->run_ev)
+        if (e) cudaEventDestroy(e);
+    ctx->host_up.release();
+    ctx->host_out.release();
     for (cudaEvent_t e : {ctx->feed_t0, ctx->feed_t1, ctx->feed_go, ctx->up_ev, ctx->ovl_go, ctx->ovl_plan, ctx->ovl_done})
         if (e) cudaEventDestroy(e);
     if (ctx->side) cudaStreamDestroy(ctx->side);
@@ -304,6 +342,9 @@ int ldsc_ctx_trim(ldsc_ctx* ctx) {
         if (x) cudaStreamSynchronize(x);
     ctx->graphs.clear();  // their kernels hold the buffers' addresses
     for (DevBuf* b : ctx->workspace()) b->release();
+    ctx->host_up.release();
+    ctx->host_out.release();
+    ctx->up_pending = false;
     ctx->sk.release();
     ctx->sk_panel = 0;
     return LDSC_OK;
@@ -513,16 +554,13 @@ int ldsc_l2_pair_count(const ldsc_l2_args* a, uint64_t* n_pairs) {
 namespace {
 
 struct Events {
-    cudaEvent_t ev[8] = {};
+    cudaEvent_t* ev;   // the context's, made at their first use
     int n = 0;
     cudaStream_t s;
-    explicit Events(cudaStream_t st) : s(st) {}
-    ~Events() {
-        for (int i = 0; i < n; i++) cudaEventDestroy(ev[i]);
-    }
+    Events(cudaEvent_t* e, cudaStream_t st) : ev(e), s(st) {}
     int mark() { return mark_on(s); }
     int mark_on(cudaStream_t on) {
-        cudaEventCreate(&ev[n]);
+        if (!ev[n]) cudaEventCreate(&ev[n]);
         cudaEventRecord(ev[n], on);
         return n++;
     }
@@ -681,6 +719,9 @@ int ensure_overlap(ldsc_ctx* ctx, int n) {
 constexpr int64_t OVERLAP_CHUNKS = 4;
 constexpr int64_t OVERLAP_FIRST_DIV = 8;
 constexpr int64_t OVERLAP_MIN_RECORDS = 16384;
+// Results up to this size leave through the context's pinned memory; a second
+// host copy of larger ones costs more than the two waits it saves.
+constexpr size_t HOST_OUT_MAX = 8ull << 20;
 
 int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double* l2_out, double* maf_out,
            ldsc_perf* perf, double upload_secs, RowFeed* feed = nullptr) {
@@ -920,6 +961,14 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     LeftLimits& L = ctx->plan_left;
     std::vector<Tile>& tiles = ctx->plan_tiles;
     const int32_t n_right = (int32_t)((m + tb - 1) / tb), n_left = (int32_t)((m + ta - 1) / ta);
+    // device ends of the plan (one buffer, filled by one copy)
+    struct {
+        const int64_t* left;
+        const Tile* tiles;
+        const uint32_t* roff;
+        const GramBlock* blocks;
+        const int32_t *ptr_r, *idx_r, *ptr_l, *idx_l;
+    } dp{};
     auto plan = [&]() -> int {
         std::string perr;
         if (!left_limits(m, a->chr, a->cm, a->bp, a->window_mode, a->window_size, a->window_snps, a->chunk_size,
@@ -936,19 +985,14 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         else
             gram_tiles(L.left, trim, 4, &tiles);
         pf.n_tiles = tiles.size();
-        CK(ctx->left.ensure(sizeof(int64_t) * nmom));
         // buffers sized by the tile count get an eighth more when they grow: a
         // later call over a few more tiles then reuses them instead of
         // allocating (a pool growth while other work runs stalls it)
         const size_t nt_room = tiles.size() + tiles.size() / 8;
-        CK(ctx->tiles.ensure(sizeof(Tile) * (nt_room + 1)));
-        CK(cudaMemcpyAsync(ctx->left.p, L.left.data(), 8 * nmom, cudaMemcpyHostToDevice, up));
-        if (!tiles.empty())
-            CK(cudaMemcpyAsync(ctx->tiles.p, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice, up));
         // CSR lists of tiles per right block and per left block: the K > 1
         // contraction passes and the K = 1 reduction of per-tile sums.  The
-        // host lists live in the context until the next call (the copies
-        // read them asynchronously).
+        // host lists live in the context until the next call, which reuses
+        // their pages.
         if (!tiles.empty()) {
             std::vector<int32_t>&ptr_r = ctx->plan_ptr_r, &ptr_l = ctx->plan_ptr_l, &idx_r = ctx->plan_idx_r,
                                   &idx_l = ctx->plan_idx_l;
@@ -976,28 +1020,54 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                     q += tiles[t].nq1 + 1u;
                 }
                 CK(ctx->rtiles.ensure(sizeof(double) * (size_t)ta * TILE_QUARTER * (q + q / 8)));
-                CK(ctx->roff.ensure(4 * nt_room));
-                CK(cudaMemcpyAsync(ctx->roff.p, roff.data(), 4 * roff.size(), cudaMemcpyHostToDevice, up));
             } else {
                 CK(ctx->prow.ensure(sizeof(double) * (size_t)ta * nt_room));
                 CK(ctx->pcol.ensure(sizeof(double) * (size_t)tb * nt_room));
             }
-            if (f64) {
-                if (K > 1) gram_blocks_of(tiles, ctx->plan_roff, &ctx->plan_blocks);
-                const size_t nb = ctx->plan_blocks.size();
-                CK(ctx->blocks.ensure(sizeof(GramBlock) * (nb + nb / 8)));
-                CK(cudaMemcpyAsync(ctx->blocks.p, ctx->plan_blocks.data(), sizeof(GramBlock) * nb, cudaMemcpyHostToDevice,
-                                   up));
-            }
-            CK(ctx->cptr_r.ensure(4 * ptr_r.size()));
-            CK(ctx->cidx_r.ensure(4 * nt_room));
-            CK(ctx->cptr_l.ensure(4 * ptr_l.size()));
-            CK(ctx->cidx_l.ensure(4 * nt_room));
-            CK(cudaMemcpyAsync(ctx->cptr_r.p, ptr_r.data(), 4 * ptr_r.size(), cudaMemcpyHostToDevice, up));
-            CK(cudaMemcpyAsync(ctx->cidx_r.p, idx_r.data(), 4 * idx_r.size(), cudaMemcpyHostToDevice, up));
-            CK(cudaMemcpyAsync(ctx->cptr_l.p, ptr_l.data(), 4 * ptr_l.size(), cudaMemcpyHostToDevice, up));
-            CK(cudaMemcpyAsync(ctx->cidx_l.p, idx_l.data(), 4 * idx_l.size(), cudaMemcpyHostToDevice, up));
+            if (f64 && K > 1) gram_blocks_of(tiles, ctx->plan_roff, &ctx->plan_blocks);
         }
+        // everything the kernels read of the plan, in one buffer and one copy
+        size_t total = 0;
+        auto place = [&](size_t bytes) {
+            const size_t at = total;
+            total += round_up(bytes, 16);
+            return at;
+        };
+        const bool any = !tiles.empty();
+        const size_t nt = tiles.size(), nb = any && f64 ? ctx->plan_blocks.size() : 0;
+        const size_t o_left = place(8 * nmom), o_tiles = place(sizeof(Tile) * nt),
+                     o_roff = place(any && K > 1 ? 4 * nt : 0), o_blocks = place(sizeof(GramBlock) * nb),
+                     o_pr = place(any ? 4 * ctx->plan_ptr_r.size() : 0), o_ir = place(4 * nt),
+                     o_pl = place(any ? 4 * ctx->plan_ptr_l.size() : 0), o_il = place(4 * nt);
+        if (ctx->up_pending) {   // an earlier call failed between its copy and its end
+            CK(cudaStreamSynchronize(s));
+            CK(cudaStreamSynchronize(ctx->copy));
+            ctx->up_pending = false;
+        }
+        uint8_t* h = ctx->host_up.ensure(total);
+        if (!h) return fail(ctx, LDSC_E_NOMEM, "out of host memory for the plan");
+        if (total > ctx->plan_dev.cap) CK(ctx->plan_dev.ensure(total + (total - o_tiles) / 8));
+        std::memcpy(h + o_left, L.left.data(), 8 * nmom);
+        if (any) {
+            std::memcpy(h + o_tiles, tiles.data(), sizeof(Tile) * nt);
+            if (K > 1) std::memcpy(h + o_roff, ctx->plan_roff.data(), 4 * nt);
+            if (nb) std::memcpy(h + o_blocks, ctx->plan_blocks.data(), sizeof(GramBlock) * nb);
+            std::memcpy(h + o_pr, ctx->plan_ptr_r.data(), 4 * ctx->plan_ptr_r.size());
+            std::memcpy(h + o_ir, ctx->plan_idx_r.data(), 4 * nt);
+            std::memcpy(h + o_pl, ctx->plan_ptr_l.data(), 4 * ctx->plan_ptr_l.size());
+            std::memcpy(h + o_il, ctx->plan_idx_l.data(), 4 * nt);
+        }
+        ctx->up_pending = true;
+        CK(cudaMemcpyAsync(ctx->plan_dev.p, h, total, cudaMemcpyHostToDevice, up));
+        const uint8_t* dv = ctx->plan_dev.as<uint8_t>();
+        dp.left = reinterpret_cast<const int64_t*>(dv + o_left);
+        dp.tiles = reinterpret_cast<const Tile*>(dv + o_tiles);
+        dp.roff = reinterpret_cast<const uint32_t*>(dv + o_roff);
+        dp.blocks = reinterpret_cast<const GramBlock*>(dv + o_blocks);
+        dp.ptr_r = reinterpret_cast<const int32_t*>(dv + o_pr);
+        dp.idx_r = reinterpret_cast<const int32_t*>(dv + o_ir);
+        dp.ptr_l = reinterpret_cast<const int32_t*>(dv + o_pl);
+        dp.idx_l = reinterpret_cast<const int32_t*>(dv + o_il);
         return join_up();
     };
 
@@ -1055,7 +1125,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         if (rc != LDSC_OK) return rc;
         rc = plan();
         if (rc != LDSC_OK) return rc;
-        ep.left = ctx->left.as<int64_t>();
+        ep.left = dp.left;
         ep.rtiles = nullptr;
         ep.prow = tiles.empty() ? nullptr : ctx->prow.as<double>();
         ep.pcol = tiles.empty() ? nullptr : ctx->pcol.as<double>();
@@ -1065,7 +1135,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         if (rc != LDSC_OK) return rc;
     }
 
-    Events ev(s);
+    Events ev(ctx->run_ev, s);
     const int e0 = ev.mark();
 
     // ---- decode ----
@@ -1116,10 +1186,10 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                         ec.prow += t0 * ta;
                         ec.pcol += t0 * tb;
                         if (fused_i8)
-                            CK(launch_gram_i8_packed(pv.rows, pv.pitch, n_used, m, ctx->tiles.as<Tile>() + t0,
+                            CK(launch_gram_i8_packed(pv.rows, pv.pitch, n_used, m, dp.tiles + t0,
                                                      (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, s));
                         else
-                            CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>() + t0,
+                            CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, dp.tiles + t0,
                                               (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, s));
                         ctx->kernels++;
                     }
@@ -1183,9 +1253,9 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         // ---- host plan (runs while the decode kernels execute) ----
         int rc = plan();
         if (rc != LDSC_OK) return rc;
-        ep.left = ctx->left.as<int64_t>();
+        ep.left = dp.left;
         ep.rtiles = (K > 1 && !tiles.empty()) ? ctx->rtiles.as<double>() : nullptr;
-        ep.roff = ctx->roff.as<uint32_t>();
+        ep.roff = dp.roff;
         ep.prow = (K == 1 && !tiles.empty()) ? ctx->prow.as<double>() : nullptr;
         ep.pcol = (K == 1 && !tiles.empty()) ? ctx->pcol.as<double>() : nullptr;
     }
@@ -1212,7 +1282,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             EpilogueArgs ec = ep;  // this launch's tiles write their sums at their own tile indices
             ec.prow += t0 * ta;
             ec.pcol += t0 * tb;
-            CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>() + t0, (int64_t)(t1 - t0), ec,
+            CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, dp.tiles + t0, (int64_t)(t1 - t0), ec,
                               nullptr, 0, ctx->sms, gs));
             ctx->kernels++;
             t0 = t1;
@@ -1224,44 +1294,55 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     if (overlap) CK(cudaStreamWaitEvent(s, ctx->ovl_ev[ov_n - 1], 0));
     if (!tiles.empty() && !stream_gram && !overlap) {
         if (d) {
-            CK(launch_gram_tf32(ctx->xsk.as<float>(), ld_sk, m, ctx->tiles.as<Tile>(), (int64_t)tiles.size(), ep,
+            CK(launch_gram_tf32(ctx->xsk.as<float>(), ld_sk, m, dp.tiles, (int64_t)tiles.size(), ep,
                                 maf_aware ? 1 : 0, ctx->sms, s));
         } else if (fused_i8) {
-            CK(launch_gram_i8_packed(pv.rows, pv.pitch, n_used, m, ctx->tiles.as<Tile>(), (int64_t)tiles.size(), ep,
+            CK(launch_gram_i8_packed(pv.rows, pv.pitch, n_used, m, dp.tiles, (int64_t)tiles.size(), ep,
                                      nullptr, 0, ctx->sms, s));
         } else if (exact_i8) {
-            CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, ctx->tiles.as<Tile>(), (int64_t)tiles.size(), ep,
+            CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, dp.tiles, (int64_t)tiles.size(), ep,
                               nullptr, 0, ctx->sms, s));
         } else {
             const PanelView pk{ctx->packed.as<uint8_t>(), nmom, n_used, (n_used + 3) / 4, kp};
-            CK(launch_gram_f64(compact ? pk : pv, compact ? nullptr : rr, st, ctx->blocks.as<GramBlock>(),
+            CK(launch_gram_f64(compact ? pk : pv, compact ? nullptr : rr, st, dp.blocks,
                                (uint32_t)ctx->plan_blocks.size(), ctx->err.as<unsigned int>() + 1, ep, ctx->sms, s));
         }
         ctx->kernels++;
         e_c = ev.mark();
         if (K > 1) {
-            CK(launch_contract(ctx->tiles.as<Tile>(), ctx->cptr_r.as<int32_t>(), ctx->cidx_r.as<int32_t>(), n_right, true,
+            CK(launch_contract(dp.tiles, dp.ptr_r, dp.idx_r, n_right, true,
                                ep, ctx->sms, s));
-            CK(launch_contract(ctx->tiles.as<Tile>(), ctx->cptr_l.as<int32_t>(), ctx->cidx_l.as<int32_t>(), n_left, false,
+            CK(launch_contract(dp.tiles, dp.ptr_l, dp.idx_l, n_left, false,
                                ep, ctx->sms, s));
             ctx->kernels += 2;
         }
     }
     if (K == 1 && !tiles.empty()) {
         // the per-tile sums into l2, in a fixed order
-        CK(launch_l2_reduce(m, ta, tb, ctx->cptr_r.as<int32_t>(), ctx->cidx_r.as<int32_t>(), ctx->cptr_l.as<int32_t>(),
-                            ctx->cidx_l.as<int32_t>(), ctx->prow.as<double>(), ctx->pcol.as<double>(),
+        CK(launch_l2_reduce(m, ta, tb, dp.ptr_r, dp.idx_r, dp.ptr_l,
+                            dp.idx_l, ctx->prow.as<double>(), ctx->pcol.as<double>(),
                             ctx->l2.as<double>(), s));
         ctx->kernels++;
     }
     const int e3 = ev.mark();
+    // results: to the caller's device buffers, or through the context's pinned
+    // memory to the caller's host arrays (those too large for it directly)
+    const size_t l2_bytes = 8 * nmom * K, maf_bytes = maf_out ? 8 * nmom : 0;
+    const bool staged = !a->out_on_device && l2_bytes + maf_bytes <= HOST_OUT_MAX;
+    uint8_t* h = ctx->host_out.ensure(16 + (staged ? l2_bytes + maf_bytes : 0));
+    if (!h) return fail(ctx, LDSC_E_NOMEM, "out of host memory for the results");
     const cudaMemcpyKind okind = a->out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    CK(cudaMemcpyAsync(l2_out, ctx->l2.p, 8 * nmom * K, okind, s));
-    if (maf_out) CK(cudaMemcpyAsync(maf_out, ctx->maf.p, 8 * nmom, okind, s));
-    unsigned int herr[4] = {0, 0, 0, 0};
-    CK(cudaMemcpyAsync(herr, ctx->err.p, 16, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(staged ? h + 16 : (void*)l2_out, ctx->l2.p, l2_bytes, okind, s));
+    if (maf_out) CK(cudaMemcpyAsync(staged ? h + 16 + l2_bytes : (void*)maf_out, ctx->maf.p, maf_bytes, okind, s));
+    CK(cudaMemcpyAsync(h, ctx->err.p, 16, cudaMemcpyDeviceToHost, s));
     const int e4 = ev.mark();
     CK(cudaStreamSynchronize(s));
+    ctx->up_pending = false;
+    const unsigned int* herr = reinterpret_cast<const unsigned int*>(h);
+    if (staged) {
+        std::memcpy(l2_out, h + 16, l2_bytes);
+        if (maf_out) std::memcpy(maf_out, h + 16 + l2_bytes, maf_bytes);
+    }
     if (herr[0] != 0)
         return fail(ctx, LDSC_E_TIMEOUT, "a device wait in the Gram kernel exceeded its bound (error word " +
                                              std::to_string(herr[0]) + ")");
@@ -1729,12 +1810,15 @@ extern "C" int ldsc_h2_batch(ldsc_ctx* ctx, const ldsc_h2_args* a, ldsc_h2_resul
                                  ctx->rg_sel.as<double>() + T, ctx->rg_sel.as<double>(), T, gs);
     }));
     ctx->kernels += (two ? 19 : 8) + (a->want_lambda_gc ? 1 : 0);
-    std::vector<RegOut> outs(T);
-    std::vector<double> sel(2 * T, NAN);
-    std::vector<int32_t> n1(two ? T : 0);
-    CK(cudaMemcpyAsync(outs.data(), ctx->rg_outs.p, sizeof(RegOut) * T, cudaMemcpyDeviceToHost, s));
-    if (a->want_lambda_gc) CK(cudaMemcpyAsync(sel.data(), ctx->rg_sel.p, 8 * 2 * (size_t)T, cudaMemcpyDeviceToHost, s));
-    if (two) CK(cudaMemcpyAsync(n1.data(), ctx->ts_n1.p, 4 * (size_t)T, cudaMemcpyDeviceToHost, s));
+    const size_t o_sel = round_up(sizeof(RegOut) * T, 16), o_n1 = o_sel + 8 * 2 * (size_t)T;
+    uint8_t* h = ctx->host_out.ensure(o_n1 + 4 * (size_t)T);
+    if (!h) return fail(ctx, LDSC_E_NOMEM, "out of host memory for the results");
+    const RegOut* outs = reinterpret_cast<const RegOut*>(h);
+    const double* sel = reinterpret_cast<const double*>(h + o_sel);
+    const int32_t* n1 = reinterpret_cast<const int32_t*>(h + o_n1);
+    CK(cudaMemcpyAsync(h, ctx->rg_outs.p, sizeof(RegOut) * T, cudaMemcpyDeviceToHost, s));
+    if (a->want_lambda_gc) CK(cudaMemcpyAsync(h + o_sel, ctx->rg_sel.p, 8 * 2 * (size_t)T, cudaMemcpyDeviceToHost, s));
+    if (two) CK(cudaMemcpyAsync(h + o_n1, ctx->ts_n1.p, 4 * (size_t)T, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     for (int t = 0; t < (two ? T : 0); t++)  // jackknife_fast on the step-1 SNPs (src/h2.rs:121-123)
         if (n1[t] < nb) return fail(ctx, LDSC_E_INVALID, "More blocks than data points.");
@@ -1894,7 +1978,8 @@ extern "C" int ldsc_h2_partitioned(ldsc_ctx* ctx, const ldsc_h2p_args* a, ldsc_h
     CK(ctx->p_sol.ensure(8 * max_gj * (size_t)(nb + 1) * P));
     CK(ctx->p_res.ensure(8 * res_len));
     CK(cudaMemcpyAsync(ctx->p_jobs.p, pj.data(), sizeof(PartJob) * T, cudaMemcpyHostToDevice, s));
-    std::vector<double> hres(res_len);
+    double* hres = reinterpret_cast<double*>(ctx->host_out.ensure(8 * res_len));
+    if (!hres) return fail(ctx, LDSC_E_NOMEM, "out of host memory for the results");
     size_t ro = 0;
     bool first = true;
     for (size_t gi = 0; gi < groups.size(); gi++) {
@@ -1911,13 +1996,13 @@ extern "C" int ldsc_h2_partitioned(ldsc_ctx* ctx, const ldsc_h2p_args* a, ldsc_h
             ro += (size_t)nj * part_result_len(gb, K, P);
         }
     }
-    CK(cudaMemcpyAsync(hres.data(), ctx->p_res.p, 8 * res_len, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(hres, ctx->p_res.p, 8 * res_len, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     ro = 0;
     for (size_t gi = 0; gi < groups.size(); gi++) {
         const int gb = gnb[gi];
         for (int t : groups[gi]) {
-            const double* R = hres.data() + ro;
+            const double* R = hres + ro;
             ro += part_result_len(gb, K, P);
             const double* est = R;
             const double* cov = est + P;
@@ -2040,8 +2125,9 @@ extern "C" int ldsc_rg_batch(ldsc_ctx* ctx, const ldsc_rg_args* a, ldsc_rg_resul
         return launch_rg_finish(ctx->rg_pairs.as<RgPairIdx>(), dout, dtd, nb, ctx->rg_res.as<RgOut>(), P, gs);
     }));
     ctx->kernels += 17;
-    std::vector<RgOut> outs(P);
-    CK(cudaMemcpyAsync(outs.data(), ctx->rg_res.p, sizeof(RgOut) * P, cudaMemcpyDeviceToHost, s));
+    const RgOut* outs = reinterpret_cast<const RgOut*>(ctx->host_out.ensure(sizeof(RgOut) * P));
+    if (!outs) return fail(ctx, LDSC_E_NOMEM, "out of host memory for the results");
+    CK(cudaMemcpyAsync(ctx->host_out.p, ctx->rg_res.p, sizeof(RgOut) * P, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     for (int p = 0; p < P; p++) {
         const RgOut& o = outs[p];

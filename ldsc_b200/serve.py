@@ -16,7 +16,7 @@ from typing import Optional
 import numpy as np
 
 from . import _lib as L
-from .api import LdscError, Panel, WindowMode, _ArgPack, _f64, _perf
+from .api import LdscError, Panel, WindowMode, _ArgPack, _f64, _perf, result_array
 from .plink import BimTable
 
 
@@ -196,11 +196,7 @@ class Server:
                                            intercept_se=r.intercept_se, mean_chi2=r.mean_chi2,
                                            n_obs=int(r.n_obs), n_blocks=nb))
             return fits, timing
-        struct = L.H2Result if kind == "h2" else L.RgResult
-        names = [f for f, _ in struct._fields_]
-        out = np.array([tuple(getattr(r, f) for f in names) for r in keep["out"]],
-                       dtype=[(f, np.float64) for f in names])
-        return out, timing
+        return result_array(keep["out"]), timing
 
     def stats(self) -> dict:
         st = L.ServerStats()

@@ -612,18 +612,25 @@ int sketch_prepare(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t n_used, uint
 struct RowFeed {
     ldsc_ctx* ctx = nullptr;
     const uint8_t* host = nullptr;  // file body (after the 3 magic bytes)
-    uint64_t bpr = 0, pitch = 0, rows = 0, per = 0;
+    uint64_t bpr = 0, pitch = 0, rows = 0, per = 0, head = 0;   // head: rows before the last chunk
     int nchunks = 0, issued = 0, queued = 0;
     uint8_t* dst = nullptr;
 
     bool started = false;
 
-    uint64_t row_end(int c) const { return std::min<uint64_t>(rows, (uint64_t)(c + 1) * per); }
+    uint64_t row_end(int c) const { return c == nchunks - 1 ? rows : std::min<uint64_t>(head, (uint64_t)(c + 1) * per); }
+    uint64_t row_begin(int c) const { return c ? row_end(c - 1) : 0; }
     // buffers and events; the panel's rows pointer is valid after this
     int prepare() {
         ldsc_ctx* c = ctx;
-        per = std::max<uint64_t>(1, (64ull << 20) / bpr);
-        nchunks = (int)((rows + per - 1) / per);
+        // 24 MB per chunk and half of that in the last: what follows the last copy
+        // (pitch, decode, Gram) has no copy to run beside.  A 250 MB file of 50,000
+        // individuals, whose copies take 4,590 us: 5,130 us per call; 32 and 16 MB
+        // 5,190, 64 and 16 MB 5,350, 64 MB throughout 5,570 (with the Gram between
+        // the chunks' decodes on one stream).
+        per = std::max<uint64_t>(1, (24ull << 20) / bpr);
+        head = rows > per ? rows - (per + 1) / 2 : 0;
+        nchunks = (int)((head + per - 1) / per) + 1;
         while ((int)c->feed_ev.size() < nchunks) {
             cudaEvent_t e;
             CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -652,7 +659,7 @@ struct RowFeed {
         }
         for (; queued < std::min(k_end, nchunks); queued++) {
             const int k = queued;
-            const uint64_t r0 = (uint64_t)k * per, r1 = row_end(k);
+            const uint64_t r0 = row_begin(k), r1 = row_end(k);
             CK(cudaMemcpyAsync(c->bed_stage.as<uint8_t>() + r0 * bpr, host + r0 * bpr, (r1 - r0) * bpr,
                                cudaMemcpyHostToDevice, c->copy));
             CK(cudaEventRecord(c->feed_ev[k], c->copy));
@@ -669,7 +676,7 @@ struct RowFeed {
         }
         for (; issued < std::min(k_end, nchunks); issued++) {
             CK(cudaStreamWaitEvent(s, c->feed_ev[issued], 0));
-            CK(launch_repitch(c->bed_stage.as<uint8_t>(), bpr, dst, pitch, (uint64_t)issued * per, row_end(issued),
+            CK(launch_repitch(c->bed_stage.as<uint8_t>(), bpr, dst, pitch, row_begin(issued), row_end(issued),
                               s));
             c->kernels++;
         }
@@ -1145,6 +1152,20 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     const bool staged_i8 = exact_i8 && !fused_i8;
     if (staged_i8) CK(ctx->ops.ensure((size_t)2 * nmom * ld_i8));
     if (chunked) {
+        // With a streamed Gram the chunks are pitched and decoded on the side
+        // stream, and the Gram launches alternate between two others: neither
+        // the next chunk's decode nor its Gram waits for a launch's last,
+        // partly filled wave.
+        cudaStream_t ds = s;
+        if (stream_gram) {
+            int rc = ensure_overlap(ctx, feed->nchunks);
+            if (rc != LDSC_OK) return rc;
+            ds = ctx->side;
+            CK(cudaEventRecord(ctx->ovl_go, s));
+            CK(cudaStreamWaitEvent(ds, ctx->ovl_go, 0));
+            CK(cudaStreamWaitEvent(ctx->gram2, ctx->ovl_go, 0));
+        }
+        int launched = 0;
         // records [r0, r1) whose rows arrived with chunks [0, k]
         int64_t r0 = 0;
         size_t t0 = 0;
@@ -1155,18 +1176,18 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                 r1 = std::lower_bound(a->bed_idx + r0, a->bed_idx + m, rend) - a->bed_idx;
             else
                 r1 = std::max<int64_t>(r0, std::min<int64_t>(m, (int64_t)rend - (int64_t)a->row_begin));
-            int rc = feed->issue_until(k + 1, s);
+            int rc = feed->issue_until(k + 1, ds);
             if (rc != LDSC_OK) return rc;
             if (r1 > r0) {
                 PanelView pc;
                 const uint64_t* list;
-                CK(rows_of(r0, r1, s, &pc, &list));
+                CK(rows_of(r0, r1, ds, &pc, &list));
                 RecStats sc = st;
                 sc.n += r0;
                 sc.s += r0;
                 sc.q += r0;
                 uint8_t* oc = staged_i8 ? ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8 : nullptr;
-                CK(launch_decode_i8(pc, list, r1 - r0, oc, staged_i8 ? ld_i8 : 0, sc, 0, s));
+                CK(launch_decode_i8(pc, list, r1 - r0, oc, staged_i8 ? ld_i8 : 0, sc, 0, ds));
                 ctx->kernels++;
                 if (stream_gram) {
                     sc.maf += r0;
@@ -1175,28 +1196,37 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                     sc.qinv += r0;
                     CK(launch_finalize_stats(r1 - r0, n_used, sc, annot_dev ? annot_dev + r0 : nullptr, 1,
                                              a->has_pq_exp, a->pq_exp, ctx->aeff.as<double>() + r0,
-                                             ctx->l2.as<double>() + r0, s, annot_ld_dev));
+                                             ctx->l2.as<double>() + r0, ds, annot_ld_dev));
                     ctx->kernels++;
                     // tiles are ordered by right block; take those whose right block is complete
                     size_t t1 = t0;
                     while (t1 < tiles.size() && (r1 == m || (int64_t)(tiles[t1].b_blk + 1) * tb <= r1)) t1++;
                     if (t1 > t0) {
                         // this launch's tiles write their sums at their own tile indices
+                        cudaStream_t gs = launched++ & 1 ? ctx->gram2 : s;
+                        CK(cudaEventRecord(ctx->ovl_ev[k], ds));
+                        CK(cudaStreamWaitEvent(gs, ctx->ovl_ev[k], 0));
                         EpilogueArgs ec = ep;
                         ec.prow += t0 * ta;
                         ec.pcol += t0 * tb;
                         if (fused_i8)
                             CK(launch_gram_i8_packed(pv.rows, pv.pitch, n_used, m, dp.tiles + t0,
-                                                     (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, s));
+                                                     (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, gs));
                         else
                             CK(launch_gram_i8(ctx->ops.as<uint8_t>(), ld_i8, m, dp.tiles + t0,
-                                              (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, s));
+                                              (int64_t)(t1 - t0), ec, nullptr, 0, ctx->sms, gs));
                         ctx->kernels++;
                     }
                     t0 = t1;
                 }
             }
             r0 = r1;
+        }
+        if (stream_gram) {   // every tile's sums and every record's statistics, before what follows
+            for (cudaStream_t x : {ds, ctx->gram2}) {
+                CK(cudaEventRecord(ctx->ovl_done, x));
+                CK(cudaStreamWaitEvent(s, ctx->ovl_done, 0));
+            }
         }
         ctx->kernels--;  // counted once below
     } else if (overlap) {

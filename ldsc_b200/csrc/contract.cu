@@ -13,6 +13,8 @@
 // carries f64 rounding only, binary and continuous columns alike.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "engine.h"
 #include "sm100.cuh"
 
@@ -25,35 +27,38 @@ constexpr int NT = 256;  // threads of k_l2_reduce
 // The contraction on the FP64 tensor path (mma.sync m8n8k4 .f64):
 //   BY_RIGHT: out rows j of the right block, out[j][c] += sum_k R[j][k] A[k][c]
 //   BY_LEFT:  out rows k of the left block,  out[k][c] += sum_j R[j][k] A[j][c]
-// One CTA owns one output block of 128 rows and up to MK = 128 annotation
+// One CTA owns 64 output rows, half a block, and up to MK = 128 annotation
 // columns (K > 128 runs column chunks).  The summed records of every tile of
-// the block go by in steps of JS = 32 (a quarter of the right block for
-// BY_LEFT, so quarters a tile leaves out cost nothing); a step's r2u values and
-// the annotation values of its 32 records are staged by cp.async into one of
-// two buffers while the MMAs run on the other.  Each of the 8 warps owns 16
-// output rows and all the chunk's columns: 2 x NF fragments of 8 x 8 f64
-// accumulators, eight k-steps of four records per staged step, so the 2 + NF
-// fragment loads of a k-step feed 2 NF MMAs and only about ceil(K / 8) fragments
-// are multiplied (a warp on 32 rows x 32 columns padded 97 columns to 128).  In a
-// BY_RIGHT step a warp whose rows the tile leaves out skips the MMAs.
-// The FP64 pipe bounds it (64 FMA per clock and SM):
-// 100,000 records x 97 columns, 2,892 tiles: 553 + 535 us against 574 + 567 us
-// with 32 x 32 warp tiles on the same tile list.
+// the block go by in steps of JS = 16; quarters that a tile leaves out, and for
+// BY_RIGHT tiles without a quarter in this half, cost nothing.  A step's r2u
+// values and the annotation values of its records are staged by cp.async into
+// one of two buffers while
+// the MMAs run on the other; the tile list is read an entry ahead.  Each of the
+// 4 warps owns 16 output rows and all the chunk's columns: 2 x NF fragments of
+// 8 x 8 f64 accumulators, four k-steps of four records per staged step, so the
+// 2 + NF fragment loads of a k-step feed 2 NF MMAs and only about ceil(K / 8)
+// fragments are multiplied.  Three CTAs share an SM: one multiplies while
+// another waits for its stage, and half blocks leave less of a last wave idle.
+// The FP64 pipe bounds it (64 FMA per clock and SM): 100,000 records x 97
+// columns, 2,892 tiles: 379 + 350 us, 70% of the pipe (steps of 32 and two CTAs:
+// 462 + 431; one CTA of 128 rows per SM and the list read in each step: 553 +
+// 535).
 // Fragment layouts of m8n8k4 (row.col): A element (lane / 4, lane % 4), B
 // element (lane % 4, lane / 4), D elements (lane / 4, 2 (lane % 4) + {0, 1}).
 // Shared rows are padded to a stride of 4 mod 16 doubles, so each half-warp's
 // 16 8-byte fragment loads hit 16 distinct bank pairs.
 constexpr int MK = 128;        // annotation columns per chunk
-constexpr int JS = 32;         // summed records per staged step
+constexpr int JS = 16;         // summed records per staged step
 constexpr int OB = TILE_RECORDS;
-constexpr int CTH = 256;       // threads
+constexpr int HB = OB / 2;     // output rows of a CTA
+constexpr int CTH = 128;       // threads
 constexpr int SLD = JS + 4;    // staged annotation stride (annotations are [column][record])
-constexpr int RLD_R = JS + 4;  // BY_RIGHT r2u stage [128 j][32 k]
-constexpr int RLD_L = OB + 4;  // BY_LEFT  r2u stage [32 j][128 k]
+constexpr int RLD_R = JS + 4;  // BY_RIGHT r2u stage [64 j][16 k]
+constexpr int RLD_L = HB + 4;  // BY_LEFT  r2u stage [16 j][64 k]
 
 template <int NF, bool BY_RIGHT>
 struct ContractShape {
-    static constexpr int R_ELEMS = BY_RIGHT ? OB * RLD_R : JS * RLD_L;
+    static constexpr int R_ELEMS = BY_RIGHT ? HB * RLD_R : JS * RLD_L;
     static constexpr int STAGE = R_ELEMS + 8 * NF * SLD;   // doubles per buffer
     static constexpr size_t smem = sizeof(double) * 2 * (size_t)STAGE;
 };
@@ -82,7 +87,7 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 // NF: fragments of 8 columns per warp (the chunk has at most 8 NF columns;
 // results past it are not stored).
 template <int NF, bool BY_RIGHT>
-__global__ void __launch_bounds__(CTH)
+__global__ void __launch_bounds__(CTH, 3)
     k_contract_mma(const Tile* __restrict__ tiles, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
                    int32_t nblocks, EpilogueArgs ep) {
     using S = ContractShape<NF, BY_RIGHT>;
@@ -93,57 +98,75 @@ __global__ void __launch_bounds__(CTH)
     const int nchunks = (K + MK - 1) / MK;
     const int fr = lane >> 2, fc = lane & 3;   // fragment row / column of this lane
 
-    for (int64_t w = blockIdx.x; w < (int64_t)nblocks * nchunks; w += gridDim.x) {
-        const int32_t blk = (int32_t)(w / nchunks);
-        const int c0 = (int)(w % nchunks) * MK;
+    for (int64_t w = blockIdx.x; w < (int64_t)nblocks * nchunks * 2; w += gridDim.x) {
+        const int half = (int)(w & 1);
+        const int32_t blk = (int32_t)(w / 2 / nchunks);
+        const int c0 = (int)(w / 2 % nchunks) * MK;
         const int kc = K - c0 < MK ? K - c0 : MK;   // columns of this chunk
         const int32_t t0 = ptr[blk], t1 = ptr[blk + 1];
         if (t0 == t1) continue;
 
-        // the staged steps run over the block's tiles: cursor (tile entry, step in it)
-        struct Cursor {
-            int32_t e;
-            int st;
+        // the staged steps run over the block's tiles: this step's tile, and the next list entry
+        struct Entry {
+            Tile tl;
+            uint32_t roff;
         };
-        auto steps_of = [&](const Tile& tl) { return BY_RIGHT ? OB / JS : (int)tl.nq1 + 1; };
-        auto issue = [&](const Cursor& cu, int b) {
-            const int32_t t = idx[cu.e];
-            const Tile tl = tiles[t];
-            const double* src = ep.rtiles + (size_t)ep.roff[t] * TILE_QUARTER * OB;
+        auto tile_of = [&](int32_t e) { return idx[e < t1 ? e : t1 - 1]; };
+        int32_t e = t0, ahead = tile_of(t0 + 1);   // the tile after next
+        Entry cur{}, next{tiles[idx[t0]], ep.roff[idx[t0]]};
+        int st = 0, steps = 0;   // step of the tile, its steps
+        int lo = 0, hi = 1;      // BY_RIGHT: the tile's quarters within this half's two
+        bool more = true;
+        auto advance = [&]() {
+            if (++st < steps) return;
+            do {
+                more = e < t1;
+                if (!more) return;
+                cur = next;
+                next = Entry{tiles[ahead], ep.roff[ahead]};
+                ahead = tile_of(++e + 1);
+                if (BY_RIGHT) {
+                    lo = max((int)cur.tl.q0 - 2 * half, 0);
+                    hi = min((int)(cur.tl.q0 + cur.tl.nq1) - 2 * half, 1);
+                }
+            } while (BY_RIGHT && lo > hi);
+            st = 0;
+            steps = (BY_RIGHT ? OB : ((int)cur.tl.nq1 + 1) * TILE_QUARTER) / JS;
+        };
+        auto issue = [&](int b) {
+            const Tile tl = cur.tl;
+            const double* src = ep.rtiles + (size_t)cur.roff * TILE_QUARTER * OB;
             double* Rs = smm + b * S::STAGE;
             double* As = Rs + S::R_ELEMS;
             if (BY_RIGHT) {
-                // the tile's rows j, values k = 32 st .. 32 st + 31: 16-byte pieces
-                const int n = ((int)tl.nq1 + 1) * TILE_QUARTER;
-                double* dst = Rs + (int)tl.q0 * TILE_QUARTER * RLD_R;
+                // the half's rows j of the tile, values k = JS st .. JS st + JS - 1: 16-byte pieces
+                const int n = (hi - lo + 1) * TILE_QUARTER;
+                const double* sr = src + (size_t)(lo + 2 * half - (int)tl.q0) * TILE_QUARTER * OB + st * JS;
+                double* dst = Rs + lo * TILE_QUARTER * RLD_R;
                 for (int q = tid; q < n * JS / 2; q += CTH) {
                     const int r = q / (JS / 2), cc = 2 * (q % (JS / 2));
-                    cp_async16(dst + r * RLD_R + cc, src + (size_t)r * OB + cu.st * JS + cc);
+                    cp_async16(dst + r * RLD_R + cc, sr + r * OB + cc);
                 }
             } else {
-                // 32 rows j of the tile's quarter st, all 128 values
-                const double* q0 = src + (size_t)cu.st * JS * OB;
+                // JS rows j of the tile, this half's 64 values
+                const double* sr = src + (size_t)st * JS * OB + half * HB;
 #pragma unroll
-                for (int q = tid; q < JS * OB / 2; q += CTH) {
-                    const int r = q / (OB / 2), cc = 2 * (q % (OB / 2));
-                    cp_async16(Rs + r * RLD_L + cc, q0 + (size_t)r * OB + cc);
+                for (int q = tid; q < JS * HB / 2; q += CTH) {
+                    const int r = q / (HB / 2), cc = 2 * (q % (HB / 2));
+                    cp_async16(Rs + r * RLD_L + cc, sr + r * OB + cc);
                 }
             }
             // annotation column c0 + c of summed record s at aeff[s + (c0 + c) m]; consecutive threads
             // take consecutive records (coalesced), zeros past m or K
-            const int64_t s0 = BY_RIGHT ? (int64_t)tl.a_blk * OB + cu.st * JS
-                                        : (int64_t)tl.b_blk * OB + ((int)tl.q0 + cu.st) * TILE_QUARTER;
-            for (int e = tid; e < 8 * NF * JS; e += CTH) {
-                const int s = e & (JS - 1), c = e / JS;
-                const bool ok = s0 + s < m && c < kc;
-                cp_async8_zfill(As + c * SLD + s, ok ? ep.aeff + (s0 + s) + (int64_t)(c0 + c) * m : ep.aeff, ok);
-            }
-        };
-        auto advance = [&](Cursor& cu) {
-            if (++cu.st == steps_of(tiles[idx[cu.e]])) {
-                cu.st = 0;
-                cu.e++;
-            }
+            const int64_t s0 = BY_RIGHT ? (int64_t)tl.a_blk * OB + st * JS
+                                        : (int64_t)tl.b_blk * OB + (int)tl.q0 * TILE_QUARTER + st * JS;
+            const int s = tid & (JS - 1);
+            const bool in = s0 + s < m;
+            const double* col = ep.aeff + (in ? s0 + s + (int64_t)(c0 + tid / JS) * m : 0);
+            double* dst = As + (tid / JS) * SLD + s;
+#pragma unroll 4
+            for (int c = tid / JS; c < 8 * NF; c += CTH / JS, col += (CTH / JS) * m, dst += (CTH / JS) * SLD)
+                cp_async8_zfill(dst, in && c < kc ? col : ep.aeff, in && c < kc);
         };
 
         double acc[2][NF][2];
@@ -152,25 +175,23 @@ __global__ void __launch_bounds__(CTH)
 #pragma unroll
             for (int j = 0; j < NF; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-        Cursor cur{t0, 0}, nxt{t0, 0};
-        issue(nxt, 0);
-        advance(nxt);
+        advance();
+        bool staged = more;                           // something is in buffer b
+        bool active = warp / 2 >= lo && warp / 2 <= hi;   // this warp's rows are in it (warp-uniform)
+        if (more) issue(0);
         cp_async_commit();
-        for (int b = 0; cur.e < t1; b ^= 1) {
-            if (nxt.e < t1) {
-                issue(nxt, b ^ 1);
-                advance(nxt);
+        for (int b = 0; staged; b ^= 1) {
+            const bool act = active;
+            advance();
+            staged = more;
+            if (more) {
+                active = warp / 2 >= lo && warp / 2 <= hi;
+                issue(b ^ 1);
             }
             cp_async_commit();
             cp_async_wait1();  // the current step's copies (this thread's) have landed
             __syncthreads();   // ... and every thread's
-            bool active = true;   // warp-uniform
-            if (BY_RIGHT) {
-                const Tile tl = tiles[idx[cur.e]];
-                const int quarter = warp >> 1;
-                active = quarter >= (int)tl.q0 && quarter <= (int)(tl.q0 + tl.nq1);
-            }
-            if (active) {
+            if (act) {
                 const double* Rs = smm + b * S::STAGE;
                 const double* As = Rs + S::R_ELEMS;
 #pragma unroll 2
@@ -190,11 +211,10 @@ __global__ void __launch_bounds__(CTH)
                 }
             }
             __syncthreads();  // this buffer is refilled by the next iteration's issue
-            advance(cur);
         }
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const int64_t row = (int64_t)blk * OB + 16 * warp + 8 * i + fr;
+            const int64_t row = (int64_t)blk * OB + half * HB + 16 * warp + 8 * i + fr;
             if (row >= m) continue;
 #pragma unroll
             for (int j = 0; j < NF; j++)
@@ -241,7 +261,8 @@ static cudaError_t run_contract(const Tile* tiles, const int32_t* ptr, const int
     cudaError_t e =
         cudaFuncSetAttribute(k_contract_mma<NF, BY_RIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int64_t work = (int64_t)nblocks * ((ep.K + MK - 1) / MK), cap = (int64_t)sms * (NF <= 7 ? 2 : 1);
+    const int64_t work = 2 * (int64_t)nblocks * ((ep.K + MK - 1) / MK);
+    const int64_t cap = (int64_t)sms * std::min<int64_t>(3, 227 * 1024 / (int64_t)(smem + 1024));
     k_contract_mma<NF, BY_RIGHT><<<(unsigned)(work < cap ? work : cap), CTH, smem, stream>>>(tiles, ptr, idx, nblocks, ep);
     return cudaGetLastError();
 }

@@ -1802,7 +1802,7 @@ extern "C" int ldsc_h2_batch(ldsc_ctx* ctx, const ldsc_h2_args* a, ldsc_h2_resul
     CK(ctx->rg_states.ensure(sizeof(RegState) * J));
     CK(ctx->rg_outs.ensure(sizeof(RegOut) * T));
     CK(ctx->rg_part.ensure(sizeof(double) * 5 * (size_t)J * nb));
-    CK(ctx->rg_sel.ensure(sizeof(double) * 2 * T));
+    CK(ctx->rg_sel.ensure(sizeof(double) * (2 * T + SELECT_LD_PARTS)));
     CK(cudaMemcpyAsync(ctx->rg_jobs.p, jobs.data(), sizeof(RegJob) * J, cudaMemcpyHostToDevice, s));
     // the whole pipeline (8 regression kernels + the median; 2 x 8 + 3 for
     // --two-step) replays as one graph
@@ -1815,9 +1815,21 @@ extern "C" int ldsc_h2_batch(ldsc_ctx* ctx, const ldsc_h2_args* a, ldsc_h2_resul
         RegJob* dj = ctx->rg_jobs.as<RegJob>();
         RegState* dst = ctx->rg_states.as<RegState>();
         cudaError_t e2;
+        // median (src/h2.rs:394-414): middle order statistic, mean of the two for even n
+        // (rank n/2 in sel[0, T), rank n/2 - 1 in sel[T, 2T) for even n)
+        const uint64_t ra = n % 2 ? n / 2 : n / 2 - 1, rb = n / 2;
+        double* sel = ctx->rg_sel.as<double>();
         if (!two) {
+            // plain jobs with a median: its first sweep does the aggregate pass
+            const bool summed = a->want_lambda_gc && !d_n && select_sums(n);
+            if (summed) {
+                e2 = launch_select_mid_sums(dj, n, ra, rb, sel + T, sel, d_ld, sel + 2 * T, nb,
+                                            ctx->rg_part.as<double>(), T, gs);
+                if (e2 != cudaSuccess) return e2;
+            }
             e2 = launch_regressions(dj, dst, ctx->rg_outs.as<RegOut>(), nullptr, ctx->rg_part.as<double>(), nullptr,
-                                    d_ld, d_wld, n, nb, a->m_snps, T, gs, nullptr, REG_FORM_HSQ_DIRECT, !d_n);
+                                    d_ld, d_wld, n, nb, a->m_snps, T, gs, nullptr, REG_FORM_HSQ_DIRECT, !d_n, summed);
+            if (summed) return e2;
         } else {
             RegOut* o12 = ctx->ts_outs.as<RegOut>();
             double* dv = ctx->ts_dv.as<double>();
@@ -1834,10 +1846,7 @@ extern "C" int ldsc_h2_batch(ldsc_ctx* ctx, const ldsc_h2_args* a, ldsc_h2_resul
                                             ctx->rg_outs.as<RegOut>(), T, gs);
         }
         if (e2 != cudaSuccess || !a->want_lambda_gc) return e2;
-        // median (src/h2.rs:394-414): middle order statistic, mean of the two for even n
-        // (rank n/2 in sel[0, T), rank n/2 - 1 in sel[T, 2T) for even n)
-        return launch_select_mid(ctx->rg_jobs.as<RegJob>(), n, n % 2 ? n / 2 : n / 2 - 1, n / 2,
-                                 ctx->rg_sel.as<double>() + T, ctx->rg_sel.as<double>(), T, gs);
+        return launch_select_mid(dj, n, ra, rb, sel + T, sel, T, gs);
     }));
     ctx->kernels += (two ? 19 : 8) + (a->want_lambda_gc ? 1 : 0);
     const size_t o_sel = round_up(sizeof(RegOut) * T, 16), o_n1 = o_sel + 8 * 2 * (size_t)T;

@@ -640,7 +640,13 @@ __global__ void __launch_bounds__(NT) k_rg_finish(const RgPairIdx* __restrict__ 
 // equal bins of the keys' upper words; the second gathers the one or two bins that hold the
 // ranks, and the gathered keys are ranked in shared memory.  A bracket that
 // misses, or a bin of more than SEL_CAP keys (ties), falls back to the
-// radix select.  1,000 traits x 200,000: 638 us (radix select alone 1,689 us).
+// radix select.  1,000 traits x 200,000: 605 us, 638 with 8-byte copies (radix
+// select alone 1,689 us).
+//
+// SUM (plain h2 jobs, n >= SEL_SAMPLE_MIN): the first sweep also adds up y, in
+// two sums per thread, and leaves the aggregate pass's sums of the whole job in
+// its first block (the others 0), so that pass need not read y again: 605 us in
+// place of 636 for the median and 273 for the pass (1,000 x 200,000).
 //
 // Radix select: 11 bits per digit, one sweep per digit; the sweep histograms
 // the keys that share the prefix fixed so far.  Once that prefix holds at most
@@ -664,20 +670,33 @@ constexpr int SEL_W = SEL_T / 32;
 constexpr int SEL_BITS = 11;
 constexpr int SEL_BINS = 1 << SEL_BITS;
 constexpr int SEL_CAP = 1024;  // keys ranked in shared memory
-constexpr int SEL_DEPTH = 6;   // ring of the sweeps
+constexpr int SEL_DEPTH = 4;   // ring of the sweeps, in pairs
 constexpr int SEL_SAMPLE = 1024, SEL_HALF = 80;   // (the sample is sorted in the candidates' place)
 constexpr uint64_t SEL_SAMPLE_MIN = 16384;   // below, three sweeps of a cached y cost less than the sort
 
-// Calls f(value, valid) for every ya of the job; the trip count is the same in
-// every lane of a warp, so f may use warp-collective operations.  Each thread
-// copies its own values through a ring in shared memory (SEL_DEPTH loads in
-// flight without registers; seven CTAs of a job each per SM).
+// Calls f(value, valid, parity of its index) for every ya of the job; the trip
+// count is the same in every lane of a warp, so f may use warp-collective
+// operations.  Each thread copies its own values through a ring in shared memory
+// (SEL_DEPTH loads in flight without registers; seven CTAs of a job each per
+// SM), two neighbours at a time: one 16-byte copy where y is aligned to it, two
+// of 8 bytes where it is not, the same values either way.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
 template <class F>
-__device__ __forceinline__ void sel_sweep(const double* __restrict__ y, uint64_t n, double (*ring)[SEL_T], F f) {
-    const int32_t steps = (int32_t)((n + SEL_T - 1) / SEL_T);   // n < 2^31
+__device__ __forceinline__ void sel_sweep(const double* __restrict__ y, uint64_t n, double2 (*ring)[SEL_T], F f) {
+    const int32_t steps = (int32_t)((n + 2 * SEL_T - 1) / (2 * SEL_T));   // n < 2^31
+    const bool wide = (reinterpret_cast<uintptr_t>(y) & 15) == 0;
     auto issue = [&](int32_t t, int slot) {
-        const uint64_t i = (uint64_t)t * SEL_T + threadIdx.x;
-        if (i < n) cp_async8(&ring[slot][threadIdx.x], y + i);
+        const uint64_t i = 2 * ((uint64_t)t * SEL_T + threadIdx.x);
+        double* dst = reinterpret_cast<double*>(&ring[slot][threadIdx.x]);
+        if (wide && i + 1 < n) {
+            cp_async16(dst, y + i);
+        } else {
+            if (i < n) cp_async8(dst, y + i);
+            if (i + 1 < n) cp_async8(dst + 1, y + i + 1);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
@@ -689,19 +708,41 @@ __device__ __forceinline__ void sel_sweep(const double* __restrict__ y, uint64_t
             if (t >= steps) break;
             issue(t + SEL_DEPTH - 1, (slot + SEL_DEPTH - 1) % SEL_DEPTH);
             asm volatile("cp.async.wait_group %0;" ::"n"(SEL_DEPTH - 1) : "memory");
-            const bool v = (uint64_t)t * SEL_T + threadIdx.x < n;
-            f(ring[slot][threadIdx.x], v);   // (nothing valid where !v)
+            const uint64_t i = 2 * ((uint64_t)t * SEL_T + threadIdx.x);
+            const double2 v = ring[slot][threadIdx.x];   // (nothing valid past n)
+            f(v.x, i < n, 0);
+            f(v.y, i + 1 < n, 1);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// Partial sums of ld for k_select_mid<true>, one per CTA.
+constexpr int LD_PARTS = SELECT_LD_PARTS;
+__global__ void __launch_bounds__(SEL_T) k_ld_parts(const double* __restrict__ ld, uint64_t n, double* __restrict__ parts) {
+    __shared__ double red[SEL_W];
+    double s = 0.0;
+    for (uint64_t i = (uint64_t)blockIdx.x * SEL_T + threadIdx.x; i < n; i += (uint64_t)gridDim.x * SEL_T) s += ld[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < SEL_W; w++) t += red[w];
+        parts[blockIdx.x] = t;
+    }
+}
+
+template <bool SUM>
 __global__ void __launch_bounds__(SEL_T, 7) k_select_mid(const RegJob* __restrict__ jobs, uint64_t n, uint64_t ra,
                                                       uint64_t rb, double* __restrict__ out_a,
-                                                      double* __restrict__ out_b) {
+                                                      double* __restrict__ out_b, const double* __restrict__ ld_parts,
+                                                      int nb, double* __restrict__ part) {
     __shared__ uint32_t hist[SEL_BINS];
     __shared__ uint64_t cand[SEL_CAP];
-    __shared__ double ring[SEL_DEPTH][SEL_T];
+    __shared__ double2 ring[SEL_DEPTH][SEL_T];
+    __shared__ double yred[SUM ? SEL_W : 1];
     __shared__ uint32_t wsum[SEL_W];
     __shared__ uint32_t s_da, s_db, s_acc_a, s_acc_b, s_cnt;
     __shared__ unsigned long long s_ka, s_kb;
@@ -784,15 +825,35 @@ __global__ void __launch_bounds__(SEL_T, 7) k_select_mid(const RegJob* __restric
         const uint32_t range = (pb < SEL_SAMPLE ? (uint32_t)(cand[pb] >> 32) : 0xFFFFFFFFu) - klo;
         const int shift = max(0, 32 - __clz((int)(range | 1u)) - SEL_BITS);   // range >> shift < SEL_BINS
         uint32_t below = 0;
-        sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+        double ysum[2] = {0.0, 0.0};
+        sel_sweep(y, n, ring, [&](const double& yv, bool v, int odd) {
             const uint32_t k = okey_hi((uint32_t)__double2hiint(yv)), t = k - klo;
+            if (SUM && v) ysum[odd] += yv;
             below += v && k < klo;
             if (v && t <= range) atomicAdd(&hist[t >> shift], 1u);
         });
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xFFFFFFFFu, below, o);
         if (lane == 0) atomicAdd(&s_cnt, below);
+        if (SUM) {
+            double t = ysum[0] + ysum[1];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+            if (lane == 0) yred[warp] = t;
+        }
         __syncthreads();   // histogram and s_cnt complete; the sample is no longer read
+        if (SUM)
+            for (int b = threadIdx.x; b < nb; b += SEL_T) {
+                double a = 0.0, l = 0.0;
+                if (b == 0) {
+                    for (int w = 0; w < SEL_W; w++) a += yred[w];
+                    for (int x = 0; x < LD_PARTS; x++) l += ld_parts[x];
+                }
+                double* out = part + ((size_t)blockIdx.x * nb + b) * 5;
+                out[0] = a;
+                out[1] = jobs[blockIdx.x].n1s * l;
+                out[2] = b == 0 ? jobs[blockIdx.x].n1s * (double)n : 0.0;
+            }
         const uint64_t nbelow = s_cnt;
         const uint64_t inside = find_bins(ra - nbelow, rb - nbelow);   // (a rank below the bracket wraps: in no bin)
         if (ra >= nbelow && rb - nbelow < inside) {
@@ -803,7 +864,7 @@ __global__ void __launch_bounds__(SEL_T, 7) k_select_mid(const RegJob* __restric
                 const uint32_t cut = min(gr, range - (da << shift));
                 if (threadIdx.x == 0) s_cnt = 0;
                 __syncthreads();
-                sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+                sel_sweep(y, n, ring, [&](const double& yv, bool v, int) {
                     if (v && okey_hi((uint32_t)__double2hiint(yv)) - g0 <= cut) cand[atomicAdd(&s_cnt, 1u)] = okey(yv);
                 });
                 __syncthreads();
@@ -821,7 +882,7 @@ __global__ void __launch_bounds__(SEL_T, 7) k_select_mid(const RegJob* __restric
             // gather the prefix's keys and rank them in shared memory
             if (threadIdx.x == 0) s_cnt = 0;
             __syncthreads();
-            sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+            sel_sweep(y, n, ring, [&](const double& yv, bool v, int) {
                 const uint64_t k = okey(yv);
                 const bool take = v && (k & pmask) == prefix;
                 const unsigned m = __ballot_sync(0xFFFFFFFFu, take);
@@ -844,7 +905,7 @@ __global__ void __launch_bounds__(SEL_T, 7) k_select_mid(const RegJob* __restric
         const uint32_t dmask = (1u << width) - 1u;
         for (int i = threadIdx.x; i < SEL_BINS; i += SEL_T) hist[i] = 0;
         __syncthreads();
-        sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+        sel_sweep(y, n, ring, [&](const double& yv, bool v, int) {
             const uint64_t k = okey(yv);
             const bool take = v && (k & pmask) == prefix;
             const uint32_t bin = take ? (uint32_t)(k >> shift) & dmask : 0xFFFFFFFFu;
@@ -873,7 +934,7 @@ __global__ void __launch_bounds__(SEL_T, 7) k_select_mid(const RegJob* __restric
             s_kb = ~0ull;
         }
         __syncthreads();
-        sel_sweep(y, n, ring, [&](const double& yv, bool v) {
+        sel_sweep(y, n, ring, [&](const double& yv, bool v, int) {
             const uint64_t k = okey(yv);
             if (v && (k & nm) == pa) atomicMax(&s_ka, (unsigned long long)k);
             if (v && (k & nm) == pb) atomicMin(&s_kb, (unsigned long long)k);
@@ -1071,7 +1132,7 @@ cudaError_t launch_twostep_combine(const RegOut* out1, const RegOut* out2, const
 
 cudaError_t launch_regressions(const RegJob* jobs, RegState* states, RegOut* outs, const RegOut* ref_outs,
                                double* part, double* tot_delete, const double* ld, const double* wld, uint64_t n,
-                               int nb, double m, int njobs, cudaStream_t s, double* dv, int form, bool plain) {
+                               int nb, double m, int njobs, cudaStream_t s, double* dv, int form, bool plain, bool summed) {
     if (njobs <= 0) return cudaSuccess;
     if (form < REG_FORM_HSQ_DIRECT || form > REG_FORM_GENCOV_PRODUCT || n >= (1ull << 31))
         return cudaErrorInvalidValue;
@@ -1100,7 +1161,7 @@ cudaError_t launch_regressions(const RegJob* jobs, RegState* states, RegOut* out
                 go(std::integral_constant<int, 1>{}, f);
         });
     };
-    sums(0);
+    if (!summed) sums(0);
     k_reg_update<0><<<ub, 128, 0, s>>>(jobs, states, ref_outs, part, n, nb, m, njobs);
     for (int it = 0; it < 2; it++) {  // irwls_ldsc: two re-weightings
         sums(1);
@@ -1121,7 +1182,19 @@ cudaError_t launch_rg_finish(const RgPairIdx* pairs, const RegOut* outs, const d
 cudaError_t launch_select_mid(const RegJob* jobs, uint64_t n, uint64_t ra, uint64_t rb, double* out_a, double* out_b,
                               int njobs, cudaStream_t s) {
     if (njobs <= 0 || n == 0 || n >= (1ull << 31) || ra > rb || rb - ra > 1 || rb >= n) return cudaErrorInvalidValue;
-    k_select_mid<<<njobs, SEL_T, 0, s>>>(jobs, n, ra, rb, out_a, out_b);
+    k_select_mid<false><<<njobs, SEL_T, 0, s>>>(jobs, n, ra, rb, out_a, out_b, nullptr, 0, nullptr);
+    return cudaGetLastError();
+}
+
+bool select_sums(uint64_t n) { return n >= SEL_SAMPLE_MIN; }
+
+cudaError_t launch_select_mid_sums(const RegJob* jobs, uint64_t n, uint64_t ra, uint64_t rb, double* out_a,
+                                   double* out_b, const double* ld, double* ld_parts, int nb, double* part, int njobs,
+                                   cudaStream_t s) {
+    if (njobs <= 0 || !select_sums(n) || n >= (1ull << 31) || ra > rb || rb - ra > 1 || rb >= n)
+        return cudaErrorInvalidValue;
+    k_ld_parts<<<LD_PARTS, SEL_T, 0, s>>>(ld, n, ld_parts);
+    k_select_mid<true><<<njobs, SEL_T, 0, s>>>(jobs, n, ra, rb, out_a, out_b, ld_parts, nb, part);
     return cudaGetLastError();
 }
 
@@ -1140,7 +1213,9 @@ cudaError_t preload_regress() {
     if (e == cudaSuccess) e = preload_kernel(k_reg_update<1>);
     if (e == cudaSuccess) e = preload_kernel(k_reg_jackknife);
     if (e == cudaSuccess) e = preload_kernel(k_rg_finish);
-    if (e == cudaSuccess) e = preload_kernel(k_select_mid);
+    if (e == cudaSuccess) e = preload_kernel(k_select_mid<false>);
+    if (e == cudaSuccess) e = preload_kernel(k_select_mid<true>);
+    if (e == cudaSuccess) e = preload_kernel(k_ld_parts);
     if (e == cudaSuccess) e = preload_kernel(k_ts_count);
     if (e == cudaSuccess) e = preload_kernel(k_ts_seps);
     if (e == cudaSuccess) e = preload_kernel(k_ts_combine);

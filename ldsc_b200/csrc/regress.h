@@ -67,11 +67,12 @@ struct RgOut {
 // REG_GENCOV jobs refer to by index.  part: njobs * nb * 5 doubles of
 // scratch; tot_delete (optional): njobs * nb; dv (optional): njobs * nb * 2
 // delete values.  plain: every job has scalar sample sizes, no block starts of
-// its own and no mask.
+// its own and no mask.  summed: part already holds the aggregate pass's sums
+// (launch_select_mid_sums).
 cudaError_t launch_regressions(const RegJob* jobs, RegState* states, RegOut* outs, const RegOut* ref_outs,
                                double* part, double* tot_delete, const double* ld, const double* wld, uint64_t n,
                                int nb, double m, int njobs, cudaStream_t s, double* dv = nullptr,
-                               int form = REG_FORM_HSQ_DIRECT, bool plain = false);
+                               int form = REG_FORM_HSQ_DIRECT, bool plain = false, bool summed = false);
 
 // --two-step block starts: for each job, mask = y < mask_max, n1 = its size,
 // and seps[b] = index of the kept SNP of rank floor(b n1 / nb) (0 and n at
@@ -94,6 +95,15 @@ cudaError_t launch_rg_finish(const RgPairIdx* pairs, const RegOut* outs, const d
 // out_a[job] and out_b[job].
 cudaError_t launch_select_mid(const RegJob* jobs, uint64_t n, uint64_t ra, uint64_t rb, double* out_a, double* out_b,
                               int njobs, cudaStream_t s);
+
+// The same for plain h2 jobs on ya, with the aggregate pass's sums of every job
+// into part (as launch_regressions lays it out) from the same sweep, where
+// select_sums(n).  ld_parts: scratch of SELECT_LD_PARTS doubles.
+constexpr int SELECT_LD_PARTS = 148;
+bool select_sums(uint64_t n);
+cudaError_t launch_select_mid_sums(const RegJob* jobs, uint64_t n, uint64_t ra, uint64_t rb, double* out_a,
+                                   double* out_b, const double* ld, double* ld_parts, int nb, double* part, int njobs,
+                                   cudaStream_t s);
 
 // ---- partitioned h2 (fit_h2_partitioned, src/regressions.rs:1121-1226) ----
 

@@ -376,6 +376,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_sketch_seg(const uint32_t* __re
 // (584); 20,011 of 100,000, d = 5,000: 513 us (the earlier form 724).
 constexpr uint32_t SKETCH_MAX_RUN = 16383;
 
+// Row length at which 256 threads stop (32 bytes per quad and 4 per bucket in 200 KB).
 __host__ __device__ inline size_t sketch6_smem(uint64_t n_used, uint32_t d) {
     return 32 * sketch_quads(n_used) + 4 * (size_t)d + 16;
 }
@@ -586,11 +587,9 @@ __global__ void __launch_bounds__(T, 1024 / T) k_sketch_row(const uint32_t* __re
 
 }  // namespace
 
-// 256 threads, and with them the order of the norm's sum, from d = 2,560 on
-// (and while the bound on the row below holds).
+// 256 threads, and with them the order of the norm's sum, for large d.
 static bool sketch_large_d(uint64_t n_used, uint32_t d) { return d >= 2560 && sketch6_smem(n_used, d) <= 200 * 1024; }
 
-// @@RULE@@
 // Row-form CTAs of an SM by shared memory.
 static int64_t sketch_ctas(size_t smem_row, int threads) {
     return std::min<int64_t>(1024 / threads, 227 * 1024 / (int64_t)(smem_row + 1024 + 4 * threads + 256));

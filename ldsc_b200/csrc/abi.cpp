@@ -817,13 +817,15 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     CK(ctx->st_n.ensure(4 * nmom));
     CK(ctx->st_s.ensure(4 * nmom));
     CK(ctx->st_q.ensure(4 * nmom));
-    CK(ctx->maf.ensure(8 * nmom));
     CK(ctx->st_mean.ensure(8 * nmom));
     CK(ctx->st_inv.ensure(8 * nmom));
     CK(ctx->st_qinv.ensure(8 * nmom));
-    CK(ctx->l2.ensure(8 * nmom * K));
+    // l2, MAF and the error words in one buffer, so one copy reads them back
+    CK(ctx->l2.ensure(8 * nmom * K + 8 * nmom + 16));
+    double* const d_l2 = ctx->l2.as<double>();
+    double* const d_maf = d_l2 + nmom * K;
+    unsigned int* const d_err = reinterpret_cast<unsigned int*>(d_maf + nmom);
     CK(ctx->aeff.ensure(8 * nmom * K));
-    CK(ctx->err.ensure(16));
     const bool maf_aware = d && a->sketch_maf_aware;
     if (maf_aware) {
         CK(ctx->st_q3.ensure(4 * nmom));
@@ -858,7 +860,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     const uint64_t annot_ld_dev = !a->annot ? 0 : (a->annot_on_device && a->annot_ld ? a->annot_ld : nmom);
     if (a->bed_idx) CK(cudaMemcpyAsync(ctx->recrows.p, a->bed_idx, 8 * nmom, cudaMemcpyHostToDevice, up));
     if (a->keep_iids) CK(cudaMemcpyAsync(ctx->keep.p, a->keep_iids, 8 * a->n_keep, cudaMemcpyHostToDevice, up));
-    CK(cudaMemsetAsync(ctx->err.p, 0, 16, s));
+    CK(cudaMemsetAsync(d_err, 0, 16, s));
 
     PanelView pv{panel->rows, panel->n_snp, panel->n_indiv, panel->bpr, panel->pitch};
     if (!a->bed_idx) {
@@ -890,7 +892,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     st.q = ctx->st_q.as<int32_t>();
     st.q3 = maf_aware ? ctx->st_q3.as<int32_t>() : nullptr;
     st.q4 = maf_aware ? ctx->st_q4.as<int32_t>() : nullptr;
-    st.maf = ctx->maf.as<double>();
+    st.maf = d_maf;
     st.mean = ctx->st_mean.as<double>();
     st.inv_std = ctx->st_inv.as<double>();
     st.qinv = ctx->st_qinv.as<double>();
@@ -1085,7 +1087,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     ep.qinv = st.qinv;
     ep.kappa = st.kappa;
     ep.aeff = ctx->aeff.as<double>();
-    ep.l2 = ctx->l2.as<double>();
+    ep.l2 = d_l2;
     ep.m = m;
     ep.K = K;
     const double N = (double)n_used;
@@ -1096,7 +1098,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     ep.n_inv_sq = (1.0 / N) * (1.0 / N);
     ep.sketch_d = (double)d;
     ep.n_used = N;
-    ep.err = ctx->err.as<unsigned int>();
+    ep.err = d_err;
 
     // Whole-file INT8 runs with one annotation column overlap the band Gram
     // with the upload too: after chunk k is decoded and finalised, the tiles
@@ -1196,7 +1198,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                     sc.qinv += r0;
                     CK(launch_finalize_stats(r1 - r0, n_used, sc, annot_dev ? annot_dev + r0 : nullptr, 1,
                                              a->has_pq_exp, a->pq_exp, ctx->aeff.as<double>() + r0,
-                                             ctx->l2.as<double>() + r0, ds, annot_ld_dev));
+                                             d_l2 + r0, ds, annot_ld_dev));
                     ctx->kernels++;
                     // tiles are ordered by right block; take those whose right block is complete
                     size_t t1 = t0;
@@ -1252,7 +1254,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             CK(launch_decode_i8(pc, list, r1 - r0, ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8, ld_i8, sc, 0,
                                 ctx->side));
             CK(launch_finalize_stats(r1 - r0, n_used, sc, annot_dev ? annot_dev + r0 : nullptr, 1, a->has_pq_exp,
-                                     a->pq_exp, ctx->aeff.as<double>() + r0, ctx->l2.as<double>() + r0, ctx->side,
+                                     a->pq_exp, ctx->aeff.as<double>() + r0, d_l2 + r0, ctx->side,
                                      annot_ld_dev));
             CK(cudaEventRecord(ctx->ovl_ev[k], ctx->side));
             ctx->kernels += 2;
@@ -1274,7 +1276,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     ctx->kernels++;
     if (!stream_gram && !overlap) {
         CK(launch_finalize_stats(m, n_used, st, annot_dev, K, a->has_pq_exp, a->pq_exp, ctx->aeff.as<double>(),
-                                 ctx->l2.as<double>(), s, annot_ld_dev));
+                                 d_l2, s, annot_ld_dev));
         ctx->kernels++;
     }
     const int e1 = ev.mark();
@@ -1335,7 +1337,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         } else {
             const PanelView pk{ctx->packed.as<uint8_t>(), nmom, n_used, (n_used + 3) / 4, kp};
             CK(launch_gram_f64(compact ? pk : pv, compact ? nullptr : rr, st, dp.blocks,
-                               (uint32_t)ctx->plan_blocks.size(), ctx->err.as<unsigned int>() + 1, ep, ctx->sms, s));
+                               (uint32_t)ctx->plan_blocks.size(), d_err + 1, ep, ctx->sms, s));
         }
         ctx->kernels++;
         e_c = ev.mark();
@@ -1351,7 +1353,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         // the per-tile sums into l2, in a fixed order
         CK(launch_l2_reduce(m, ta, tb, dp.ptr_r, dp.idx_r, dp.ptr_l,
                             dp.idx_l, ctx->prow.as<double>(), ctx->pcol.as<double>(),
-                            ctx->l2.as<double>(), s));
+                            d_l2, s));
         ctx->kernels++;
     }
     const int e3 = ev.mark();
@@ -1359,19 +1361,25 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     // memory to the caller's host arrays (those too large for it directly)
     const size_t l2_bytes = 8 * nmom * K, maf_bytes = maf_out ? 8 * nmom : 0;
     const bool staged = !a->out_on_device && l2_bytes + maf_bytes <= HOST_OUT_MAX;
-    uint8_t* h = ctx->host_out.ensure(16 + (staged ? l2_bytes + maf_bytes : 0));
+    uint8_t* h = ctx->host_out.ensure(16 + (staged ? l2_bytes + 8 * nmom : 0));
     if (!h) return fail(ctx, LDSC_E_NOMEM, "out of host memory for the results");
-    const cudaMemcpyKind okind = a->out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    CK(cudaMemcpyAsync(staged ? h + 16 : (void*)l2_out, ctx->l2.p, l2_bytes, okind, s));
-    if (maf_out) CK(cudaMemcpyAsync(staged ? h + 16 + l2_bytes : (void*)maf_out, ctx->maf.p, maf_bytes, okind, s));
-    CK(cudaMemcpyAsync(h, ctx->err.p, 16, cudaMemcpyDeviceToHost, s));
+    const uint8_t* h_err = h;
+    if (staged) {
+        CK(cudaMemcpyAsync(h, d_l2, l2_bytes + 8 * nmom + 16, cudaMemcpyDeviceToHost, s));
+        h_err = h + l2_bytes + 8 * nmom;
+    } else {
+        const cudaMemcpyKind okind = a->out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+        CK(cudaMemcpyAsync(l2_out, d_l2, l2_bytes, okind, s));
+        if (maf_out) CK(cudaMemcpyAsync(maf_out, d_maf, maf_bytes, okind, s));
+        CK(cudaMemcpyAsync(h, d_err, 16, cudaMemcpyDeviceToHost, s));
+    }
     const int e4 = ev.mark();
     CK(cudaStreamSynchronize(s));
     ctx->up_pending = false;
-    const unsigned int* herr = reinterpret_cast<const unsigned int*>(h);
+    const unsigned int* herr = reinterpret_cast<const unsigned int*>(h_err);
     if (staged) {
-        std::memcpy(l2_out, h + 16, l2_bytes);
-        if (maf_out) std::memcpy(maf_out, h + 16 + l2_bytes, maf_bytes);
+        std::memcpy(l2_out, h, l2_bytes);
+        if (maf_out) std::memcpy(maf_out, h + l2_bytes, maf_bytes);
     }
     if (herr[0] != 0)
         return fail(ctx, LDSC_E_TIMEOUT, "a device wait in the Gram kernel exceeded its bound (error word " +

@@ -314,13 +314,14 @@ def run_sketch_workload(args, ctx, stream):
                "device_ms_per_call": float(np.mean([o[2].device_ms for o in outs])),
                "sketch_roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                                    "frac": achieved / hbm, "algorithmic_bytes": alg_bytes, "peak_source": src},
-               # the TF32 band Gram: every tile computes 64 x 128 record pairs over hi/lo rows
+               # the TF32 band Gram: a tile computes 128 x 128 record pairs (fewer where it is cut
+               # to the quarters it needs) over hi/lo rows
                # (4 products of round_up(d, 32) terms per pair, 8 flops per term); useful
                # work is 2 d flops per in-band pair
                "sketch_gram_roofline": {"bound": "tensor (TF32)", "unit": "TFLOP/s",
-                                        "achieved": 8.0 * ((d + 31) // 32 * 32) * 64 * 128 * perf.n_tiles
+                                        "achieved": 8.0 * ((d + 31) // 32 * 32) * 128 * 128 * perf.n_tiles
                                         / gram_s / 1e12,
-                                        "peak": tf32_peak, "frac": 8.0 * ((d + 31) // 32 * 32) * 64 * 128
+                                        "peak": tf32_peak, "frac": 8.0 * ((d + 31) // 32 * 32) * 128 * 128
                                         * perf.n_tiles / gram_s / 1e12 / tf32_peak,
                                         "useful_tflops": 2.0 * d * npairs / gram_s / 1e12,
                                         "tiles": int(perf.n_tiles), "peak_source": src,
@@ -956,7 +957,7 @@ def main():
     achieved = ops / gram_avg / 1e12
     roofline = {"bound": "tensor", "achieved": achieved, "peak": int8_peak, "unit": "TFLOP/s",
                 "frac": achieved / int8_peak, "traffic": committed_traffic("k_gram_tc"),
-                "kernel": "k_gram_tc<4,0,4,0> (tcgen05.mma kind::i8, TMA-staged operand rows)",
+                "kernel": "k_gram_tc<3,0,8,0> (tcgen05.mma kind::i8, TMA-staged operand rows)",
                 "note": "int8 ops counted like flops (2 per MAC, 4 products per pair); peak = 2 x "
                         + ("measured bf16 dense burst (MEASURED_PEAKS.json)" if src == "measured" else
                            "fallback bf16 dense burst 1590 TFLOP/s (MEASURED_PEAKS.json absent)")

@@ -74,31 +74,52 @@ struct DevBuf {
 // trim): page-locked up to PINNED_MAX, so a copy neither blocks the host nor goes
 // through the driver's staging buffer; larger, or where none can be locked,
 // ordinary memory.  One pageable copy of each result left the device idle
-// for 25 to 50 us before the next could start.
+// for 25 to 50 us before the next could start.  Locking and unlocking pages waits
+// for the device and stalls the other contexts on it, so a context starts with
+// what most calls need, growth at least doubles, and what was outgrown is kept
+// until the trim.
 struct HostBuf {
     static constexpr size_t PINNED_MAX = 64ull << 20;
+    struct Block {
+        uint8_t* p;
+        bool pinned;
+    };
     uint8_t* p = nullptr;
     size_t cap = 0;
-    bool pinned = false;
+    std::vector<Block> blocks;   // the last one is p
     uint8_t* ensure(size_t bytes) {   // null: out of memory
         if (bytes <= cap && p) return p;
-        release();
-        bytes += bytes / 8 + 4096;
-        pinned = bytes <= PINNED_MAX && cudaHostAlloc(reinterpret_cast<void**>(&p), bytes, cudaHostAllocDefault) == cudaSuccess;
-        if (!pinned) {
+        bytes = std::max(bytes + bytes / 8 + 4096, 2 * cap);
+        Block b{nullptr, false};
+        b.pinned = bytes <= PINNED_MAX &&
+                   cudaHostAlloc(reinterpret_cast<void**>(&b.p), bytes, cudaHostAllocDefault) == cudaSuccess;
+        if (!b.pinned) {
             cudaGetLastError();
-            p = static_cast<uint8_t*>(std::malloc(bytes));
+            b.p = static_cast<uint8_t*>(std::malloc(bytes));
+            if (!b.p) return nullptr;
         }
-        cap = p ? bytes : 0;
+        blocks.push_back(b);
+        p = b.p;
+        cap = bytes;
         return p;
     }
     void release() {
-        if (p && pinned) cudaFreeHost(p);
-        if (p && !pinned) std::free(p);
+        for (const Block& b : blocks) {
+            if (b.pinned)
+                cudaFreeHost(b.p);
+            else
+                std::free(b.p);
+        }
+        blocks.clear();
         p = nullptr;
         cap = 0;
     }
 };
+
+// Results up to this size leave through the context's page-locked memory; a
+// second host copy of larger ones costs more than the two waits it saves.
+constexpr size_t HOST_OUT_MAX = 8ull << 20;
+constexpr size_t HOST_UP_START = 4ull << 20;   // plan of 400,000 records
 
 uint64_t round_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
@@ -273,6 +294,8 @@ int ldsc_ctx_create(int device, uint32_t flags, ldsc_ctx** out) {
         return LDSC_E_CUDA;
     }
     c->stream = c->own;
+    c->host_out.ensure(HOST_OUT_MAX + (1 << 16));
+    c->host_up.ensure(HOST_UP_START);
     for (DevBuf* b : c->workspace()) b->owner = &c->stream;
     for (DevBuf* b : {&c->sk.perm, &c->sk.seg, &c->sk.segt, &c->sk.pp}) b->owner = &c->stream;
     // keep freed workspace in the pool for the next call instead of returning it
@@ -726,9 +749,6 @@ int ensure_overlap(ldsc_ctx* ctx, int n) {
 constexpr int64_t OVERLAP_CHUNKS = 4;
 constexpr int64_t OVERLAP_FIRST_DIV = 8;
 constexpr int64_t OVERLAP_MIN_RECORDS = 16384;
-// Results up to this size leave through the context's pinned memory; a second
-// host copy of larger ones costs more than the two waits it saves.
-constexpr size_t HOST_OUT_MAX = 8ull << 20;
 
 int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double* l2_out, double* maf_out,
            ldsc_perf* perf, double upload_secs, RowFeed* feed = nullptr) {

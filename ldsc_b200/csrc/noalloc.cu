@@ -24,6 +24,7 @@
 // again before this entry point is used.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 #include <string>
@@ -94,9 +95,9 @@ extern "C" int ldsc_l2_int8_noalloc(const uint8_t* d_rows, uint64_t pitch, uint6
     std::vector<int64_t> lv(left, left + m);
     std::vector<Tile> tiles;
     gram_tiles(lv, gram_trims(ld), 4, &tiles);
-    // the documented limit counts 8 bytes per 64 x 128 records of the band, at
-    // least as many as there are whole tiles
-    const uint64_t tile_room = band_tiles(lv, 64, 128).size();
+    // the documented limit counts 8 bytes per band tile of 64 x 128 records, at
+    // least as many as there are Gram tiles
+    const uint64_t tile_room = std::max<uint64_t>(band_tiles(lv, 64, 128).size(), tiles.size());
     uint64_t off = 0;
     auto take = [&](uint64_t bytes) {
         const uint64_t o = off;

@@ -204,11 +204,19 @@ void gram_tiles(const std::vector<int64_t>& left, bool trim, int max_quarters, s
         for (int64_t a = kmin / T; kmax >= kmin && a <= kmax / T; a++) {
             const int64_t k0 = a * T, k1 = k0 + T - 1;
             int first = 4, last = -1;
-            for (int q = 0; q < nq; q++)
-                if (lo[q] <= k1 && hi[q] >= k0 && lo[q] <= hi[q]) {
+            for (int q = 0; q < nq; q++) {
+                if (lo[q] > k1 || hi[q] < k0) continue;
+                // a pair left[j] <= k < j with k in the block: the first or second record has one,
+                // except at the band's ends and where windows are empty
+                bool any = false;
+                const int64_t ja = j0 + q * Q, jb = ja + Q < m ? ja + Q : m;
+                for (int64_t j = ja; j < jb && !any; j++)
+                    any = (left[j] > k0 ? left[j] : k0) <= (j - 1 < k1 ? j - 1 : k1);
+                if (any) {
                     first = q < first ? q : first;
                     last = q;
                 }
+            }
             if (!trim && last >= 0) {
                 first = 0;
                 last = 3;

@@ -45,7 +45,8 @@ void gram_blocks_of(const std::vector<Tile>& tiles, const std::vector<uint32_t>&
 // second form refills *out, keeping its storage.
 std::vector<Tile> band_tiles(const std::vector<int64_t>& left, int ta, int tb);
 // Gram tiles of the band (Tile, engine.h): per right block of 128 records the
-// left blocks it pairs with.  With trim, each is cut to the quarters of the
+// left blocks that hold an in-band pair with it, so there are never more whole
+// tiles than band tiles of 64 x 128.  With trim, each is cut to the quarters of the
 // right block that hold in-band pairs, and then into pieces of at most
 // max_quarters.  Ordered by right block, then left block.
 void gram_tiles(const std::vector<int64_t>& left, bool trim, int max_quarters, std::vector<Tile>* tiles);

@@ -127,10 +127,11 @@ __global__ void __launch_bounds__(32 * WARPS, 1)
                 for (int i = 0; i < 4; i++) {
                     const int64_t k = k0 + 8 * i + fr;
                     const double v = acc[i][j][h];
-                    const double r2u = pair_in_band(k, jj, m, ep.left) ? v * v * ep.n_inv_sq_r2u_a + ep.r2u_b : 0.0;
-                    if (ep.K == 1) {
-                        rs[i] += r2u * aj;
-                        cs[j][h] += r2u * ak[i];
+                    const bool in = pair_in_band(k, jj, m, ep.left);
+                    const double r2u = in ? v * v * ep.n_inv_sq_r2u_a + ep.r2u_b : 0.0;
+                    if (ep.K == 1) {   // (a masked pair adds 0 whatever its annotation, inf and NaN too)
+                        rs[i] += in ? r2u * aj : 0.0;
+                        cs[j][h] += in ? r2u * ak[i] : 0.0;
                     } else {
                         rt[(size_t)cj * TILE_RECORDS + 8 * i + fr] = r2u;
                     }

@@ -143,6 +143,15 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
+// Whether an annotation may enter a block's sums ahead of the pair's mask and
+// of r^2's other factors: 0, or of a size (2^-700 .. 2^700) that neither
+// overflows nor loses bits there.  A negative exponent of p q makes it inf at a
+// monomorphic record, and a column may hold inf or NaN: 0 x inf of a masked pair
+// would reach records outside the window.
+__device__ __forceinline__ bool plain_annot(double a) {
+    return a == 0.0 || ((uint32_t)__double2hiint(a) & 0x7FFFFFFFu) - (323u << 20) < (1400u << 20);
+}
+
 // Right-record constants and partial sums of the tile being finished
 // (double-buffered: a tile's sums leave while the next tile starts).
 struct EpiTile {
@@ -526,6 +535,7 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
             tc_fence_after();
             aphase ^= 1;
             const double a_rows = ep.K == 1 ? warp_sum(ak) : 0.0;   // annotation sum of the warp's rows
+            const bool plain_rows = __all_sync(0xFFFFFFFFu, plain_annot(ak));
 #pragma unroll 1
             for (int g = 0; g < NG; g++) {
                 const int cg = (ew >> 2) * NG + g, c0 = cg * 8 * nq;   // columns [c0, c0 + 8 nq) of the tile
@@ -536,8 +546,9 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                 const int64_t lo = ll > klo ? ll : klo, hi = jl - 1 < klo + 31 ? jl - 1 : klo + 31;
                 const bool any = __any_sync(0xFFFFFFFFu, jl < m && lo <= hi) || dbg != nullptr;
                 const bool all = __all_sync(0xFFFFFFFFu, jl < m && ll <= klo && klo + 31 < jl);
+                const bool plain = __all_sync(0xFFFFFFFFu, plain_annot(E.qa[cl].y)) && plain_rows;
                 // K = 1, INT8, a block inside the band: sums of X^2 / (n V), scaled at the end
-                const bool raw = MODE == 0 && all && ep.K == 1 && dbg == nullptr;
+                const bool raw = MODE == 0 && all && plain && ep.K == 1 && dbg == nullptr;
                 double rs[2] = {0.0, 0.0};
                 double* rt = ep.K == 1 ? nullptr : ep.rtiles + ((size_t)ep.roff[t] * TILE_QUARTER + c0) * TA + row;
                 if (!any) {
@@ -550,7 +561,8 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                     else
                         for (int c = 0; c < 8 * nq; c++) rt[(size_t)c * TA] = 0.0;
                 } else {
-                    // WHAT 0: K = 1, raw; 1: K = 1; 2: K > 1.  F32: sketch, the f32 form of r2u
+                    // WHAT 0: K = 1, raw; 1: K = 1; 2: K > 1; 3: K = 1, annotations that are not plain.
+                    // F32: sketch, the f32 form of r2u
                     auto finish = [&](auto what, auto f32) {
                         constexpr int WHAT = decltype(what)::value;
                         constexpr bool F32 = decltype(f32)::value;
@@ -568,7 +580,7 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                                 tc_fence_before();
                                 mbar_arrive(tempty);
                             }
-                            if (WHAT == 1 && dbg != nullptr && row >= dbg_row && row < dbg_row + 64) {
+                            if ((WHAT == 1 || WHAT == 3) && dbg != nullptr && row >= dbg_row && row < dbg_row + 64) {
 #pragma unroll
                                 for (int i = 0; i < 8; i++)
 #pragma unroll
@@ -602,11 +614,16 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                                     cv[i] = x2 * ck;
                                     continue;
                                 }
+                                bool in = true;
                                 if (!all) {
                                     const int64_t j = j0 + cb + i;
-                                    if (!(j < m && k < j && E.left[cb + i] <= k)) r2u = 0.0;
+                                    in = j < m && k < j && E.left[cb + i] <= k;
+                                    if (!in) r2u = 0.0;
                                 }
-                                if (WHAT == 1) {
+                                if (WHAT == 3) {   // masked pairs by the product
+                                    rs[i & 1] = in ? fma(r2u, E.qa[cb + i].y, rs[i & 1]) : rs[i & 1];
+                                    cv[i] = in ? r2u * ak : 0.0;
+                                } else if (WHAT == 1) {
                                     rs[i & 1] = fma(r2u, E.qa[cb + i].y, rs[i & 1]);
                                     cv[i] = r2u * ak;
                                 } else {
@@ -629,6 +646,8 @@ __global__ void __launch_bounds__(GRAM_BOUND, 1)
                             finish(std::integral_constant<int, 2>{}, f32);
                         else if (MODE == 0 && raw)
                             finish(std::integral_constant<int, 0>{}, f32);
+                        else if (!plain)
+                            finish(std::integral_constant<int, 3>{}, f32);
                         else
                             finish(std::integral_constant<int, 1>{}, f32);
                     };

@@ -1119,6 +1119,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     ep.sketch_d = (double)d;
     ep.n_used = N;
     ep.err = d_err;
+    ep.special = d_err + 2;
 
     // Whole-file INT8 runs with one annotation column overlap the band Gram
     // with the upload too: after chunk k is decoded and finalised, the tiles
@@ -1296,7 +1297,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     ctx->kernels++;
     if (!stream_gram && !overlap) {
         CK(launch_finalize_stats(m, n_used, st, annot_dev, K, a->has_pq_exp, a->pq_exp, ctx->aeff.as<double>(),
-                                 d_l2, s, annot_ld_dev));
+                                 d_l2, s, annot_ld_dev, K > 1 ? d_err + 2 : nullptr));
         ctx->kernels++;
     }
     const int e1 = ev.mark();
@@ -1366,7 +1367,8 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
                                ep, ctx->sms, s));
             CK(launch_contract(dp.tiles, dp.ptr_l, dp.idx_l, n_left, false,
                                ep, ctx->sms, s));
-            ctx->kernels += 2;
+            CK(launch_contract_special(dp.tiles, dp.ptr_r, dp.idx_r, dp.ptr_l, dp.idx_l, ep, ctx->sms, s));
+            ctx->kernels += 3;
         }
     }
     if (K == 1 && !tiles.empty()) {

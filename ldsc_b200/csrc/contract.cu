@@ -11,11 +11,16 @@
 // Everything is f64 -- the r2u values as the epilogue formed them, the
 // effective annotations as given, the products and sums -- so each l2_jC
 // carries f64 rounding only, binary and continuous columns alike.
+//
+// Pairs outside the band are 0 in a tile, and 0 x inf would be NaN at records
+// whose windows do not hold the annotation's record.  So the passes take an inf
+// or NaN annotation as 0, and a third kernel adds it to the record's partners.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "engine.h"
+#include "epilogue.cuh"
 #include "sm100.cuh"
 
 namespace ldsc {
@@ -97,6 +102,7 @@ __global__ void __launch_bounds__(CTH, 3)
     const int64_t m = ep.m;
     const int nchunks = (K + MK - 1) / MK;
     const int fr = lane >> 2, fc = lane & 3;   // fragment row / column of this lane
+    const bool special = *ep.special != 0;
 
     for (int64_t w = blockIdx.x; w < (int64_t)nblocks * nchunks * 2; w += gridDim.x) {
         const int half = (int)(w & 1);
@@ -190,6 +196,11 @@ __global__ void __launch_bounds__(CTH, 3)
             }
             cp_async_commit();
             cp_async_wait1();  // the current step's copies (this thread's) have landed
+            if (special) {     // inf and NaN among the annotations it copied
+                double* a = smm + b * S::STAGE + S::R_ELEMS + (tid / JS) * SLD + (tid & (JS - 1));
+                for (int c = tid / JS; c < 8 * NF; c += CTH / JS, a += (CTH / JS) * SLD)
+                    if (!isfinite(*a)) *a = 0.0;
+            }
             __syncthreads();   // ... and every thread's
             if (act) {
                 const double* Rs = smm + b * S::STAGE;
@@ -223,6 +234,43 @@ __global__ void __launch_bounds__(CTH, 3)
                     const int c = 8 * j + 2 * fc + h;
                     if (c < kc) ep.l2[row + (int64_t)(c0 + c) * m] += acc[i][j][h];
                 }
+        }
+    }
+}
+
+// Annotations that are inf or NaN, one warp each: a r2u_rp into l2 of every
+// partner p of its record r, from the tiles of r's left block (r on the left)
+// and of its right block.  (Sums with inf or NaN do not depend on their order.)
+__global__ void __launch_bounds__(CTH) k_contract_special(const Tile* __restrict__ tiles, const int32_t* __restrict__ ptr_r,
+                                                          const int32_t* __restrict__ idx_r, const int32_t* __restrict__ ptr_l,
+                                                          const int32_t* __restrict__ idx_l, EpilogueArgs ep) {
+    if (*ep.special == 0) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t m = ep.m, total = m * ep.K, warps = (int64_t)gridDim.x * (CTH / 32);
+    for (int64_t e0 = 32 * ((int64_t)blockIdx.x * (CTH / 32) + (threadIdx.x >> 5)); e0 < total; e0 += 32 * warps) {
+        unsigned found = __ballot_sync(0xFFFFFFFFu, e0 + lane < total && !isfinite(ep.aeff[e0 + lane]));
+        for (; found; found &= found - 1) {
+            const int64_t e = e0 + __ffs(found) - 1, r = e % m;
+            const double a = ep.aeff[e];
+            double* l2 = ep.l2 + (e - r);   // the annotation's column
+            const int64_t blk = r / OB;
+            const int at = (int)(r % OB);
+            for (int32_t i = ptr_l[blk]; i < ptr_l[blk + 1]; i++) {
+                const Tile tl = tiles[idx_l[i]];
+                const double* src = ep.rtiles + (size_t)ep.roff[idx_l[i]] * TILE_QUARTER * OB + at;
+                const int64_t j0 = (int64_t)tl.b_blk * OB + tl.q0 * TILE_QUARTER;
+                for (int x = lane; x < ((int)tl.nq1 + 1) * TILE_QUARTER; x += 32)
+                    if (pair_in_band(r, j0 + x, m, ep.left)) atomicAdd(l2 + j0 + x, src[(size_t)x * OB] * a);
+            }
+            for (int32_t i = ptr_r[blk]; i < ptr_r[blk + 1]; i++) {
+                const Tile tl = tiles[idx_r[i]];
+                const int row = at - (int)tl.q0 * TILE_QUARTER;
+                if (row < 0 || row >= ((int)tl.nq1 + 1) * TILE_QUARTER) continue;
+                const double* src = ep.rtiles + ((size_t)ep.roff[idx_r[i]] * TILE_QUARTER + row) * OB;
+                const int64_t k0 = (int64_t)tl.a_blk * OB;
+                for (int x = lane; x < OB; x += 32)
+                    if (pair_in_band(k0 + x, r, m, ep.left)) atomicAdd(l2 + k0 + x, src[x] * a);
+            }
         }
     }
 }
@@ -285,6 +333,12 @@ cudaError_t launch_contract(const Tile* tiles, const int32_t* ptr, const int32_t
 #undef LDSC_CONTRACT
 }
 
+cudaError_t launch_contract_special(const Tile* tiles, const int32_t* ptr_r, const int32_t* idx_r, const int32_t* ptr_l,
+                                    const int32_t* idx_l, const EpilogueArgs& ep, int sms, cudaStream_t stream) {
+    k_contract_special<<<(unsigned)(4 * sms), CTH, 0, stream>>>(tiles, ptr_r, idx_r, ptr_l, idx_l, ep);
+    return cudaGetLastError();
+}
+
 cudaError_t preload_contract() {
     cudaError_t e = preload_kernel(k_contract_mma<1, true>);
     if (e == cudaSuccess) e = preload_kernel(k_contract_mma<1, false>);
@@ -300,6 +354,7 @@ cudaError_t preload_contract() {
     if (e == cudaSuccess) e = preload_kernel(k_contract_mma<13, false>);
     if (e == cudaSuccess) e = preload_kernel(k_contract_mma<16, true>);
     if (e == cudaSuccess) e = preload_kernel(k_contract_mma<16, false>);
+    if (e == cudaSuccess) e = preload_kernel(k_contract_special);
     if (e == cudaSuccess) e = preload_kernel(k_l2_reduce);
     return e;
 }

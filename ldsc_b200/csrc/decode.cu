@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) k_decode_i8(PanelView p, const uint64_t* 
 // term r2u_jj * a_j = a_j.
 __global__ void k_finalize(int64_t m, uint64_t n_indiv, RecStats st, const double* __restrict__ annot,
                            uint64_t annot_ld, int32_t K, int has_pq, double pq_exp, double* __restrict__ aeff,
-                           double* __restrict__ l2_init) {
+                           double* __restrict__ l2_init, unsigned int* __restrict__ special) {
     int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= m) return;
     const int64_t n = st.n[r], s = st.s[r], q = st.q[r];
@@ -154,12 +154,15 @@ __global__ void k_finalize(int64_t m, uint64_t n_indiv, RecStats st, const doubl
         }
         st.kappa[r] = kap;
     }
+    bool other = false;   // inf or NaN
     for (int32_t c = 0; c < K; c++) {
         double a = annot ? annot[r + c * annot_ld] : 1.0;
         a *= pq;
+        other |= !isfinite(a);
         aeff[r + (int64_t)c * m] = a;
         l2_init[r + (int64_t)c * m] = a;
     }
+    if (other && special) atomicOr(special, 1u);
 }
 
 // One thread per 4-byte word of the pitched rows; the source is the file's
@@ -283,13 +286,13 @@ cudaError_t launch_repitch(const uint8_t* src, uint64_t bpr, uint8_t* dst, uint6
 
 cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st, const double* annot,
                                   int32_t K, int has_pq, double pq_exp, double* aeff,
-                                  double* l2_init, cudaStream_t stream, uint64_t annot_ld) {
+                                  double* l2_init, cudaStream_t stream, uint64_t annot_ld, unsigned int* special) {
     if (m <= 0) return cudaSuccess;
     // blocks of 64: in an overlapped run the SMs are held by the Gram, and a block
     // of 256 does not find its registers there until a Gram CTA ends
     k_finalize<<<(unsigned)((m + 63) / 64), 64, 0, stream>>>(m, n_indiv, st, annot,
                                                               annot_ld ? annot_ld : (uint64_t)m, K, has_pq,
-                                                              pq_exp, aeff, l2_init);
+                                                              pq_exp, aeff, l2_init, special);
     return cudaGetLastError();
 }
 

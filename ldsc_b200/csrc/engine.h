@@ -69,6 +69,7 @@ struct EpilogueArgs {
     // records (k) in f64, from quarter roff[t] (32 x 128 values each) of rtiles
     double* rtiles;
     const uint32_t* roff;
+    const unsigned int* special;   // K > 1: non-zero if an annotation is inf or NaN
     // K = 1: tile t's row sums (ta values at prow + t * ta: sum_j r2u a_j for
     // each left record k) and column sums (tb values at pcol + t * tb), added
     // to l2 in a fixed order by launch_l2_reduce; null = atomics into l2
@@ -90,11 +91,12 @@ cudaError_t launch_compact(const PanelView& p, const uint64_t* rec_rows, int64_t
 cudaError_t launch_decode_i8(const PanelView& p, const uint64_t* rec_rows, int64_t m, uint8_t* ops, uint64_t ld,
                              RecStats st, int want_moments, cudaStream_t stream);
 
-// Finalise per-record stats: maf, mean, inv_std, qinv, pq, kappa, aeff.
+// Finalise per-record stats: maf, mean, inv_std, qinv, pq, kappa, aeff.  special
+// (optional, zeroed) becomes non-zero if an effective annotation is inf or NaN.
 cudaError_t launch_finalize_stats(int64_t m, uint64_t n_indiv, RecStats st,
                                   const double* annot, int32_t K, int has_pq, double pq_exp,
                                   double* aeff, double* l2_init,
-                                  cudaStream_t stream, uint64_t annot_ld = 0);
+                                  cudaStream_t stream, uint64_t annot_ld = 0, unsigned int* special = nullptr);
 
 // Rows [r0, r1) of a packed BED body (bpr bytes per row, as in the file) to
 // the pitched panel layout; pad bytes are zeroed.
@@ -174,6 +176,10 @@ cudaError_t launch_gram_tf32(const float* ops, uint64_t ld, int64_t m, const Til
 // ptr/idx: CSR lists of tile indices per right block (by_right) or per left block.
 cudaError_t launch_contract(const Tile* tiles, const int32_t* ptr, const int32_t* idx, int32_t nblocks, bool by_right,
                             const EpilogueArgs& ep, int sms, cudaStream_t stream);
+// What the two passes leave out: annotations that are inf or NaN, into the l2 of
+// their records' partners (nothing to do unless *ep.special).
+cudaError_t launch_contract_special(const Tile* tiles, const int32_t* ptr_r, const int32_t* idx_r, const int32_t* ptr_l,
+                                    const int32_t* idx_l, const EpilogueArgs& ep, int sms, cudaStream_t stream);
 
 // Load a kernel's code on the current device now.  With lazy module loading
 // (the CUDA 12 default) a kernel is loaded at its first launch, which can

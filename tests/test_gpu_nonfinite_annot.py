@@ -110,3 +110,41 @@ def test_annotation_values_reach_the_window_only(ctx, fused_ctx, form, masking):
     panel.close()
     assert np.isfinite(want).sum() > 300
     _same(got, want)
+
+
+@pytest.mark.parametrize("masking", [True, False])
+@pytest.mark.parametrize("k_annot", [2, 20, 131])     # fragments of one and two, and a second chunk of columns
+@pytest.mark.parametrize("form", ["fp64", "int8", "int8_fused", "sketch"])
+def test_columns_with_special_values(ctx, fused_ctx, form, k_annot, masking):
+    """Several columns: each with its own special values equals the run on that
+    column alone, and the columns without any are what they are without them."""
+    from ldsc_b200.api import WindowMode, run_l2
+    n = 333
+    body, snps = _panel(n, [310])
+    m = len(snps.chr)
+    c = fused_ctx if form == "int8_fused" else ctx
+    panel = c.upload(body, n)
+
+    def l2_of(A, **kw):
+        out, _, _ = run_l2(c, snps, panel, WindowMode.Cm(1.3), 50, snp_level_masking=masking, annot=A,
+                           yes_really=True, **kw, **FORMS[form])
+        return out
+
+    rng = np.random.default_rng(k_annot)
+    A = rng.normal(size=(m, k_annot))
+    plain = l2_of(A)
+    B = A.copy()
+    B[5, 0], B[300, 0], B[310, 0] = np.inf, -np.inf, np.nan
+    B[1349, k_annot - 1] = -np.inf
+    got = l2_of(B)
+    mixed = sorted({0, k_annot - 1})
+    for col in mixed:
+        _same(got[:, col], l2_of(B[:, col:col + 1])[:, 0])
+        assert 300 < np.isfinite(got[:, col]).sum() < m
+    rest = [x for x in range(k_annot) if x not in mixed]
+    assert np.array_equal(got[:, rest], plain[:, rest])
+    if form != "sketch":   # negative exponent: every column of the monomorphic record is inf
+        pq = l2_of(A, pq_exp=-0.5)
+        for col in mixed:
+            _same(pq[:, col], l2_of(A[:, col:col + 1], pq_exp=-0.5)[:, 0])
+    panel.close()

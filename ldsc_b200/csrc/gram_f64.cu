@@ -35,6 +35,23 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
+// The epilogue's sums for a block with an inf or NaN annotation, masked by the
+// product: v[8 i + 2 j + h] is pair (k + 8 i, j0 + 8 j + h); o: 4 row sums, 8
+// column sums.  Its own function, so that the usual path keeps its registers
+// (with a select on every product there, the Gram and its reduction took 1,704 us
+// at the size above; this way 1,620).
+__device__ __noinline__ void masked_sums(const double* v, double* o, int64_t k, int64_t j0, int64_t m,
+                                         const int64_t* left, const double* aeff, double r2u_a, double r2u_b) {
+    for (int i = 0; i < 12; i++) o[i] = 0.0;
+    for (int p = 0; p < 32; p++) {
+        const int64_t kk = k + 8 * (p / 8), jj = j0 + 8 * (p / 2 % 4) + p % 2;
+        if (!pair_in_band(kk, jj, m, left)) continue;
+        const double r2u = v[p] * v[p] * r2u_a + r2u_b;
+        o[p / 8] += r2u * aeff[jj];
+        o[4 + p % 8] += r2u * aeff[kk];
+    }
+}
+
 __global__ void __launch_bounds__(32 * WARPS, 1)
     k_gram_f64(PanelView p, const uint64_t* __restrict__ rec_rows, RecStats st, const GramBlock* __restrict__ blocks,
                uint32_t n_blocks, unsigned int* __restrict__ next, EpilogueArgs ep) {
@@ -127,17 +144,30 @@ __global__ void __launch_bounds__(32 * WARPS, 1)
                 for (int i = 0; i < 4; i++) {
                     const int64_t k = k0 + 8 * i + fr;
                     const double v = acc[i][j][h];
-                    const bool in = pair_in_band(k, jj, m, ep.left);
-                    const double r2u = in ? v * v * ep.n_inv_sq_r2u_a + ep.r2u_b : 0.0;
-                    if (ep.K == 1) {   // (a masked pair adds 0 whatever its annotation, inf and NaN too)
-                        rs[i] += in ? r2u * aj : 0.0;
-                        cs[j][h] += in ? r2u * ak[i] : 0.0;
+                    const double r2u = pair_in_band(k, jj, m, ep.left) ? v * v * ep.n_inv_sq_r2u_a + ep.r2u_b : 0.0;
+                    if (ep.K == 1) {
+                        rs[i] += r2u * aj;
+                        cs[j][h] += r2u * ak[i];
                     } else {
                         rt[(size_t)cj * TILE_RECORDS + 8 * i + fr] = r2u;
                     }
                 }
             }
-        if (ep.K == 1) {   // the block's row and column sums; launch_l2_reduce adds them to l2
+        if (ep.K == 1) {
+            // inf or NaN among the block's annotations: 0 x inf of a masked pair is no part of a sum
+            const bool fin = (k0 + lane >= m || isfinite(__ldg(ep.aeff + k0 + lane))) &&
+                             (j0 + lane >= m || isfinite(__ldg(ep.aeff + j0 + lane)));
+            if (!__all_sync(0xFFFFFFFFu, fin)) {
+                double v[32], o[12];
+#pragma unroll
+                for (int i = 0; i < 32; i++) v[i] = acc[i / 8][i / 2 % 4][i % 2];
+                masked_sums(v, o, k0 + fr, j0 + 2 * fc, m, ep.left, ep.aeff, ep.n_inv_sq_r2u_a, ep.r2u_b);
+#pragma unroll
+                for (int i = 0; i < 4; i++) rs[i] = o[i];
+#pragma unroll
+                for (int i = 0; i < 8; i++) cs[i / 2][i % 2] = o[4 + i];
+            }
+            // the block's row and column sums; launch_l2_reduce adds them to l2
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 rs[i] += __shfl_xor_sync(0xFFFFFFFFu, rs[i], 1);

@@ -1835,12 +1835,14 @@ extern "C" int ldsc_h2_batch(ldsc_ctx* ctx, const ldsc_h2_args* a, ldsc_h2_resul
     CK(ctx->rg_sel.ensure(sizeof(double) * (2 * T + SELECT_LD_PARTS)));
     CK(cudaMemcpyAsync(ctx->rg_jobs.p, jobs.data(), sizeof(RegJob) * J, cudaMemcpyHostToDevice, s));
     // the whole pipeline (8 regression kernels + the median; 2 x 8 + 3 for
-    // --two-step) replays as one graph
+    // --two-step) replays as one graph; its key holds the address of every
+    // buffer its kernels use, so a graph whose buffer has moved is not replayed
     const std::vector<uint64_t> gkey{1, (uint64_t)T, n, (uint64_t)nb, dbits(a->m_snps), (uint64_t)a->want_lambda_gc,
                                      (uint64_t)d_ld, (uint64_t)d_wld, (uint64_t)ctx->rg_jobs.p,
                                      (uint64_t)ctx->rg_states.p, (uint64_t)ctx->rg_outs.p, (uint64_t)ctx->rg_part.p,
                                      (uint64_t)ctx->rg_sel.p, (uint64_t)two, (uint64_t)ctx->ts_seps.p,
-                                     (uint64_t)ctx->ts_dv.p, (uint64_t)ctx->ts_outs.p, (uint64_t)(d_n != nullptr)};
+                                     (uint64_t)ctx->ts_n1.p, (uint64_t)ctx->ts_cnt.p, (uint64_t)ctx->ts_dv.p,
+                                     (uint64_t)ctx->ts_outs.p, (uint64_t)(d_n != nullptr)};
     CK(graph_launch(ctx, gkey, s, [&](cudaStream_t gs) -> cudaError_t {
         RegJob* dj = ctx->rg_jobs.as<RegJob>();
         RegState* dst = ctx->rg_states.as<RegState>();

@@ -482,6 +482,15 @@ int ldsc_debug_gram_i8_tile(ldsc_ctx *ctx, const ldsc_panel *panel, uint64_t k0,
 int64_t ldsc_debug_gram_tiles(const int64_t *left, uint64_t n_snp, int32_t trim, int32_t max_quarters,
                               uint32_t *out, uint64_t cap);
 
+/* Compares the engine's short root, quotient and reciprocal with the IEEE
+ * operations on the device, over `count` arguments from index `first` on:
+ *   which 0: f32 square root, the argument's bits are the index;
+ *   which 1: f32 quotient, numerator of either sign and magnitude 2^-20 .. 2^40,
+ *            denominator 4 .. 2^30, both mixed from the index;
+ *   which 2: f64 reciprocal, over the exponents it accepts, mixed from the index.
+ * out[0]: results that differ, out[1]: the largest difference in places. */
+int ldsc_debug_approx(ldsc_ctx *ctx, int32_t which, uint64_t first, uint64_t count, uint64_t *out);
+
 #ifdef __cplusplus
 }
 #endif

@@ -167,6 +167,7 @@ SIGNATURES = {
     "ldsc_debug_gram_i8_tile": (C.c_int, [C.c_void_p, C.c_void_p, C.c_uint64, C.c_uint64,
                                           C.c_void_p]),
     "ldsc_debug_gram_tiles": (C.c_int64, [C.c_void_p, C.c_uint64, C.c_int32, C.c_int32, C.c_void_p, C.c_uint64]),
+    "ldsc_debug_approx": (C.c_int, [C.c_void_p, C.c_int32, C.c_uint64, C.c_uint64, C.c_void_p]),
     "ldsc_l2_int8_noalloc": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint64, C.c_void_p,
                                        C.c_void_p, C.c_void_p, C.c_void_p]),
     "ldsc_noalloc_last_error": (C.c_int, [C.c_char_p, C.c_size_t]),

@@ -1606,6 +1606,21 @@ int ldsc_sketch_project(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t b, uint
     return LDSC_OK;
 }
 
+int ldsc_debug_approx(ldsc_ctx* ctx, int32_t which, uint64_t first, uint64_t count, uint64_t* out) {
+    if (!ctx || !out) return LDSC_E_INVALID;
+    std::lock_guard<std::mutex> g(ctx->mu);
+    if (which < 0 || which > 2) return fail(ctx, LDSC_E_INVALID, "unknown operation");
+    CK(cudaSetDevice(ctx->device));
+    cudaStream_t s = ctx->stream;
+    CK(ctx->err.ensure(16));
+    CK(cudaMemsetAsync(ctx->err.p, 0, 16, s));
+    CK(launch_debug_approx(which, first, count, ctx->err.as<unsigned long long>(), s));
+    ctx->kernels++;
+    CK(cudaMemcpyAsync(out, ctx->err.p, 16, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return LDSC_OK;
+}
+
 int ldsc_debug_gram_i8_tile(ldsc_ctx* ctx, const ldsc_panel* panel, uint64_t k0, uint64_t j0, int32_t* out) {
     if (!ctx || !panel || !out) return LDSC_E_INVALID;
     std::lock_guard<std::mutex> g(ctx->mu);

@@ -181,6 +181,9 @@ cudaError_t launch_contract(const Tile* tiles, const int32_t* ptr, const int32_t
 cudaError_t launch_contract_special(const Tile* tiles, const int32_t* ptr_r, const int32_t* idx_r, const int32_t* ptr_l,
                                     const int32_t* idx_l, const EpilogueArgs& ep, int sms, cudaStream_t stream);
 
+// Short approximations against the IEEE operations (ldsc_debug_approx); out: two zeroed device words.
+cudaError_t launch_debug_approx(int which, uint64_t first, uint64_t count, unsigned long long* out, cudaStream_t stream);
+
 // Load a kernel's code on the current device now.  With lazy module loading
 // (the CUDA 12 default) a kernel is loaded at its first launch, which can
 // stall work already running on the device; contexts load every kernel of the

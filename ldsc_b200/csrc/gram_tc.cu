@@ -81,6 +81,7 @@
 
 #include <type_traits>
 
+#include "approx.cuh"
 #include "engine.h"
 #include "epilogue.cuh"
 #include "expand.cuh"
@@ -179,24 +180,6 @@ __device__ __forceinline__ double sketch_r2u(float val, double kap, const Epilog
     const double disc = dm3 * dm3 + 8.0 * (ep.sketch_d * tilde - 1.0);
     const double r2 = disc >= 0.0 ? (-dm3 + sqrt(disc)) * 0.25 : 0.0;
     return r2 * ep.r2u_a + ep.r2u_b;
-}
-
-// Square root and quotient of normal f32 numbers well inside the range: the
-// hardware's approximation and one correction from the exact remainder
-// (Newton's step for the root, Markstein's final correction for the quotient),
-// with no branch for special cases.  Against the IEEE operations: all 226
-// million x in [8, 2^30) equal; 1 of 3 billion quotients differs, by one place.
-__device__ __forceinline__ float sqrt_nr(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    const float s = x * y;
-    return fmaf(fmaf(-s, s, x), 0.5f * y, s);
-}
-__device__ __forceinline__ float div_nr(float a, float b) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-    const float q = a * y;
-    return fmaf(fmaf(-q, b, a), y, q);
 }
 
 // Sketch constants in f32 for sketch_r2u_f32.

@@ -17,6 +17,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "approx.cuh"
 #include "engine.h"
 #include "regress.h"
 
@@ -187,22 +188,6 @@ __global__ void __launch_bounds__(RJ * 32, form_kind(FORM) == REG_HSQ ? 3 : 1)
 #pragma unroll
         for (int q = 0; q < NQ; q++) out[q] = s[q];
     }
-}
-
-// 1 / d for positive d from the hardware's approximation of the upper word
-// (about 20 bits) by one step of Halley's iteration, which triples the bits:
-// with e = 1 - d r, 1/d = r / (1 - e) = r (1 + e + e^2 + ...), so r + r (e + e^2)
-// leaves e^3.  Without the division's own range checks the chains of a step
-// interleave.  Values outside the normal range's middle take the division.
-__device__ __forceinline__ bool recip_plain(double d) {
-    const uint32_t e = ((uint32_t)__double2hiint(d) >> 20);   // sign and exponent: 0x3FF at 1
-    return e - 2u < 2042u;
-}
-__device__ __forceinline__ double recip_halley(double d) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = fma(-d, r, 1.0);
-    return fma(r, fma(e, e, e), r);
 }
 
 // The same sums for plain jobs: scalar sample sizes, the blocks of sep(), no

@@ -197,8 +197,9 @@ __global__ void __launch_bounds__(RJ * 32, form_kind(FORM) == REG_HSQ ? 3 : 1)
 // shared.  The regressor's scale c = Nx / nbar is a constant of the job and
 // multiplies the finished sums (l in place of x0 = c l), so a term costs 12 f64
 // instructions, 3 of them the reciprocal.  A lane takes SNPs lane, lane + 32,
-// ... of the block whatever J is, so a job's sums do not depend on the other
-// jobs of the call.  Bound by the f64 pipe (half busy) and the LSU (70%) in the
+// ... of the block whatever J is, and each job's denominators choose between
+// iteration and division for that job alone, so a job's sums do not depend on
+// the other jobs of the call.  Bound by the f64 pipe (half busy) and the LSU (70%) in the
 // weighted pass, by DRAM (6 TB/s) in the aggregate pass.  1,000 traits x 200,000
 // SNPs: weighted pass 385 us, aggregate pass 269 us (k_reg_sums: 650 and 331 us).
 // Variants of the weighted pass, same sizes: loads in registers, four jobs per
@@ -262,7 +263,9 @@ __global__ void __launch_bounds__(RJ * 32, 3)
     auto step = [&](auto v_c, const double (&y)[2][J], const double (&l)[2], const double (&wl)[2]) {
         constexpr int V = decltype(v_c)::value;
         double d[V][J], w[V][J];
-        bool plain_range = true;
+        bool plain_range[J], every = true;
+#pragma unroll
+        for (int j = 0; j < J; j++) plain_range[j] = true;
 #pragma unroll
         for (int v = 0; v < V; v++) {
             const double ocd = fmax(wl[v], 1.0) * (KIND == REG_HSQ ? 2.0 : 1.0), l1 = fmax(l[v], 1.0);
@@ -272,10 +275,12 @@ __global__ void __launch_bounds__(RJ * 32, 3)
                 double t = c * c;
                 if (KIND == REG_GENCOV) t = fma(fma(ka[j], l1, ia[j]), fma(kb[j], l1, ib[j]), t);
                 d[v][j] = t * ocd;
-                plain_range &= recip_plain(d[v][j]);
+                plain_range[j] &= recip_plain(d[v][j]);
             }
         }
-        if (plain_range) {
+#pragma unroll
+        for (int j = 0; j < J; j++) every &= plain_range[j];
+        if (every) {
 #pragma unroll
             for (int v = 0; v < V; v++)
 #pragma unroll
@@ -284,7 +289,7 @@ __global__ void __launch_bounds__(RJ * 32, 3)
 #pragma unroll
             for (int v = 0; v < V; v++)
 #pragma unroll
-                for (int j = 0; j < J; j++) w[v][j] = 1.0 / d[v][j];
+                for (int j = 0; j < J; j++) w[v][j] = plain_range[j] ? recip_halley(d[v][j]) : 1.0 / d[v][j];
         }
 #pragma unroll
         for (int v = 0; v < V; v++)

@@ -99,3 +99,31 @@ def test_lambda_gc_two_sweeps(ctx, kind, m):
     got = h2_batch(ctx, np.stack([y, y[::-1].copy()]), [1e5, 1e5], ld, ld, 1e6, 7)
     for t in range(2):
         assert got[t]["lambda_gc"] == np.median(y) / 0.4549
+
+
+@pytest.mark.parametrize("case", ["nan_chi2", "huge_n"])
+def test_a_job_beside_one_out_of_range(ctx, case):
+    """A neighbour whose weights are NaN, or so small that their denominators leave
+    the reciprocal's range, changes no bit of the other jobs' results.  (The
+    reciprocal and the division differ by one place in 1 of 3,400 weights, and
+    few of those reach a result: many jobs of few SNPs.)"""
+    from ldsc_b200.api import h2_batch, rg_batch
+    m, nb, T = 150, 50, 20_000
+    _, ld, wld, n, z = _inputs(m, T, 11)
+    want = h2_batch(ctx, z * z, n, ld, wld, 1e6, nb)
+    bad = np.arange(1, T, 2)
+    rest = np.arange(0, T, 2)
+    chi2, n_bad = z * z, n.copy()
+    if case == "nan_chi2":
+        chi2[bad, 100] = np.nan
+    else:
+        n_bad[bad] = 1e300
+    got = h2_batch(ctx, chi2, n_bad, ld, wld, 1e6, nb)
+    for k in want.dtype.names:
+        np.testing.assert_array_equal(got[k][rest], want[k][rest])
+    # the two h2 fits of a pair lie in one warp
+    z1, n1, z2, n2 = z[::2], n[::2], z[1::2], n[1::2]
+    want = rg_batch(ctx, z1, z2, n1, n2, ld, wld, 1e6, nb)
+    got = rg_batch(ctx, z1, z2, np.full(T // 2, np.nan if case == "nan_chi2" else 1e300), n2, ld, wld, 1e6, nb)
+    for k in ("h2_2", "h2_2_se"):
+        np.testing.assert_array_equal(got[k], want[k])

@@ -123,6 +123,14 @@ constexpr size_t HOST_UP_START = 4ull << 20;   // plan of 400,000 records
 
 uint64_t round_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
+// --keep: pitch of a compacted row, and the records compacted at a time where the
+// decode that follows is their only reader (the FP64 Gram reads all of them
+// later): 64 MB, which the decode finds in L2.
+uint64_t compact_pitch(uint64_t n_keep) { return round_up((n_keep + 3) / 4, 16); }
+int64_t compact_records(uint64_t n_keep, int64_t m) {
+    return std::min<int64_t>(m, std::max<int64_t>(1, (int64_t)((64ull << 20) / compact_pitch(n_keep))));
+}
+
 // Instantiated CUDA graphs of fixed launch sequences, keyed by everything
 // their kernels' parameters depend on (sizes and buffer addresses).
 struct GraphCache {
@@ -536,7 +544,9 @@ int ldsc_l2_workspace_bytes(const ldsc_l2_args* a, uint64_t n_indiv, uint64_t* b
     if (f64) b += 16 * nt_room * (sizeof(GramBlock) + (K == 1 ? 8 * 64 + 16 : 0)) + (K == 1 ? 4 * (2 * (m / 32) + 4) : 0);
     if (a->annot && !a->annot_on_device) b += 8 * m * K;
     if (a->bed_idx) b += 8 * m;
-    if (a->keep_iids) b += 8 * a->n_keep + (d ? 0 : m * round_up((n_used + 3) / 4, 16));  // indices, compacted rows
+    // indices, compacted rows (all of them for the FP64 Gram)
+    if (a->keep_iids)
+        b += 8 * a->n_keep + (d ? 0 : (f64 ? m : (uint64_t)compact_records(n_used, (int64_t)m)) * compact_pitch(n_used));
     // INT8 operand rows (the default two-pass form; an upper bound for the fused one)
     if (exact_i8) b += 2 * m * round_up(n_used, 128);
     else if (d) b += 8 * m * round_up(d, 32);
@@ -891,20 +901,35 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     // --keep (exact forms): the kept individuals' rows are compacted first, and
     // everything after reads those
     const bool compact = a->keep_iids && !d;
-    const uint64_t kp = round_up((n_used + 3) / 4, 16);
-    if (compact) CK(ctx->packed.ensure((size_t)kp * nmom));
-    // rows of records [r0, r1) as the decode kernels read them (row list, or null for rows in order)
-    auto rows_of = [&](int64_t r0, int64_t r1, cudaStream_t on, PanelView* v, const uint64_t** list) -> cudaError_t {
-        *v = pv;
-        if (!rr) v->rows = pv.rows + (uint64_t)r0 * pv.pitch;
-        *list = rr ? rr + r0 : nullptr;
-        if (!compact) return cudaSuccess;
-        uint8_t* dst = ctx->packed.as<uint8_t>() + (size_t)r0 * kp;
-        const cudaError_t e = launch_compact(*v, *list, r1 - r0, ctx->keep.as<int64_t>(), n_used, dst, kp, on);
-        *v = PanelView{dst, (uint64_t)(r1 - r0), n_used, (n_used + 3) / 4, kp};
-        *list = nullptr;
-        ctx->kernels++;
-        return e;
+    const uint64_t kp = compact_pitch(n_used);
+    const int64_t piece = compact && !f64 ? compact_records(n_used, m) : m;
+    if (compact) CK(ctx->packed.ensure((size_t)kp * piece));
+    const uint64_t ld_i8 = round_up(n_used, 128);
+    // statistics (sc, of record r0) and operand rows (oc, or none) of records [r0, r1)
+    auto decode = [&](int64_t r0, int64_t r1, uint8_t* oc, const RecStats& sc, cudaStream_t on) -> cudaError_t {
+        for (int64_t p0 = r0; p0 < r1; p0 += piece) {
+            const int64_t p1 = std::min(r1, p0 + piece), at = p0 - r0;
+            PanelView v = pv;
+            if (!rr) v.rows = pv.rows + (uint64_t)p0 * pv.pitch;
+            const uint64_t* list = rr ? rr + p0 : nullptr;
+            if (compact) {
+                uint8_t* dst = ctx->packed.as<uint8_t>() + (f64 ? (size_t)p0 * kp : 0);
+                const cudaError_t e = launch_compact(v, list, p1 - p0, ctx->keep.as<int64_t>(), n_used, dst, kp, on);
+                if (e != cudaSuccess) return e;
+                v = PanelView{dst, (uint64_t)(p1 - p0), n_used, (n_used + 3) / 4, kp};
+                list = nullptr;
+                ctx->kernels++;
+            }
+            RecStats sp = sc;
+            sp.n += at;
+            sp.s += at;
+            sp.q += at;
+            const cudaError_t e =
+                launch_decode_i8(v, list, p1 - p0, oc ? oc + (size_t)2 * at * ld_i8 : nullptr, oc ? ld_i8 : 0, sp, 0, on);
+            if (e != cudaSuccess) return e;
+            if (at) ctx->kernels++;   // (the caller counts one)
+        }
+        return cudaSuccess;
     };
     RecStats st{};
     st.n = ctx->st_n.as<int32_t>();
@@ -1169,7 +1194,6 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
     const int e0 = ev.mark();
 
     // ---- decode ----
-    const uint64_t ld_i8 = round_up(n_used, 128);
     const uint64_t ld_sk = round_up(d ? d : 1, 32);  // 128-byte operand rows for TMA
     int e_sk = -1, e_side = -1;
     const bool staged_i8 = exact_i8 && !fused_i8;
@@ -1202,15 +1226,12 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             int rc = feed->issue_until(k + 1, ds);
             if (rc != LDSC_OK) return rc;
             if (r1 > r0) {
-                PanelView pc;
-                const uint64_t* list;
-                CK(rows_of(r0, r1, ds, &pc, &list));
                 RecStats sc = st;
                 sc.n += r0;
                 sc.s += r0;
                 sc.q += r0;
                 uint8_t* oc = staged_i8 ? ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8 : nullptr;
-                CK(launch_decode_i8(pc, list, r1 - r0, oc, staged_i8 ? ld_i8 : 0, sc, 0, ds));
+                CK(decode(r0, r1, oc, sc, ds));
                 ctx->kernels++;
                 if (stream_gram) {
                     sc.maf += r0;
@@ -1261,9 +1282,6 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         CK(cudaStreamWaitEvent(ctx->side, ctx->ovl_go, 0));
         for (int k = 0; k < ov_n; k++) {
             const int64_t r0 = ov_b[k], r1 = ov_b[k + 1];
-            PanelView pc;
-            const uint64_t* list;
-            CK(rows_of(r0, r1, ctx->side, &pc, &list));
             RecStats sc = st;
             sc.n += r0;
             sc.s += r0;
@@ -1272,8 +1290,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
             sc.mean += r0;
             sc.inv_std += r0;
             sc.qinv += r0;
-            CK(launch_decode_i8(pc, list, r1 - r0, ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8, ld_i8, sc, 0,
-                                ctx->side));
+            CK(decode(r0, r1, ctx->ops.as<uint8_t>() + (size_t)2 * r0 * ld_i8, sc, ctx->side));
             CK(launch_finalize_stats(r1 - r0, n_used, sc, annot_dev ? annot_dev + r0 : nullptr, 1, a->has_pq_exp,
                                      a->pq_exp, ctx->aeff.as<double>() + r0, d_l2 + r0, ctx->side,
                                      annot_ld_dev));
@@ -1283,10 +1300,7 @@ int run_l2(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a, double
         e_side = ev.mark_on(ctx->side);
         ctx->kernels--;  // counted once below
     } else if (!d) {
-        PanelView pc;
-        const uint64_t* list;
-        CK(rows_of(0, m, s, &pc, &list));
-        CK(launch_decode_i8(pc, list, m, staged_i8 ? ctx->ops.as<uint8_t>() : nullptr, staged_i8 ? ld_i8 : 0, st, 0, s));
+        CK(decode(0, m, staged_i8 ? ctx->ops.as<uint8_t>() : nullptr, st, s));
     } else {
         // fused: moments + CountSketch rows in one pass over the permuted panel
         CK(launch_sketch_seg(skc->pp.as<uint32_t>() + (rr ? 0 : a->row_begin * skc->pitch_words), skc->pitch_words,
@@ -1473,20 +1487,32 @@ int ldsc_snp_stats(ldsc_ctx* ctx, const ldsc_panel* panel, const ldsc_l2_args* a
         pv.n_snp -= a->row_begin;
     }
     const uint64_t* rr = a->bed_idx ? ctx->recrows.as<uint64_t>() : nullptr;
-    if (a->keep_iids) {
-        const uint64_t kp = round_up((n_used + 3) / 4, 16);
-        CK(ctx->packed.ensure((size_t)kp * m));
-        CK(launch_compact(pv, rr, m, ctx->keep.as<int64_t>(), n_used, ctx->packed.as<uint8_t>(), kp, s));
-        ctx->kernels++;
-        pv = PanelView{ctx->packed.as<uint8_t>(), (uint64_t)m, n_used, (n_used + 3) / 4, kp};
-        rr = nullptr;
-    }
     RecStats st{};
     st.n = ctx->st_n.as<int32_t>();
     st.s = ctx->st_s.as<int32_t>();
     st.q = ctx->st_q.as<int32_t>();
-    CK(launch_decode_i8(pv, rr, m, nullptr, 0, st, 0, s));
-    ctx->kernels++;
+    if (!a->keep_iids) {
+        CK(launch_decode_i8(pv, rr, m, nullptr, 0, st, 0, s));
+        ctx->kernels++;
+    } else {
+        const uint64_t kp = compact_pitch(n_used);
+        const int64_t piece = compact_records(n_used, m);
+        CK(ctx->packed.ensure((size_t)kp * piece));
+        for (int64_t r0 = 0; r0 < m; r0 += piece) {
+            const int64_t r1 = std::min(m, r0 + piece);
+            PanelView v = pv;
+            if (!rr) v.rows = pv.rows + (uint64_t)r0 * pv.pitch;
+            CK(launch_compact(v, rr ? rr + r0 : nullptr, r1 - r0, ctx->keep.as<int64_t>(), n_used,
+                              ctx->packed.as<uint8_t>(), kp, s));
+            v = PanelView{ctx->packed.as<uint8_t>(), (uint64_t)(r1 - r0), n_used, (n_used + 3) / 4, kp};
+            RecStats sp = st;
+            sp.n += r0;
+            sp.s += r0;
+            sp.q += r0;
+            CK(launch_decode_i8(v, nullptr, r1 - r0, nullptr, 0, sp, 0, s));
+            ctx->kernels += 2;
+        }
+    }
     std::vector<int32_t> hn((size_t)m), hs((size_t)m), hq((size_t)m);
     CK(cudaMemcpyAsync(hn.data(), st.n, 4 * (size_t)m, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(hs.data(), st.s, 4 * (size_t)m, cudaMemcpyDeviceToHost, s));

@@ -38,8 +38,10 @@ def call_bytes_per_record(snps: BimTable, n_indiv: int, mode: WindowMode, chunk_
     if rc != L.LDSC_OK:
         raise LdscError(rc, "workspace estimate failed")
     bpr = (n_indiv + 3) // 4
-    # the panel row, and with a sketch its bucket-major copy
-    return out.value / m + bpr * (2 if sketch else 1)
+    # the panel row, and with a sketch its bucket-major copy; a slice too short to
+    # fill the bounded buffer of compacted rows (--keep) holds all of its own
+    kept = 0 if iid_indices is None or sketch else (len(iid_indices) + 63) // 64 * 16
+    return out.value / m + bpr * (2 if sketch else 1) + kept
 
 
 def max_records_for_budget(snps: BimTable, n_indiv: int, budget_bytes: int, **kw) -> int:

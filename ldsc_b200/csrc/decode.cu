@@ -74,8 +74,12 @@ __device__ __forceinline__ void expand16(uint32_t w, uint8_t* grow, uint8_t* mro
 }
 
 // A warp decodes 2,048 individuals per step: lane l takes words l, l+32,
-// l+64, l+96 of the step (loads issued together, stores coalesced).
-__global__ void __launch_bounds__(256) k_decode_i8(PanelView p, const uint64_t* __restrict__ rec_rows,
+// l+64, l+96 of the step (loads issued together, stores coalesced).  Six blocks
+// per SM hold it to 40 registers, so that three fit beside a Gram CTA of long
+// rows (320 threads x 96) and one beside a Gram CTA of short ones (576); without
+// the bound it took 46, which left two and none.  Alone it reads faster too:
+// 100,000 records of 10,000 individuals 540 -> 503 us with the finalisation.
+__global__ void __launch_bounds__(256, 6) k_decode_i8(PanelView p, const uint64_t* __restrict__ rec_rows,
                                                    int64_t m, uint8_t* __restrict__ ops, uint64_t ld,
                                                    RecStats st, int want_moments) {
     const int lane = threadIdx.x & 31;

@@ -17,7 +17,6 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <algorithm>
 #include <atomic>
@@ -27,6 +26,7 @@
 
 #include "../../include/ldsc_b200.h"
 #include "engine.h"
+#include "hostbuf.h"
 #include "plan.h"
 #include "regress.h"
 
@@ -67,52 +67,6 @@ struct DevBuf {
     template <typename T>
     T* as() const {
         return reinterpret_cast<T*>(p);
-    }
-};
-
-// Host end of a call's copies, kept by the context (grow-only, given back by a
-// trim): page-locked up to PINNED_MAX, so a copy neither blocks the host nor goes
-// through the driver's staging buffer; larger, or where none can be locked,
-// ordinary memory.  One pageable copy of each result left the device idle
-// for 25 to 50 us before the next could start.  Locking and unlocking pages waits
-// for the device and stalls the other contexts on it, so a context starts with
-// what most calls need, growth at least doubles, and what was outgrown is kept
-// until the trim.
-struct HostBuf {
-    static constexpr size_t PINNED_MAX = 64ull << 20;
-    struct Block {
-        uint8_t* p;
-        bool pinned;
-    };
-    uint8_t* p = nullptr;
-    size_t cap = 0;
-    std::vector<Block> blocks;   // the last one is p
-    uint8_t* ensure(size_t bytes) {   // null: out of memory
-        if (bytes <= cap && p) return p;
-        bytes = std::max(bytes + bytes / 8 + 4096, 2 * cap);
-        Block b{nullptr, false};
-        b.pinned = bytes <= PINNED_MAX &&
-                   cudaHostAlloc(reinterpret_cast<void**>(&b.p), bytes, cudaHostAllocDefault) == cudaSuccess;
-        if (!b.pinned) {
-            cudaGetLastError();
-            b.p = static_cast<uint8_t*>(std::malloc(bytes));
-            if (!b.p) return nullptr;
-        }
-        blocks.push_back(b);
-        p = b.p;
-        cap = bytes;
-        return p;
-    }
-    void release() {
-        for (const Block& b : blocks) {
-            if (b.pinned)
-                cudaFreeHost(b.p);
-            else
-                std::free(b.p);
-        }
-        blocks.clear();
-        p = nullptr;
-        cap = 0;
     }
 };
 
@@ -373,8 +327,8 @@ int ldsc_ctx_trim(ldsc_ctx* ctx) {
         if (x) cudaStreamSynchronize(x);
     ctx->graphs.clear();  // their kernels hold the buffers' addresses
     for (DevBuf* b : ctx->workspace()) b->release();
-    ctx->host_up.release();
-    ctx->host_out.release();
+    ctx->host_up.trim();
+    ctx->host_out.trim();
     ctx->up_pending = false;
     ctx->sk.release();
     ctx->sk_panel = 0;

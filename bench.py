@@ -249,6 +249,21 @@ def _timed_passes(ctx, stream, fn, warmup, steps):
     return e0.elapsed_time(e1) / 1e3, outs
 
 
+def sketch_gram_executed(left, d):
+    """(tiles, record pairs multiplied) of the sketch Gram over the window limits
+    `left`: tiles of 128 x 128 records, cut to the quarters of 32 right records
+    they need while a row has fewer than 100 steps of 128 bytes."""
+    import ctypes
+    from ldsc_b200 import _lib
+    lib = _lib.load()
+    left = np.ascontiguousarray(left, dtype=np.int64)
+    trim = int((d + 31) // 32 * 32 * 4 // 128 < 100)
+    n = lib.ldsc_debug_gram_tiles(left.ctypes.data, len(left), trim, 4, None, 0)
+    tiles = np.zeros((n, 4), dtype=np.uint32)
+    lib.ldsc_debug_gram_tiles(left.ctypes.data, len(left), trim, 4, tiles.ctypes.data_as(ctypes.c_void_p), n)
+    return n, int(tiles[:, 3].sum()) * 128 * 32
+
+
 def run_sketch_workload(args, ctx, stream):
     """Fused CountSketch l2: N=100,000 x M=200,000 (1% missing, 150 cM),
     --sketch d --snp-level-masking, 1 cM.  Prints one JSON line per d with
@@ -258,7 +273,7 @@ def run_sketch_workload(args, ctx, stream):
     f32 --sketch path (seed-42 stream) and both sketches' Pearson r against
     the oracle's exact l2 on that sample."""
     from ldsc_b200 import synth
-    from ldsc_b200.api import WindowMode, pair_count, run_l2
+    from ldsc_b200.api import WindowMode, left_limits, pair_count, run_l2
     from ldsc_b200.plink import BimTable
     spec = synth.spec_sketch()
     if args.sketch_snps:
@@ -304,6 +319,9 @@ def run_sketch_workload(args, ctx, stream):
         bpr = (spec.n_indiv + 3) // 4
         alg_bytes = m * bpr + m * d * 4 + spec.n_indiv * 4
         achieved = alg_bytes / sk_s / 1e9
+        gram_tiles, gram_pairs = sketch_gram_executed(left_limits(snps, wm, 200, snp_level_masking=True), d)
+        assert gram_tiles == perf.n_tiles
+        gram_tflops = 8.0 * ((d + 31) // 32 * 32) * gram_pairs / gram_s / 1e12
         out = {"workload": "sketch", "config": {"n_indiv": spec.n_indiv, "n_snp": m, "sketch_d": d,
                                                 "window": "1 cM", "snp_level_masking": True},
                "metric": "r2 pairs/sec (sketch form)", "value": npairs * args.steps / t, "unit": "r2 pairs/s",
@@ -314,15 +332,11 @@ def run_sketch_workload(args, ctx, stream):
                "device_ms_per_call": float(np.mean([o[2].device_ms for o in outs])),
                "sketch_roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                                    "frac": achieved / hbm, "algorithmic_bytes": alg_bytes, "peak_source": src},
-               # the TF32 band Gram: a tile computes 128 x 128 record pairs (fewer where it is cut
-               # to the quarters it needs) over hi/lo rows
-               # (4 products of round_up(d, 32) terms per pair, 8 flops per term); useful
-               # work is 2 d flops per in-band pair
-               "sketch_gram_roofline": {"bound": "tensor (TF32)", "unit": "TFLOP/s",
-                                        "achieved": 8.0 * ((d + 31) // 32 * 32) * 128 * 128 * perf.n_tiles
-                                        / gram_s / 1e12,
-                                        "peak": tf32_peak, "frac": 8.0 * ((d + 31) // 32 * 32) * 128 * 128
-                                        * perf.n_tiles / gram_s / 1e12 / tf32_peak,
+               # the TF32 band Gram: the record pairs its tiles multiply, over hi/lo rows (4 products
+               # of round_up(d, 32) terms per pair, 8 flops per term); useful work is 2 d flops per
+               # in-band pair
+               "sketch_gram_roofline": {"bound": "tensor (TF32)", "unit": "TFLOP/s", "achieved": gram_tflops,
+                                        "peak": tf32_peak, "frac": gram_tflops / tf32_peak,
                                         "useful_tflops": 2.0 * d * npairs / gram_s / 1e12,
                                         "tiles": int(perf.n_tiles), "peak_source": src,
                                         "note": "peak = half the bf16 dense burst (dense TF32 is half rate)"},

@@ -15,7 +15,7 @@
 // and its reads do not conflict.
 //
 // Bound by the FP64 pipe.  2,490 individuals x 18,627 records, 1 cM, chunks of
-// 200: 1,590 us, 31 TFLOP/s over the blocks multiplied (columns written as f64 rows and multiplied in 128 x 128 tiles on the
+// 200: 1,610 us, 31 TFLOP/s over the blocks multiplied (columns written as f64 rows and multiplied in 128 x 128 tiles on the
 // SIMT pipe: decode 141 us + Gram 3,184 us).
 #include <cuda_runtime.h>
 

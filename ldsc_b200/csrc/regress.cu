@@ -667,8 +667,9 @@ constexpr uint64_t SEL_SAMPLE_MIN = 16384;   // below, three sweeps of a cached 
 // Calls f(value, valid, parity of its index) for every ya of the job; the trip
 // count is the same in every lane of a warp, so f may use warp-collective
 // operations.  Each thread copies its own values through a ring in shared memory
-// (SEL_DEPTH loads in flight without registers; seven CTAs of a job each per
-// SM), two neighbours at a time: one 16-byte copy where y is aligned to it, two
+// (SEL_DEPTH loads in flight without registers; six CTAs of a job each per SM by
+// their 32.9 KB of shared memory, so 1,000 jobs are a wave of 888 and a second of
+// 112), two neighbours at a time: one 16-byte copy where y is aligned to it, two
 // of 8 bytes where it is not, the same values either way.
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem)
